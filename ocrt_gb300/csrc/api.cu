@@ -2102,10 +2102,9 @@ int ocean_solve(int n, const ocrt_case *cases, const ocrt_opts *opts, int opp, c
         LAUNCH(&plan, KC_COXMUNK, k_water_modes<<<(n + 127) / 128, 128, 0, st>>>(d_op, n, GW.px, GW.pix_task0, GeW.NR,
                                                                                  GW.edge));
         const int Mc = std::max(Ma, Mw);
-        const size_t extra = 3 * (size_t)(Mc + 1) + GeW.NR + (GeW.NR + 1) / 2 + 1;
-        const size_t smem = iface_smem_bytes(Mc, 128, (int)extra);
+        const size_t smem = couple_wa_smem_bytes(Mc, GeW.NR);
         CK(cudaFuncSetAttribute(k_couple_wa, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(smem + 1024, 227 * 1024)));
-        LAUNCH(&plan, KC_COXMUNK, k_couple_wa<<<dim3(GeA.NR + 1, n), 128, smem, st>>>(
+        LAUNCH(&plan, KC_COXMUNK, k_couple_wa<<<dim3(GeA.NR + 1, n), 256, smem, st>>>(
                    d_op, n, GA.px, GW.px, GW.pix_task0, GA.gmu, Nw, GeA.NR, GeW.NR, GW.edge, d_glo, d_ext3, d_view));
     }
     // ---- pass 3: the atmosphere driven by the water-leaving radiance ----

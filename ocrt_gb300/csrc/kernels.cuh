@@ -360,9 +360,17 @@ __global__ void k_ocean_final(const OceanPix *op, int P, const PixDev *pxa, cons
                               const double *gmu, const double *gw, int N, int NRw, const double *edge_w,
                               const double *view, const double *top, const ocrt_result *r1, const ocrt_result *rw,
                               const ocrt_result *r3, ocrt_result *out, ocrt_ocean_result *wout);
-// shared-memory bytes of the interface-projection kernels for M modes
+// shared memory of the interface-projection kernels for M modes on nphi
+// azimuths (an even count, sampled on its half grid): floats of the cos/sin
+// table, one Mueller sample set and its projection, and the bytes with
+// extra_doubles accumulators behind them
+__host__ __device__ inline size_t iface_floats(int M, int nphi)
+{
+    const size_t hp = nphi / 2 + 1;
+    return ((size_t)(M + 1) * 2 * hp + 9 * hp + (size_t)(M + 1) * 9 + 1) & ~(size_t)1;
+}
 inline size_t iface_smem_bytes(int M, int nphi, int extra_doubles)
 {
-    return sizeof(float) * ((size_t)(M + 1) * nphi * 2 + (size_t)nphi * 9 + (((size_t)(M + 1) * 9 + 1) & ~(size_t)1)) +
-           sizeof(double) * (size_t)extra_doubles;
+    return sizeof(float) * iface_floats(M, nphi) + sizeof(double) * (size_t)extra_doubles;
 }
+size_t couple_wa_smem_bytes(int M, int NRw);

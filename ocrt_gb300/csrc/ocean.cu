@@ -118,9 +118,9 @@ __device__ void taw_mueller(float mu_i, float si, float mu_o, float so, float cp
 // Water -> air facet transmission Mueller, air cosine mu2 (sine s2), upwelling
 // water cosine mu1 (sine s1) (shared/surface.c:648-764); the facet tilt from
 // the normal N = n p1 - p2: tan^2(beta) = |N_h|^2 / N_z^2.  Sines as for
-// taw_mueller.
-__device__ void twa_mueller(float mu2, float s2, float mu1, float s1, float cphi, float sphi, float s2v, float slen,
-                            float n, int qc, float *T)
+// taw_mueller; S is the pair's shadowing factor.
+__device__ __forceinline__ void twa_mueller(float mu2, float s2, float mu1, float s1, float cphi, float sphi, float s2v,
+                                            float S, float n, int qc, float *T)
 {
 #pragma unroll
     for (int e = 0; e < 9; ++e) T[e] = 0.f;
@@ -142,7 +142,6 @@ __device__ void twa_mueller(float mu2, float s2, float mu1, float s1, float cphi
     const float ts = 1.f + rs, tp = n * (1.f + rp);
     const float cb2 = cb * cb, tb2 = Nh2 / (Nz * Nz);
     const float P = expf(-tb2 / s2v) / (3.14159265f * s2v);
-    const float S = 1.f / (1.f + sancer_f(mu1, slen) + sancer_f(mu2, slen));
     const float common = (maf * maf) / (n * mu1 * mu2 * Nsq) * (P / (cb2 * cb2)) * S;
     const float fs = common * ts * ts, fp = common * tp * tp, fsp = common * ts * tp;
     const float f1 = qc == 1 ? 0.5f * (fp - fs) : 0.5f * (fs - fp);
@@ -151,34 +150,44 @@ __device__ void twa_mueller(float mu2, float s2, float mu1, float s1, float cphi
     rotate_f(0.5f * (fs + fp), f1, fsp, c1, si1, c2, si2, T);
 }
 
-// Shared-memory table of cos(m phi_q), sin(m phi_q) on the midpoint grid
-// phi_q = (q + 1/2) 2 pi / nphi for m <= M: cs[(m * nphi + q) * 2 + {0, 1}].
-__device__ void fill_cs(float *cs, int M, int nphi)
+// The interface kernels are sampled on the half azimuth grid
+// phi_q = (q + 1/2) 2 pi / nphi, q < nphi / 2: under phi -> -phi the entries
+// 0, 1, 3, 4, 8 of a Mueller matrix are even and 2, 5, 6, 7 odd, so the other
+// half adds the same again (half the Mueller evaluations and half the
+// projection of the full grid).  Rows of half + 1 floats keep the lanes that
+// read different entries or modes at one azimuth on different banks.
+//
+// Shared-memory table of cos(m phi_q), sin(m phi_q), m <= M:
+// cs[(2 m + {0, 1}) * (half + 1) + q].
+__device__ void fill_cs(float *cs, int M, int half)
 {
-    for (int x = threadIdx.x; x < (M + 1) * nphi; x += blockDim.x) {
-        const int m = x / nphi, q = x - m * nphi;
+    for (int x = threadIdx.x; x < (M + 1) * half; x += blockDim.x) {
+        const int m = x / half, q = x - m * half;
         float s, c;
         // m (2q + 1) / nphi reduced exactly before the pi-scaled sincos
-        const long long num = (long long)m * (2 * q + 1) % (2LL * nphi);
-        sincospif((float)num / (float)nphi, &s, &c);
-        cs[2 * x] = c; cs[2 * x + 1] = s;
+        const long long num = (long long)m * (2 * q + 1) % (4LL * half);
+        sincospif((float)num / (float)(2 * half), &s, &c);
+        cs[(2 * m) * (half + 1) + q] = c;
+        cs[(2 * m + 1) * (half + 1) + q] = s;
     }
 }
 
-// Fourier coefficients of one kernel sampled by the block in Rq[nphi][9]:
-// out[m][e] = (dphi / (2 pi or pi)) sum_q Rq[q][e] {cos, sin}(m phi_q), with
-// the incoming-U column of m > 0 negated when fold_u (T_aw, T_wa: surface.c
-// :1680-1684, 1722-1729).  Ends with a block barrier.
-__device__ void project_block(const float *Rq, const float *cs, int nphi, int M, bool fold_u, float *out)
+// Fourier coefficients of one kernel sampled by the block in
+// Rq[entry * (half + 1) + q]: out[m][e] = 2 (dphi / (2 pi or pi)) sum_q Rq {cos, sin}(m phi_q),
+// with the incoming-U column of m > 0 negated when fold_u (T_aw, T_wa:
+// surface.c:1680-1684, 1722-1729).  Ends with a block barrier.
+__device__ void project_block(const float *Rq, const float *cs, int half, int M, bool fold_u, float *out)
 {
-    const float dphi = 6.28318530718f / (float)nphi;
+    const float dphi = 6.28318530718f / (float)half;          // 2 x the full grid's step
     for (int o = threadIdx.x; o < (M + 1) * 9; o += blockDim.x) {
         const int m = o / 9, e = o - 9 * m;
         const int sin_e = (e == 2 || e == 5 || e == 6 || e == 7);
-        const float *t = cs + (size_t)m * nphi * 2 + sin_e;
-        float acc = 0.f;
-        for (int q = 0; q < nphi; ++q) acc = fmaf(Rq[q * 9 + e], t[2 * q], acc);
-        float v = acc * dphi * (m == 0 ? 0.159154943092f : 0.318309886184f);
+        const float *t = cs + (size_t)(2 * m + sin_e) * (half + 1), *r = Rq + e * (half + 1);
+        float a0 = 0.f, a1 = 0.f;
+        int q = 0;
+        for (; q + 1 < half; q += 2) { a0 = fmaf(r[q], t[q], a0); a1 = fmaf(r[q + 1], t[q + 1], a1); }
+        if (q < half) a0 = fmaf(r[q], t[q], a0);
+        float v = (a0 + a1) * dphi * (m == 0 ? 0.159154943092f : 0.318309886184f);
         if (fold_u && m > 0 && (e == 2 || e == 5)) v = -v;
         out[o] = v;
     }
@@ -233,10 +242,11 @@ __global__ void k_rww(const TaskDev *tasks, const PixDev *px, int p0, const int 
     if (d.medium != 1 || o >= d.n_ring) return;
     const int N = G.N, M = d.M;
     extern __shared__ float sm[];
-    float *cs = sm;                                  // [(M+1) nphi 2]
-    float *Rq = cs + (size_t)(M + 1) * nphi * 2;     // [nphi][9]
-    float *out = Rq + (size_t)nphi * 9;              // [(M+1) 9]
-    fill_cs(cs, M, nphi);
+    const int half = nphi / 2;
+    float *cs = sm;                                        // [2 (M + 1)][half + 1]
+    float *Rq = cs + (size_t)(M + 1) * 2 * (half + 1);     // [9][half + 1]
+    float *out = Rq + 9 * (size_t)(half + 1);              // [(M+1) 9]
+    fill_cs(cs, M, half);
     const float s2v = (float)slope_variance(d.wind, d.sigma_type), slen = sqrtf(s2v);
     const float mo = (float)ring_mu(d, gmu, N, o), nw = (float)d.n_water;
     const float lo = sancer_f(mo, slen);
@@ -245,15 +255,17 @@ __global__ void k_rww(const TaskDev *tasks, const PixDev *px, int p0, const int 
     for (int i = 0; i < N; ++i) {
         const float mi = (float)gmu[i];
         const float lam = lo + sancer_f(mi, slen);
-        for (int q = threadIdx.x; q < nphi; q += blockDim.x) {
+        for (int q = threadIdx.x; q < half; q += blockDim.x) {
             const float phi = (q + 0.5f) * dphi;
-            float sp, cp;
+            float sp, cp, R[9];
             sincosf(phi, &sp, &cp);
             const float sh = sinf(0.5f * phi);
-            coxmunk_R<float>(mo, mi, cp, sp, sh * sh, s2v, lam, nw, d.q_conv, Rq + q * 9, nullptr, true);
+            coxmunk_R<float>(mo, mi, cp, sp, sh * sh, s2v, lam, nw, d.q_conv, R, nullptr, true);
+#pragma unroll
+            for (int e = 0; e < 9; ++e) Rq[e * (half + 1) + q] = R[e];
         }
         __syncthreads();
-        project_block(Rq, cs, nphi, M, false, out);
+        project_block(Rq, cs, half, M, false, out);
         for (int x = threadIdx.x; x < (M + 1) * 9; x += blockDim.x) {
             const int m = x / 9, e = x - 9 * m;
             const TaskDev tk = tasks[pix_task0[p] + m];
@@ -350,13 +362,13 @@ __global__ void k_couple_aw(const OceanPix *op, int P, const int *task0_a, const
     const int iw = blockIdx.x, p = blockIdx.y;
     if (p >= P || iw >= N) return;
     const OceanPix &o = op[p];
-    const int M = o.M, nphi = 128;
+    const int M = o.M, nphi = 128, half = nphi / 2;
     extern __shared__ float sm[];
     float *cs = sm;
-    float *Rq = cs + (size_t)(M + 1) * nphi * 2;
-    float *out = Rq + (size_t)nphi * 9;
-    double *acc = reinterpret_cast<double *>(out + (((M + 1) * 9 + 1) & ~1));
-    fill_cs(cs, M, nphi);
+    float *Rq = cs + (size_t)(M + 1) * 2 * (half + 1);
+    float *out = Rq + 9 * (size_t)(half + 1);
+    double *acc = reinterpret_cast<double *>(sm + iface_floats(M, nphi));
+    fill_cs(cs, M, half);
     for (int x = threadIdx.x; x < 3 * (M + 1); x += blockDim.x) acc[x] = 0.0;
     const float s2v = (float)slope_variance(o.wind, o.st), nw = (float)o.nw;
     const float muw = (float)gmu[iw], sw = (float)sqrt(fmax(0.0, 1.0 - gmu[iw] * gmu[iw]));
@@ -364,14 +376,16 @@ __global__ void k_couple_aw(const OceanPix *op, int P, const int *task0_a, const
     __syncthreads();
     for (int ja = 0; ja < N; ++ja) {
         const float mua = (float)gmu[ja], sa = (float)sqrt(fmax(0.0, 1.0 - gmu[ja] * gmu[ja]));
-        for (int q = threadIdx.x; q < nphi; q += blockDim.x) {
+        for (int q = threadIdx.x; q < half; q += blockDim.x) {
             const float phi = (q + 0.5f) * dphi;
-            float sp, cp;
+            float sp, cp, R[9];
             sincosf(phi, &sp, &cp);
-            taw_mueller(mua, sa, muw, sw, cp, sp, s2v, nw, o.qc, Rq + q * 9);
+            taw_mueller(mua, sa, muw, sw, cp, sp, s2v, nw, o.qc, R);
+#pragma unroll
+            for (int e = 0; e < 9; ++e) Rq[e * (half + 1) + q] = R[e];
         }
         __syncthreads();
-        project_block(Rq, cs, nphi, M, true, out);
+        project_block(Rq, cs, half, M, true, out);
         for (int x = threadIdx.x; x < 3 * (M + 1); x += blockDim.x) {
             const int m = x / 3, s = x - 3 * m;
             const double *eb = edge_a + ((size_t)(task0_a[o.pa] + m) * NRa + ja) * OCRT_EDGE;
@@ -446,11 +460,33 @@ __global__ void k_water_modes(OceanPix *op, int P, const PixDev *pxw, const int 
 // (the pass-3 bottom source, modes 0..min(M, m_nodes)), ja == NRa the view
 // (modes 0..m_nodes).  Results on the water solve's F_w scale (x F_w / pi),
 // which pass 3 carries to the TOA unchanged (rt_water_rt.c:7438-7440).
-__global__ void k_couple_wa(const OceanPix *op, int P, const PixDev *pxa, const PixDev *pxw, const int *task0_w,
-                            const double *gmu, int N, int NRa, int NRw, const double *edge_w, const double *glo,
-                            double *ext3, double *view)
+//
+// The field enters linearly through its two bracketing ring nodes, so the
+// quadrature nodes' matrices are first summed per ring node at every azimuth
+// (weights xi w (1 - t) and xi w t), and only the ring nodes' sums are
+// projected onto the modes and contracted with the field: about 35
+// projections per block instead of 1120.  Bound: FP32 issue of the Mueller
+// evaluations.  The quadrature nodes of one ring segment are consecutive, so
+// a thread (azimuth q, node class) keeps the segment's two sums of 9 entries
+// in registers; the node constants (FP64 differences, then FP32) are formed
+// once per block, as FP64 issues at 2 per clock and SM here.
+#define CWA_WIN 1024
+#define CWA_GLO 96
+#define CWA_NODES (CWA_WIN + CWA_GLO)
+#define CWA_GRP 4                                   // node classes (256 threads over 64 azimuths)
+size_t couple_wa_smem_bytes(int M, int NRw)
 {
-    const int ja = blockIdx.x, p = blockIdx.y;
+    return sizeof(double) * (3 * (size_t)(M + 1) + NRw) +
+           sizeof(float) * (iface_floats(M, 128) + 5 * (size_t)CWA_NODES + (size_t)CWA_GRP * 18 * 64 + 9 * 64) +
+           sizeof(int) * 3 * ((size_t)NRw + 1) + 16;
+}
+
+__global__ void __launch_bounds__(256)
+k_couple_wa(const OceanPix *op, int P, const PixDev *pxa, const PixDev *pxw, const int *task0_w,
+            const double *gmu, int N, int NRa, int NRw, const double *edge_w, const double *glo,
+            double *ext3, double *view)
+{
+    const int ja = blockIdx.x, p = blockIdx.y, tid = threadIdx.x;
     if (p >= P) return;
     const OceanPix &o = op[p];
     const PixDev &da = pxa[o.pa];
@@ -465,33 +501,41 @@ __global__ void k_couple_wa(const OceanPix *op, int P, const PixDev *pxa, const 
         mua = o.mu_va;
         M = o.m_nodes;
     }
-    const int nphi = 128, NWIN = 1024, NGLO = 96, NTOT = NWIN + NGLO;
-    extern __shared__ float sm[];
-    float *cs = sm;
-    float *Rq = cs + (size_t)(M + 1) * nphi * 2;
-    float *out = Rq + (size_t)nphi * 9;
-    double *acc = reinterpret_cast<double *>(out + (((M + 1) * 9 + 1) & ~1));
-    double *wmu = acc + 3 * (M + 1);                 // sorted unique water cosines
-    int *wsrc = reinterpret_cast<int *>(wmu + NRw);  // their ring slots
+    constexpr int half = 64;
+    extern __shared__ double smd[];
+    double *acc = smd;                               // [3 (M + 1)]
+    double *wmu = acc + 3 * (M + 1);                 // sorted unique water cosines [NRw]
+    float *cs = reinterpret_cast<float *>(wmu + NRw);
+    float *Rq = cs + (size_t)(M + 1) * 2 * (half + 1);
+    float *out = Rq + 9 * (half + 1);
+    float *nd = cs + iface_floats(M, 2 * half);      // [5][CWA_NODES]: mu, sine, shadowing, xi w (1 - t), xi w t
+    float *part = nd + 5 * CWA_NODES;                // [CWA_GRP][18][half]
+    float *carry = part + CWA_GRP * 18 * half;       // [9][half]: the next ring node's sum so far
+    int *wsrc = reinterpret_cast<int *>(carry + 9 * half);   // ring slots of wmu [NRw]
+    int *wbeg = wsrc + NRw, *gbeg = wbeg + NRw + 1;  // first window / Gauss node of each segment
+    __shared__ double srt[OCRT_MAX_N + OCRT_MAX_EXTRA];
+    __shared__ int sid[OCRT_MAX_N + OCRT_MAX_EXTRA];
     __shared__ int nu_s;
-    fill_cs(cs, M, nphi);
-    for (int x = threadIdx.x; x < 3 * (M + 1); x += blockDim.x) acc[x] = 0.0;
-    if (threadIdx.x == 0) {
-        const int n = dw.n_ring;
-        int ord[OCRT_MAX_N + OCRT_MAX_EXTRA];
-        for (int a = 0; a < n; ++a) ord[a] = a;
-        for (int a = 1; a < n; ++a) {
-            const int k = ord[a];
-            const double mk = ring_mu(dw, gmu, N, k);
-            int b = a - 1;
-            while (b >= 0 && ring_mu(dw, gmu, N, ord[b]) > mk) { ord[b + 1] = ord[b]; --b; }
-            ord[b + 1] = k;
+    fill_cs(cs, M, half);
+    for (int x = tid; x < 3 * (M + 1); x += blockDim.x) acc[x] = 0.0;
+    for (int x = tid; x < 9 * half; x += blockDim.x) carry[x] = 0.f;
+    const int n = dw.n_ring;
+    if (tid < n) {
+        const double mk = ring_mu(dw, gmu, N, tid);
+        int r = 0;
+        for (int b = 0; b < n; ++b) {
+            const double mb = ring_mu(dw, gmu, N, b);
+            r += (mb < mk || (mb == mk && b < tid)) ? 1 : 0;
         }
+        srt[r] = mk;
+        sid[r] = tid;
+    }
+    __syncthreads();
+    if (tid == 0) {
         int w = 0;
         for (int a = 0; a < n; ++a) {
-            const double m = ring_mu(dw, gmu, N, ord[a]);
-            if (w > 0 && fabs(m - wmu[w - 1]) < 1e-12) continue;
-            wmu[w] = m; wsrc[w] = ord[a]; ++w;
+            if (w > 0 && fabs(srt[a] - wmu[w - 1]) < 1e-12) continue;
+            wmu[w] = srt[a]; wsrc[w] = sid[a]; ++w;
         }
         nu_s = w;
     }
@@ -501,45 +545,98 @@ __global__ void k_couple_wa(const OceanPix *op, int P, const PixDev *pxa, const 
     double lo = mws - 0.30, hi = mws + 0.30;
     if (lo < 1e-6) lo = 1e-6;
     if (hi > 1.0 - 1e-9) hi = 1.0 - 1e-9;
-    const double hstep = (hi - lo) / (double)(NWIN - 1);
-    const float dphi = 6.28318530718f / (float)nphi;
+    const double hstep = (hi - lo) / (double)(CWA_WIN - 1);
+    auto node = [&](int i) -> double { return i < CWA_WIN ? lo + hstep * (double)i : glo[i - CWA_WIN]; };
     __syncthreads();
     const int nu = nu_s;
-    const double *ew = edge_w + (size_t)task0_w[o.pw] * NRw * OCRT_EDGE;
-    for (int i = 0; i < NTOT; ++i) {
-        double xi, wi;
-        if (i < NWIN) { xi = lo + hstep * (double)i; wi = ((i == 0 || i == NWIN - 1) ? 0.5 : 1.0) * hstep; }
-        else { xi = glo[i - NWIN]; wi = (xi > lo && xi < hi) ? 0.0 : glo[NGLO + i - NWIN]; }
-        if (wi == 0.0) continue;
-        const float sxi = (float)sqrt(fmax(0.0, 1.0 - xi * xi));
-        for (int q = threadIdx.x; q < nphi; q += blockDim.x) {
-            const float phi = (q + 0.5f) * dphi;
-            float sp, cp;
-            sincosf(phi, &sp, &cp);
-            twa_mueller((float)mua, sva, (float)xi, sxi, cp, sp, s2v, slen, nw, o.qc, Rq + q * 9);
+    // segment s holds the nodes with wmu[s] < xi <= wmu[s + 1]; the first and
+    // the last also what lies outside (the end pairs extrapolate)
+    for (int s = tid; s < nu; s += blockDim.x) {
+        int w = 0, g = 0;
+        if (s > 0 && s < nu - 1) {
+            const double v = wmu[s];
+            w = min(CWA_WIN, max(0, (int)floor((v - lo) / hstep) - 1));
+            while (w < CWA_WIN && !(node(w) > v)) ++w;
+            while (g < CWA_GLO && !(glo[g] > v)) ++g;
+        } else if (s == nu - 1) {
+            w = CWA_WIN; g = CWA_GLO;
         }
-        __syncthreads();
-        project_block(Rq, cs, nphi, M, true, out);
-        // linear interpolation (end pairs extrapolate) on the sorted ring
-        int hi_i = 1;
-        while (hi_i < nu && wmu[hi_i] < xi) hi_i++;
-        int lo_i = hi_i - 1;
-        if (hi_i >= nu) { hi_i = nu - 1; lo_i = nu - 2; }
-        if (lo_i < 0) { lo_i = 0; hi_i = 1; }
-        const double t = (xi - wmu[lo_i]) / (wmu[hi_i] - wmu[lo_i]);
-        for (int x = threadIdx.x; x < 3 * (M + 1); x += blockDim.x) {
-            const int m = x / 3, s = x - 3 * m;
-            const float *T = out + m * 9 + s * 3;
-            const double *ea = ew + ((size_t)m * NRw + wsrc[lo_i]) * OCRT_EDGE;
-            const double *eb = ew + ((size_t)m * NRw + wsrc[hi_i]) * OCRT_EDGE;
-            double v = 0.0;
-            for (int u = 0; u < 3; ++u) v += (double)T[u] * ((1.0 - t) * ea[u] + t * eb[u]);
-            acc[x] += (m == 0 ? 2.0 * OCRT_PI : OCRT_PI) * xi * wi * v;
-        }
-        __syncthreads();
+        wbeg[s] = w;
+        gbeg[s] = g;
     }
+    __syncthreads();
+    const float lama = sancer_f((float)mua, slen);
+    for (int i = tid; i < CWA_NODES; i += blockDim.x) {
+        const double xi = node(i);
+        const double wi = i < CWA_WIN ? ((i == 0 || i == CWA_WIN - 1) ? 0.5 : 1.0) * hstep
+                                      : ((xi > lo && xi < hi) ? 0.0 : glo[CWA_GLO + i - CWA_WIN]);
+        const int *beg = i < CWA_WIN ? wbeg : gbeg;
+        const int id = i < CWA_WIN ? i : i - CWA_WIN;
+        int a = 0, b = nu - 1;                       // beg[a] <= id < beg[b]
+        while (b - a > 1) { const int c = (a + b) >> 1; if (beg[c] <= id) a = c; else b = c; }
+        const float x = (float)xi, d0 = (float)(xi - wmu[a]), d1 = (float)(wmu[a + 1] - xi);
+        const float wx = x * (float)wi / (float)(wmu[a + 1] - wmu[a]);
+        nd[i] = x;
+        nd[CWA_NODES + i] = sqrtf(fmaxf(0.f, (float)(1.0 - xi) * (1.f + x)));
+        nd[2 * CWA_NODES + i] = 1.f / (1.f + sancer_f(x, slen) + lama);
+        nd[3 * CWA_NODES + i] = wx * d1;
+        nd[4 * CWA_NODES + i] = wx * d0;
+    }
+    __syncthreads();
+    const double *ew = edge_w + (size_t)task0_w[o.pw] * NRw * OCRT_EDGE;
+    // projection of ring node s from Rq and its contraction with the field
+    auto contract = [&](int s) {
+        project_block(Rq, cs, half, M, true, out);
+        for (int x = tid; x < 3 * (M + 1); x += blockDim.x) {
+            const int m = x / 3, r = x - 3 * m;
+            const float *T = out + m * 9 + r * 3;
+            const double *e = ew + ((size_t)m * NRw + wsrc[s]) * OCRT_EDGE;
+            const double v = (double)T[0] * e[0] + (double)T[1] * e[1] + (double)T[2] * e[2];
+            acc[x] += (m == 0 ? 2.0 * OCRT_PI : OCRT_PI) * v;
+        }
+    };
+    const int q = tid & (half - 1), grp = tid >> 6;
+    float sp, cp;
+    sincosf((q + 0.5f) * (3.14159265359f / (float)half), &sp, &cp);
+    for (int s = 0; s + 1 < nu; ++s) {
+        float a[9], b[9];
+#pragma unroll
+        for (int e = 0; e < 9; ++e) a[e] = b[e] = 0.f;
+        const int w0 = wbeg[s], nwin = wbeg[s + 1] - w0, g0 = gbeg[s], nn = nwin + gbeg[s + 1] - g0;
+        for (int k = grp; k < nn; k += CWA_GRP) {
+            const int i = k < nwin ? w0 + k : CWA_WIN + g0 + (k - nwin);
+            const float wa = nd[3 * CWA_NODES + i], wb = nd[4 * CWA_NODES + i];
+            if (wa == 0.f && wb == 0.f) continue;
+            float T[9];
+            twa_mueller((float)mua, sva, nd[i], nd[CWA_NODES + i], cp, sp, s2v, nd[2 * CWA_NODES + i], nw, o.qc, T);
+#pragma unroll
+            for (int e = 0; e < 9; ++e) { a[e] = fmaf(wa, T[e], a[e]); b[e] = fmaf(wb, T[e], b[e]); }
+        }
+#pragma unroll
+        for (int e = 0; e < 9; ++e) {
+            part[(grp * 18 + e) * half + q] = a[e];
+            part[(grp * 18 + 9 + e) * half + q] = b[e];
+        }
+        __syncthreads();
+        for (int x = tid; x < 9 * half; x += blockDim.x) {
+            const int e = x / half, qq = x - e * half;
+            float va = carry[x], vb = 0.f;
+#pragma unroll
+            for (int g = 0; g < CWA_GRP; ++g) {
+                va += part[(g * 18 + e) * half + qq];
+                vb += part[(g * 18 + 9 + e) * half + qq];
+            }
+            Rq[e * (half + 1) + qq] = va;
+            carry[x] = vb;
+        }
+        __syncthreads();
+        contract(s);
+    }
+    for (int x = tid; x < 9 * half; x += blockDim.x) Rq[(x / half) * (half + 1) + (x % half)] = carry[x];
+    __syncthreads();
+    contract(nu - 1);
     const double f = o.F_w / OCRT_PI;
-    for (int x = threadIdx.x; x < 3 * (M + 1); x += blockDim.x) {
+    for (int x = tid; x < 3 * (M + 1); x += blockDim.x) {
         if (ja < NRa) ext3[(size_t)o.ext_off + ((size_t)(x / 3) * NRa + ja) * 3 + (x % 3)] = f * acc[x];
         else view[(size_t)p * 3 * (OCRT_MAX_M + 1) + x] = f * acc[x];
     }
