@@ -608,7 +608,7 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
         (rc = alloc(g.Eatt, g.any_rough ? g.nlev * G.NR : 1)) || (rc = alloc(g.lvf, 3 * g.nlev)) ||
         (rc = alloc(g.lam, (size_t)g.P * (G.N + 2))) ||
         (rc = alloc(g.frs, (size_t)g.P * G.NR * 9)) ||
-        (rc = alloc(g.kappa, g.P)) || (rc = alloc(g.taudir, g.P)) ||
+        (rc = alloc(g.kappa, (size_t)g.P * (IPSS_SPLIT + 1))) || (rc = alloc(g.taudir, g.P)) ||
         (rc = alloc(g.active_cnt, (size_t)g.max_orders + 2)) || (rc = alloc(g.mol_cnt, (size_t)g.max_orders + 2)) ||
         (rc = alloc(g.work, 4 * ((size_t)g.max_orders + 2))) || (rc = alloc(g.err, 2)) ||
         (rc = alloc(g.alist[0], g.wave_tasks)) || (rc = alloc(g.alist[1], g.wave_tasks)) ||
@@ -1165,19 +1165,19 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
     if (g.any_pssa) {
         int maxnt = 0;
         for (const PixDev &d : g.hpx) maxnt = std::max(maxnt, d.nt);
-        const size_t smem = sizeof(double) * (6 * (size_t)maxnt + 6) + sizeof(int) * ((size_t)maxnt + 1);
-        LAUNCH(plan, KC_IPSS, k_ipss<<<P, 256, smem, st>>>(g.px, P, g.h, g.z, g.xd, g.yd,
+        const size_t smem = ipss_smem_bytes(maxnt);
+        LAUNCH(plan, KC_IPSS, k_ipss<<<dim3(IPSS_SPLIT, P), IPSS_THREADS, smem, st>>>(g.px, P, g.h, g.z, g.xd, g.yd,
                                                            g.any_gas ? g.tabs : nullptr, g.mb, g.vk_th, g.vk_p11,
                                                            g.kappa, g.taudir));
         if (g.any_lut)
-            LAUNCH(plan, KC_IPSS, k_ipss_lut<<<dim3(std::min(g.lut_ptmax, 2048), P), 256, smem, st>>>(
+            LAUNCH(plan, KC_IPSS, k_ipss_lut<<<dim3(std::min(g.lut_ptmax, 2048), P), IPSS_THREADS, smem, st>>>(
                        g.px, P, g.h, g.z, g.xd, g.yd, g.any_gas ? g.tabs : nullptr, g.mb, g.vk_th, g.vk_p11,
                        g.lut_vza, g.lut_raa, g.lut_kappa));
     }
     if (g.any_lut)
         LAUNCH(plan, KC_FINAL, k_lut_final<<<dim3((g.lut_ptmax + 127) / 128, P), 128, 0, st>>>(g.px, P, make_lut(g),
                                                                                               g.pix_task0));
-    LAUNCH(plan, KC_FINAL, k_finalize<<<(P + 127) / 128, 128, 0, st>>>(g.px, P, g.state, g.tout, g.gmu, g.gw, g.h,
+    LAUNCH(plan, KC_FINAL, k_finalize<<<(P + 3) / 4, 128, 0, st>>>(g.px, P, g.state, g.tout, g.gmu, g.gw, g.h,
                                                               g.kappa, g.taudir, g.res));
     return OCRT_OK;
 }
@@ -1218,6 +1218,7 @@ int ocrt_gb_init(int device)
     CK(cudaFuncSetAttribute(k_coxmunk_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(k_coxmunk_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     CK(cudaFuncSetAttribute(k_ipss, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CK(cudaFuncSetAttribute(k_ipss_lut, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(k_tables, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(tables_tc_init());
     CK(cudaFuncSetAttribute(k_value_pfm, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));

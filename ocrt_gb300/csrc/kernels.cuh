@@ -320,12 +320,17 @@ __global__ void k_extract(BatchBufs B, WaveBufs W, Geom G, int t0, int nt_tasks)
 __global__ void k_stop_check(const int *active_after_last, int *flag);
 
 // post.cu
+// blocks a pixel's line-of-sight nodes are spread over: 8 x 128 threads hold the
+// 800 nodes of 400 layers once
+#define IPSS_SPLIT 8
+#define IPSS_THREADS 128
+size_t ipss_smem_bytes(int nl);
 __global__ void k_ipss(const PixDev *px, int P, const double *h, const double *z,
                        const double *xd, const double *yd, const double *tabs,
-                       const double *mb, const double *vk_th, const double *vk_p11, double *kappa, double *tau_dir);
+                       const double *mb, const double *vk_th, const double *vk_p11, double *part, double *tau_dir);
 __global__ void k_finalize(const PixDev *px, int P, const TaskState *state, const TaskOut *tout,
                            const double *gmu, const double *gw, const double *h,
-                           const double *kappa, const double *tau_dir, ocrt_result *res);
+                           const double *kpart, const double *tau_dir, ocrt_result *res);
 
 // ocean.cu — coupled atmosphere-ocean solve
 #define OCRT_EDGE 12      // doubles per (task, ring slot) of k_edges

@@ -171,7 +171,7 @@ extern "C" int ocrt_gb_solve_case_noalloc(const ocrt_case *cs, const ocrt_opts *
     float *frs = cv.take<float>((size_t)NR * 9);
     const int La1 = aer ? aer->L_max + 1 : 1;
     double *mb = cv.take<double>(La1), *mg = cv.take<double>(La1), *ma = cv.take<double>(La1), *mz = cv.take<double>(La1);
-    double *kappa = cv.take<double>(1), *taudir = cv.take<double>(1);
+    double *kappa = cv.take<double>(IPSS_SPLIT + 1), *taudir = cv.take<double>(1);
     int *active = cv.take<int>((size_t)opts->max_orders + 2);
     int *molcnt = cv.take<int>((size_t)opts->max_orders + 2);
     int *work = cv.take<int>(4 * ((size_t)opts->max_orders + 2));
@@ -279,8 +279,7 @@ extern "C" int ocrt_gb_solve_case_noalloc(const ocrt_case *cs, const ocrt_opts *
         NA_LAUNCH(k_extract<<<(nw + 127) / 128, 128, 0, st>>>(B, W, G, t0, nw));
     }
     if (opts->pssa) {
-        const size_t smem = sizeof(double) * (6 * (size_t)nt + 6) + sizeof(int) * ((size_t)nt + 1);
-        NA_LAUNCH(k_ipss<<<1, 256, smem, st>>>(px, 1, h, z, xd, yd, opts->gas ? tabs : nullptr, mb, nullptr, nullptr,
+        NA_LAUNCH(k_ipss<<<dim3(IPSS_SPLIT, 1), IPSS_THREADS, ipss_smem_bytes(nt), st>>>(px, 1, h, z, xd, yd, opts->gas ? tabs : nullptr, mb, nullptr, nullptr,
                                                kappa, taudir));
     }
     NA_LAUNCH(k_finalize<<<1, 32, 0, st>>>(px, 1, state, tout, gmu, gw, h, kappa, taudir, res));
