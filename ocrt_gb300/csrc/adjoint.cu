@@ -744,8 +744,8 @@ __global__ void __launch_bounds__(512) k_adj_grad(BatchBufs B, WaveBufs W, AdjBu
         const double acc = accf;
         const double tdn = exp(-d.tau_total / d.mu0);
         const double fs = (tk.m == 0 ? OCRT_PI : 0.5 * OCRT_PI) * d.mu0;
-        const float *RsW = A.srfW + tk.srf_off + (size_t)G.NR * N * 9;
-        const float *Rs = W.srf + tk.srf_off + (size_t)G.NR * N * 9;
+        const float *RsW = A.srfW + tk.srf_off + G.srf_sun;
+        const float *Rs = W.srf + tk.srf_off + G.srf_sun;
         const double E = (double)B.Eatt[(d.lev_off + nt) * NR + g];
         const double sw = acc + fs * tdn * E * (double)RsW[g * 9 + s * 3];
         const double ss = fs * tdn * E * (double)Rs[g * 9 + s * 3];
@@ -838,8 +838,8 @@ __global__ void k_adj_pixel(BatchBufs B, WaveBufs W, AdjBufs A, Geom G, int p0, 
                 double w[3];
                 mode_weights(d, m, cot, w);
                 const double fs = (m == 0 ? OCRT_PI : 0.5 * OCRT_PI) * d.mu0;
-                const float *Rs = W.srf + tk.srf_off + (size_t)NR * N * 9;
-                const float *RsW = A.srfW + tk.srf_off + (size_t)NR * N * 9;
+                const float *Rs = W.srf + tk.srf_off + G.srf_sun;
+                const float *RsW = A.srfW + tk.srf_off + G.srf_sun;
                 for (int cc = 0; cc < nc; ++cc) {
                     const int gg = cols[cc];
                     const double mug = gg < N ? B.gmu[gg] : d.mu_view;

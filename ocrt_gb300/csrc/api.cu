@@ -338,6 +338,12 @@ struct Group {
     float *F = nullptr, *J = nullptr, *ops = nullptr;
     float *opt = nullptr;    // pre-split operator tiles of the tensor-core pass (2 x wave_ops floats)
     bool tabs_tc = false;    // phase tables on tcgen05 (k_tables_tc)
+    // every order of a task in one CTA (k_orders): parity operators and molecular
+    // row factors per wave task, task counters
+    bool fused = false;
+    unsigned char *popt = nullptr;
+    float *molc = nullptr;
+    int *ocnt = nullptr;
     bool keep_tot = false;   // keep the order totals at every level (set before build_group)
     float *gtab = nullptr;   // its Gauss bases in the chunk order (k_basis_perm)
     float *atab = nullptr;   // and the Gauss rows of its A tiles, split and swizzled
@@ -427,7 +433,7 @@ void free_group(Group &g)
                     g.ldt, g.lss, g.cot, g.lamd, g.ATot, g.gout, g.grad, g.dTc, g.dCa, g.dCb, g.srfW, g.AF, g.AJ,
                     g.Abc, g.Ast, g.acnt, g.awork, g.opsT, g.alcnt, g.aswork, g.adjlist[0], g.adjlist[1],
                     g.lut_vza, g.lut_raa, g.lut_samp, g.lut_kappa, g.lut_out, g.vk_th, g.vk_p11, g.vkV, g.gtab,
-                    g.atab, g.sprod, g.gcoef};
+                    g.atab, g.sprod, g.gcoef, g.popt, g.molc, g.ocnt};
     for (void *p : ptrs) dfree(p);
 }
 
@@ -533,12 +539,27 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
         g.any_pssa |= o.pssa != 0;
         g.hpx.push_back(d);
     }
+    // All orders in one kernel (k_orders) for forward groups whose shape it
+    // holds: faster at every size measured, from one pixel (24 streams, 40 layers:
+    // 0.71 ms a solve against 1.41) to 192 pixels at 32 streams and 200 layers
+    // (15.6 ms against 25.5).  An adjoint needs the order totals of every level
+    // in its own form, and a named scan, order-1 or source implementation keeps
+    // the separate passes.
+    int kmax = 0;
+    for (const PixDev &d : g.hpx) kmax = std::max(kmax, d.nt + 1);
+    g.fused = ncot == 0 && orders_supported(G, kmax) && !force_simt() &&
+              !getenv("OCRT_GB_SCAN") && !getenv("OCRT_GB_PRIMARY");
+    if (g.fused) {
+        g.G.srf_rp = (3 * G.NR + 31) & ~31;
+        g.G.srf_sun = 3 * G.N * g.G.srf_rp;
+    }
+    const size_t srf_elems = (size_t)g.G.srf_sun + (size_t)G.NR * 9;
     g.T = task;
     g.nlev = lev; g.ncoef = coef; g.nmom = mb.size();
     // ---- waves of whole pixels under the workspace budget ----
     const size_t budget = wave_budget_bytes();
     const size_t op_elems = (size_t)G.NP * G.CIN;
-    const bool tiles = tc_supported(G) && !force_simt();
+    const bool tiles = tc_supported(G) && !force_simt() && !g.fused;
     Wave w{0, 0, 0, 0, 0, 0, 0, 0, false, false};
     size_t bytes = 0;
     auto close = [&](int pend) {
@@ -555,12 +576,13 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
         const size_t K = d.nt + 1, nm = d.M + 1;
         const bool rough = (d.surface == 2 && d.wind > 0.0) || d.medium == 1;   // water: R_ww kernels
         const size_t pf = nm * K * G.LDC;
-        const size_t po = (nm + 2 * std::min<size_t>(nm, 3)) * op_elems;
-        const size_t ps = rough ? nm * ((size_t)G.NR * G.N * 9 + (size_t)G.NR * 9) : 0;
+        const size_t po = g.fused ? 0 : (nm + 2 * std::min<size_t>(nm, 3)) * op_elems;
+        const size_t ps = rough ? nm * srf_elems : 0;
         size_t pb = pf * 12 + po * (tiles ? 12 : 4) + ps * 4 + nm * (4 * G.LDC + 24 * G.NR + 3 * (1 + G.E) * (g.Lmax + 1)) * 4;
         if (ncot > 0)   // adjoint fields, dR/dW, per-task partials
             pb += (size_t)ncot * (pf * 12 + nm * (G.NR * 3 * 4 + sizeof(TaskState) + (3 * K + 4) * 8)) + ps * 4 +
                   nm * (size_t)2 * (G.CIN + 32) * ((G.COUT + 31) & ~31) * 4;
+        if (g.fused) pb += nm * (par_bytes(G) + OR_MOLC * 4);
         if (g.any_vk)   // the value kernel's tables of the pixel
             pb += (size_t)(g.Mmax + 1) * (G.N + 1) * 2 * G.NR * 4;
         if (q > w.p0 && bytes + pb > budget) {
@@ -572,14 +594,14 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
         for (size_t m = 0; m < nm; ++m) {
             tk[m].fld_off = (long long)w.fld; w.fld += K * G.LDC;
             tk[m].tail_off = (long long)w.tail; w.tail += 2 * (size_t)G.LDC;
-            tk[m].op_off = (long long)w.ops; w.ops += op_elems;
+            tk[m].op_off = (long long)w.ops; w.ops += g.fused ? 0 : op_elems;
             if (m <= 2) {
-                tk[m].mol_off = (long long)w.ops; w.ops += op_elems;
-                tk[m].uv_off = (long long)w.ops; w.ops += op_elems;
+                tk[m].mol_off = (long long)w.ops; w.ops += g.fused ? 0 : op_elems;
+                tk[m].uv_off = (long long)w.ops; w.ops += g.fused ? 0 : op_elems;
             } else {
                 tk[m].mol_off = tk[m].uv_off = -1;
             }
-            if (rough) { tk[m].srf_off = (long long)w.srf; w.srf += (size_t)G.NR * G.N * 9 + (size_t)G.NR * 9; }
+            if (rough) { tk[m].srf_off = (long long)w.srf; w.srf += srf_elems; }
             else tk[m].srf_off = -1;
             tk[m].has_mol = m <= 2;
         }
@@ -664,10 +686,13 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
     }
     if (g.smap_ok && g.ncot > 0 && g.AF && !adj_scan_column())
         g.amap_ok = adj_scan_tma_maps(G, g.AF, g.ATot, g.wave_fld * g.ncot, g.Cq, g.ncoef / G.NR, &g.amap) == 0;
-    g.use_tc = tc_supported(G) && !force_simt();
+    g.use_tc = tc_supported(G) && !force_simt() && !g.fused;
+    if (g.fused && ((rc = alloc(g.popt, (size_t)g.wave_tasks * par_bytes(G))) ||
+                    (rc = alloc(g.molc, (size_t)g.wave_tasks * OR_MOLC)) || (rc = alloc(g.ocnt, 2))))
+        return rc;
     if (g.use_tc && (rc = alloc(g.opt, 2 * g.wave_ops))) return rc;
     if (g.use_tc && (rc = alloc(g.molV, (size_t)3 * 32 * G.CIN))) return rc;
-    g.tabs_tc = g.use_tc && tables_tc_supported(G, g.Lmax) && !force_simt_tables();
+    g.tabs_tc = (g.use_tc || g.fused) && tables_tc_supported(G, g.Lmax, g.fused) && !force_simt_tables();
     if (g.tabs_tc && ((rc = alloc(g.gtab, tables_tc_gt_floats(G.N, g.Mmax, g.Lmax))) ||
                       (rc = alloc(g.atab, tables_tc_at_floats(g.Mmax, g.Lmax))) ||
                       (rc = alloc(g.sprod, (size_t)g.wave_tasks * G.N * 16))))
@@ -689,7 +714,7 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
         g.use_tc_adj = true;
     }
     for (Wave &w : g.waves) {
-        w.n_simt = g.use_tc ? 0 : w.t1 - w.t0;
+        w.n_simt = g.use_tc || g.fused ? 0 : w.t1 - w.t0;
         w.n_tc = g.use_tc ? w.t1 - w.t0 : 0;
         w.n_mol = 0;
         for (int t = w.t0; t < w.t1; ++t) w.n_mol += g.htask[t].has_mol ? 1 : 0;
@@ -924,7 +949,7 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
     const int poll = 4;
     // ---- transport-scan implementation: forced, tuned, or being tuned ----
     std::vector<int> scan_cands;
-    if (!g.Cq) {
+    if (!g.Cq || g.fused) {
         scan_cands.push_back(SK_COLUMN);
     } else {
         scan_cands.push_back(SK_QUAD);
@@ -962,7 +987,7 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
         // the plain operators are read only off the forward tensor-core path; the
         // molecular factors it reads are written in full by k_tables, and
         // k_tables_tc writes every row of the plain operator it keeps
-        if (!g.use_tc || (g.ncot > 0 && !g.tabs_tc)) CK(cudaMemsetAsync(g.ops, 0, sizeof(float) * w.ops, st));
+        if (!g.fused && (!g.use_tc || (g.ncot > 0 && !g.tabs_tc))) CK(cudaMemsetAsync(g.ops, 0, sizeof(float) * w.ops, st));
         CK(cudaMemsetAsync(g.pvec, 0, sizeof(float) * (size_t)nw * 2 * G.LDC, st));
         if (g.any_flat) CK(cudaMemsetAsync(g.fvec, 0, sizeof(float) * (size_t)nw * 24 * G.NR, st));
         CK(cudaMemsetAsync(g.active_cnt, 0, sizeof(int) * ((size_t)g.max_orders + 2), st));
@@ -975,7 +1000,7 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
             LAUNCH(plan, KC_TABLES, k_value_pfm<<<dim3(((G.N + 1) * 2 * G.NR + 127) / 128, w.p1 - w.p0), 128,
                                                   value_kernel_smem_bytes(g.vk_nmax), st>>>(
                        g.px, w.p0, G, g.gmu, g.vk_th, g.vk_p11, g.vkV, g.vk_stride));
-        const int plain_ops = (!g.use_tc || g.ncot > 0) ? 1 : 0;
+        const int plain_ops = !g.fused && (!g.use_tc || g.ncot > 0) ? 1 : 0;
         int rc = 0;
         if (g.tabs_tc) {
             // the aerosol operator and the sun-outgoing products on tcgen05, then
@@ -983,17 +1008,20 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
             LAUNCH(plan, KC_TABLES, k_tables_tc<<<std::min(nw, g_nsm), tables_tc_threads(),
                                                   tables_tc_smem_bytes(G, g.Lmax), st>>>(
                        g.tasks, w.t0, nw, g.px, G, g.Lmax, g.gtab, g.atab, g.Bx, g.gw, g.mb, g.mg, g.ma, g.mz, g.ops, W.opt,
-                       plain_ops, g.any_vk ? g.vkV : nullptr, w.p0, g.vk_stride, g.sprod, g.err));
+                       plain_ops, g.any_vk ? g.vkV : nullptr, w.p0, g.vk_stride, g.sprod, g.err, g.popt, g.Bp, g.Br, g.Bt));
             LAUNCH(plan, KC_TABLES, k_tables<<<dim3(nw, 1), 64, tables_smem_bytes(64, G.N, g.Lmax), st>>>(
                        g.tasks, w.t0, nw, g.px, G, g.Lmax, g.Bp, g.Br, g.Bt, g.Bx, g.gw, g.mb, g.mg, g.ma, g.mz,
                        g.ops, g.pvec, W.fvec, W.opt, plain_ops, g.any_vk ? g.vkV : nullptr, w.p0, g.vk_stride,
-                       g.sprod));
+                       g.sprod, g.molc, g.popt));
         } else {
             auto tables = [&](int b) {
                 k_tables<<<dim3(nw, tables_yblocks(b, G.NR, G.N)), b, tables_smem_bytes(b, G.N, g.Lmax), st>>>(
                     g.tasks, w.t0, nw, g.px, G, g.Lmax, g.Bp, g.Br, g.Bt, g.Bx, g.gw, g.mb, g.mg, g.ma, g.mz, g.ops,
-                    g.pvec, W.fvec, W.opt, plain_ops, g.any_vk ? g.vkV : nullptr, w.p0, g.vk_stride, nullptr);
+                    g.pvec, W.fvec, W.opt, plain_ops, g.any_vk ? g.vkV : nullptr, w.p0, g.vk_stride, nullptr, g.molc,
+                    g.popt);
             };
+            // the rows and columns of the parity operator that no pair writes
+            if (g.fused) CK(cudaMemsetAsync(g.popt, 0, (size_t)nw * par_bytes(G), st));
             int tb = 256;
             rc = tuned_block("k_tables", (const void *)k_tables, {G.N, g.Lmax, g.Mmax}, !capture, st, tables, &tb);
             if (rc) return rc;
@@ -1042,7 +1070,13 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
         const int tc_grid = std::min(w.n_tc * mtiles, g_nsm);
         const int mol_grid = std::min(w.n_mol * ltiles, 4 * g_nsm);
         const int scan_grid = std::min(nw, 8 * g_nsm), scan4_grid = std::min(nw, 16 * g_nsm);
-        if (w.any_top) {
+        const int or_grid = std::min(nw, g_nsm);
+        if (g.fused) LAUNCH(plan, KC_SCAN, k_orders_reset<<<1, 32, 0, st>>>(g.ocnt));
+        if (w.any_top && g.fused) {
+            // skylight first-scatter source of the water column (see below)
+            LAUNCH(plan, KC_PRIMARY, k_dtop_field<<<nw, 256, 0, st>>>(B, W, G, w.t0));
+            LAUNCH(plan, KC_SOURCE_TC, orders_launch(true, or_grid, st, B, W, G, w.t0, nw, w.Kmax, g.popt, g.molc, g.ocnt));
+        } else if (w.any_top) {
             // skylight first-scatter source of the water column: the source pass
             // over the unscattered skylight field, every task active, into J
             const int itd = g.max_orders + 1;
@@ -1062,8 +1096,11 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
             LAUNCH(plan, KC_PRIMARY, k_primary4<<<nw, scan4_threads(G), 0, st>>>(B, W, G, w.t0));
         else
             LAUNCH(plan, KC_PRIMARY, k_primary<<<nw, scan_threads, 0, st>>>(B, W, G, w.t0));
-        LAUNCH(plan, KC_PRIMARY, k_compact<<<1, COMPACT_THREADS, 0, st>>>(B, w.t0, nw, 2));
-        for (int it = 2; it <= g.max_orders; ++it) {
+        if (g.fused)
+            LAUNCH(plan, KC_SOURCE_TC, orders_launch(false, or_grid, st, B, W, G, w.t0, nw, w.Kmax, g.popt, g.molc, g.ocnt + 1));
+        else
+            LAUNCH(plan, KC_PRIMARY, k_compact<<<1, COMPACT_THREADS, 0, st>>>(B, w.t0, nw, 2));
+        for (int it = 2; !g.fused && it <= g.max_orders; ++it) {
             if (w.n_simt)
                 LAUNCH(plan, KC_SOURCE, k_source_simt<<<sgrid, 256, 0, st>>>(B, W, G, w.t0, it));
             if (w.n_tc)
@@ -1225,6 +1262,7 @@ int ocrt_gb_init(int device)
     CK(cudaFuncSetAttribute(k_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(k_scan4, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(scan_tma_init());
+    CK(orders_init());
     CK(cudaFuncSetAttribute(k_adj_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(k_source_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     CK(cudaFuncSetAttribute(k_source_tc_xs, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
@@ -1486,10 +1524,10 @@ int ocrt_gb_plan_kernel_stats(ocrt_plan *plan, int cls, const char **name, doubl
                 const TaskDev &tk = g.htask[t];
                 const PixDev &d = g.hpx[tk.pix];
                 const double K = tk.K, nt = d.nt, ords = std::max(0, st[t].orders - 1);
-                const int sc = g.use_tc ? KC_SOURCE_TC : KC_SOURCE;
+                const int sc = g.use_tc || g.fused ? KC_SOURCE_TC : KC_SOURCE;
                 plan->flops[sc] += ords * 72.0 * N * N * K;
                 plan->bytes[sc] += ords * (K * 6 * N + K * 6 * NR + 36.0 * N * NR) * 4.0;
-                if (tk.has_mol && g.use_tc) {          // dense U V inside the tensor-core pass
+                if (tk.has_mol && (g.use_tc || g.fused)) {          // dense U V inside the tensor-core pass
                     plan->flops[KC_SOURCE_TC] += ords * 72.0 * N * N * K;
                     plan->bytes[KC_SOURCE_TC] += ords * (36.0 * N * NR) * 4.0;
                 } else if (tk.has_mol) {               // rank-24 form on CUDA cores

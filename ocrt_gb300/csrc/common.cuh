@@ -103,7 +103,24 @@ struct Geom {
     // the coupled ocean reads level 1); 0: only at the TOA and BOA output
     // levels, the interior ones neither read nor written
     int tot_all;
+    // Rough-surface kernels of a task: the Gauss part, then at srf_sun the sun
+    // column [NR][9].  srf_rp 0: [o][i][9]; else the row form [3 i-Stokes][N][srf_rp]
+    // with the outgoing rows contiguous (surface row so * N + o, zero-weight
+    // slots 3N + 3 (o - N) + so), which the fused order kernel reads coalesced.
+    int srf_rp, srf_sun;
 };
+
+__host__ __device__ inline int srf_row(const Geom &G, int o, int so)
+{
+    return o < G.N ? so * G.N + o : 3 * G.N + 3 * (o - G.N) + so;
+}
+
+// Entry e = 3 so + si of the kernel from Gauss slot i to ring slot o.
+__host__ __device__ inline size_t srf_entry(const Geom &G, int o, int i, int e)
+{
+    if (G.srf_rp == 0) return ((size_t)o * G.N + i) * 9 + e;
+    return ((size_t)(e % 3) * G.N + i) * G.srf_rp + srf_row(G, o, e / 3);
+}
 
 __host__ __device__ inline Geom make_geom(int N, int E = 1)
 {
@@ -119,6 +136,8 @@ __host__ __device__ inline Geom make_geom(int N, int E = 1)
     g.LDC = (g.COUT + 31) & ~31;
     g.NP = (g.COUT + 15) & ~15;
     g.tot_all = 1;
+    g.srf_rp = 0;
+    g.srf_sun = g.NR * N * 9;
     return g;
 }
 
@@ -188,6 +207,66 @@ __host__ __device__ inline float round_tf32f(float v)
     unsigned u; memcpy(&u, &v, 4); u = (u + 0x1000u) & 0xFFFFE000u; float r; memcpy(&r, &u, 4); return r;
 #endif
 }
+
+#ifdef __CUDACC__
+// A pair of FP32 values as three packed bf16 pairs v = p0 + p1 + p2 (each
+// piece rounded to nearest from what the earlier ones left, so the residual is
+// below 2^-25 of the value); low half = a, high half = b.
+__device__ __forceinline__ void split_bf16x3(float a, float b, uint32_t *p)
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p[i]) : "f"(b), "f"(a));
+        if (i < 2) {
+            a -= __uint_as_float(p[i] << 16);
+            b -= __uint_as_float(p[i] & 0xffff0000u);
+        }
+    }
+}
+#endif
+
+// Parity operator of the fused order kernel (orders.cu), per task: for each
+// incoming Stokes component (chunk) and each bf16 piece a K-major
+// SWIZZLE_128B tile of par_rows rows x 64 columns; column 32 parity + i.
+__host__ __device__ inline int par_rows(const Geom &g) { return (3 * g.NR + 3 + 7) & ~7; }
+__host__ __device__ inline size_t par_bytes(const Geom &g) { return (size_t)9 * par_rows(g) * 128; }
+// byte offset of column pair (col even) of a row inside one tile
+__host__ __device__ inline uint32_t par_swz(int row, int col)
+{
+    return (uint32_t)row * 128u + ((uint32_t)((col >> 3) ^ (row & 7)) << 4) + (uint32_t)(col & 7) * 2u;
+}
+
+#ifdef __CUDACC__
+// Entries of one parity block for an outgoing and an incoming slot, [out s][in s]:
+// X the pair sums (numbering of k_tables) over the l with this parity of l + m,
+// Y those over the others.
+__device__ __forceinline__ void par_coefs(const float *X, const float *Y, float *c)
+{
+    c[0] = X[0];  c[1] = X[10];         c[2] = -X[9];
+    c[3] = X[1];  c[4] = Y[3] + X[4];   c[5] = -(X[5] + Y[6]);
+    c[6] = -X[2]; c[7] = -(X[11] + Y[12]); c[8] = X[7] + Y[8];
+}
+// Molecular functional f of incoming I, Q, U (l = 2 bases P, R, T of the slot):
+// xi_A = b2 P.I + g2 (R.Q - T.U), xi_B = g2 P.I + a2 (R.Q - T.U), xi_0 = 1.I (m = 0)
+__device__ __forceinline__ void par_functional(int f, int m, double depol, float P, float R, float T, float *c)
+{
+    const double A = 2.0 * (1.0 - depol) / (2.0 + depol);
+    const float b2 = (float)(0.5 * A), g2 = (float)(-A * sqrt(1.5)), a2 = (float)(3.0 * A);
+    const float cp = f == 0 ? b2 : g2, cr = f == 0 ? g2 : a2;
+    c[0] = f == 2 ? (m == 0 ? 1.f : 0.f) : cp * P;
+    c[1] = f == 2 ? 0.f : cr * R;
+    c[2] = f == 2 ? 0.f : -cr * T;
+}
+// one entry (times the quadrature weight) into a task's tiles
+__device__ __forceinline__ void par_put(unsigned char *P, const Geom &g, int si, int row, int col, float v)
+{
+    uint32_t p[3];
+    split_bf16x3(v, 0.f, p);
+    for (int q = 0; q < 3; ++q)
+        *reinterpret_cast<uint16_t *>(P + (size_t)(3 * si + q) * par_rows(g) * 128 + par_swz(row, col & ~1) +
+                                      2 * (col & 1)) = (uint16_t)p[q];
+}
+#endif
 
 // Operator entry (row, cin) into the pre-split tensor-core tiles of one
 // operator: per 32-column K tile kt, a tf32 hi tile then a lo tile of NP rows

@@ -323,8 +323,8 @@ k_coxmunk_tc(const TaskDev *tasks, const PixDev *px, int p0, const int *pix_task
         const float ca = live ? pf[2 * pp] : 0.f, cb = live ? pf[2 * pp + 1] : 0.f;
         // normalisation x2 (half grid) x dphi / (2 pi) for m = 0 and dphi / pi for m > 0
         const float scale0 = 2.f / (float)nphi, scale1 = 4.f / (float)nphi;
-        const size_t offp = i < N ? ((size_t)o * N + i) * 9 + e : (size_t)G.NR * N * 9 + (size_t)o * 9 + e;
-        const size_t offt = ((size_t)i * N + o) * 9 + et;
+        const size_t offp = i < N ? srf_entry(G, o, i, e) : (size_t)G.srf_sun + (size_t)o * 9 + e;
+        const size_t offt = i < N && o < N ? srf_entry(G, i, o, et) : 0;
         const uint32_t tb = tmem + ((uint32_t)(warp * 32) << 16);
         for (int cb16 = 0; cb16 < NN / 16; ++cb16) {
             float v[16], vt[16];

@@ -70,23 +70,27 @@ __global__ void k_tables(const TaskDev *tasks, int t0, int nt_tasks, const PixDe
                          const double *gw,
                          const double *mb, const double *mg, const double *ma, const double *mz,
                          float *ops, float *pvec, float *fvec, float *opt, int plain,
-                         const float *V, int vp0, long long vstride, const float *sprod);
+                         const float *V, int vp0, long long vstride, const float *sprod, float *molc = nullptr,
+                         unsigned char *popt = nullptr);
+#define OR_MOLC 128     // floats per wave task of the molecular row factors (molc)
 // tables_tc.cu: phase tables and the aerosol operator tiles with the sums over
 // l on tcgen05 (the pair part of k_tables; k_tables then runs with sprod for
 // the molecular operator and the solar row).  GT: the Gauss bases in the chunk
 // order, AT: the Gauss rows of the A tiles split and swizzled (k_basis_perm,
-// grid (blocks, M + 1)); sprod[task][N][16]: the S and D sums of the eight
+// grid (blocks, M + 1)).  popt: the parity operator of the fused order kernel
+// instead of the tiles opt and the plain operator; sprod[task][N][16]: the S and D sums of the eight
 // sun-outgoing products of every Gauss slot.
 __global__ void k_basis_perm(int N, int M, int L, const float *Bp, const float *Br, const float *Bt, float *GT,
                              float *AT);
 __global__ void k_tables_tc(const TaskDev *tasks, int t0, int nt_tasks, const PixDev *px, Geom G, int L,
                             const float *GT, const float *AT, const float *Bx, const double *gw, const double *mb,
                             const double *mg, const double *ma, const double *mz, float *ops, float *opt, int plain,
-                            const float *V, int vp0, long long vstride, float *sprod, int *err);
+                            const float *V, int vp0, long long vstride, float *sprod, int *err, unsigned char *popt,
+                            const float *Bp, const float *Br, const float *Bt);
 size_t tables_tc_smem_bytes(const Geom &G, int L);
 size_t tables_tc_gt_floats(int N, int M, int L);
 size_t tables_tc_at_floats(int M, int L);
-bool tables_tc_supported(const Geom &G, int L);
+bool tables_tc_supported(const Geom &G, int L, bool parity);
 int tables_tc_threads();
 cudaError_t tables_tc_init();
 // value.cu: the aerosol value kernel's I-I tables V[pixel - p0][m][row][column]
@@ -379,3 +383,13 @@ inline size_t iface_smem_bytes(int M, int nphi, int extra_doubles)
     return sizeof(float) * iface_floats(M, nphi) + sizeof(double) * (size_t)extra_doubles;
 }
 size_t couple_wa_smem_bytes(int M, int NRw);
+
+// orders.cu: every order of a task in one CTA (parity operator popt from
+// k_tables_tc, molecular row factors molc[wave task][128] from k_tables)
+bool orders_supported(const Geom &G, int Kmax);
+size_t orders_smem_bytes(const Geom &G, int Kmax);
+cudaError_t orders_init();
+// source: k_orders_source (the source of the field at hand into J), else k_orders
+void orders_launch(bool source, int grid, cudaStream_t st, const BatchBufs &B, const WaveBufs &W, const Geom &G, int t0,
+                   int nw, int Kmax, const unsigned char *popt, const float *molc, int *counter);
+__global__ void k_orders_reset(int *counter);

@@ -93,7 +93,7 @@ __global__ void k_lut_sample(BatchBufs B, WaveBufs W, LutBufs Lb, Geom G, int t0
     }
     const float fs_tdn = d.rough ? (float)((tk.m == 0 ? OCRT_PI : 0.5 * OCRT_PI) * d.mu0 *
                                            exp(-d.tau_total / d.mu0)) : 0.f;
-    const float *Rs = d.rough ? W.srf + tk.srf_off + (size_t)G.NR * G.N * 9 : nullptr;
+    const float *Rs = d.rough ? W.srf + tk.srf_off + G.srf_sun : nullptr;
     for (int j = threadIdx.x; j < n; j += blockDim.x) {
         int slot;
         if (vpos < 0) slot = j;

@@ -217,7 +217,7 @@ __global__ void k_edges(BatchBufs B, WaveBufs W, Geom G, int t0, int nw, double 
     for (int s = 0; s < 3; ++s) {
         double u = tot_value(W, tk, G, 0, nt, col_of(G, s, 0, g));
         if (seed) {
-            const float *Rs = W.srf + tk.srf_off + (size_t)G.NR * G.N * 9;
+            const float *Rs = W.srf + tk.srf_off + G.srf_sun;
             u -= (double)(fs_tdn * B.Eatt[(d.lev_off + 0) * G.NR + g] * Rs[g * 9 + s * 3]);
         }
         e[s] = u;
@@ -269,7 +269,7 @@ __global__ void k_rww(const TaskDev *tasks, const PixDev *px, int p0, const int 
         for (int x = threadIdx.x; x < (M + 1) * 9; x += blockDim.x) {
             const int m = x / 9, e = x - 9 * m;
             const TaskDev tk = tasks[pix_task0[p] + m];
-            srf[tk.srf_off + ((size_t)o * N + i) * 9 + e] = out[x];
+            srf[tk.srf_off + srf_entry(G, o, i, e)] = out[x];
         }
         __syncthreads();
     }

@@ -1,0 +1,749 @@
+// orders.cu — the successive orders of a task (pixel, Fourier mode) in one
+// persistent kernel: source contraction on tcgen05 (rt_sos_operator.c:206-424),
+// surface boundary condition (rt_surface_boundary.c:137-208), linear-in-tau
+// transport (rt_layer_transport.c:107-208), order totals and the convergence
+// test (rt_solver.c:2178-2197, 2923-3150), order after order without leaving
+// the CTA.
+//
+// Tasks are independent, and what an order of a task reads is small: its
+// operator (120 KB here) and its field (33 x 6 columns x levels).  Sweeping one
+// order over all tasks at a time (k_source_tc, k_scan_tma) reads both from HBM
+// and writes the source J for the scan to read back, about 1.1 MB per task and
+// order at 200 levels.  Here a CTA takes a task through all of its orders: the
+// operator sits in shared memory, the field makes its round trip through L2,
+// the source never leaves tensor memory, and there are no per-order launches,
+// lists or host polls.
+//
+// Parity form.  Mirroring the hemispheres (up <-> down, U -> -U) leaves the
+// phase operator unchanged, so with F+- = F_up +- sigma F_dn (sigma = 1, 1, -1
+// for I, Q, U) it splits into two blocks of half the size:
+//     D+- = A+- (x F+-),  J_up = D+ + D-,  J_dn = sigma (D+ - D-)
+// (x the aerosol fraction of the level; with a molecular term, m <= 2, it is
+// applied to J instead),
+// half the multiplications and half the operator.  A+- are the even- and
+// odd-(l + m) sums of the phase tables.  Operands are three bf16 pieces each
+// (split_bf16x3) and six products (all but those below 2^-26): FP32-level
+// accuracy at the cost of 3xTF32 in tensor time and 3/4 of its shared memory.
+// Per task: D+-[row][level] (FP32 in TMEM), rows = 3N Gauss outputs (s, g), 3E
+// zero-weight outputs and, for m <= 2, three molecular functionals (xi_A, xi_B,
+// xi_0), which give the molecular source as row factor x xi.
+//
+// Measured, 192 pixels x 17 modes at 32 streams and 200 levels (32420
+// order-modes, rough surface, aerosol): 6.7 ms for all orders against 16.7 ms
+// of source and scan passes; 24 streams, which the tensor-core source does not
+// take, 3.7 ms against 19 ms of CUDA-core source, molecular and scan passes; one
+// pixel at 400 levels 0.38 ms against 1.4 ms.  What bounds it is an order's serial
+// chain (field rows back from L2, split, three stages of MMA per tile, recurrence,
+// boundary, residual): about 39 000 cycles at 265 levels where the MMAs alone
+// take 13 000 (1440 per tile and component) and the recurrence 8 500 (32 per
+// level); with one task a CTA these overlap only within the task.
+// Against FP64 solves (240 pixels, 24 streams) the reflectance error is 9.3e-7
+// rms, 9.4e-7 with FP32 CUDA-core products.
+//
+// Levels run along the MMA's N, so a thread of a scan warp owns one output row
+// and finds the levels of its recurrence in consecutive TMEM columns.  Tiles
+// of 112 levels arrive in the order 0, T-1, 1, T-2, ...: the downward scan
+// starts at the top and the upward one at the bottom while the other tiles are
+// still being multiplied.  Two tiles fit in TMEM; a tile a scan cannot use yet
+// is kept if no later tile needs its place, else its source rows go to J.
+//
+// Roles (16 warps, one CTA per SM; four warps per scheduler, so 128 registers a
+// thread):
+//   warps 0-3    upward scan (TMEM lane quadrant = warp), boundary condition
+//   warps 4-7    downward scan
+//   warps 8-14   producers, 16 levels each: field rows of a tile and one incoming Stokes
+//                component (loaded a stage ahead) -> F+-, split, swizzled
+//                K-major B tile (128-byte rows: [F+ 32 | F- 32]) of a 2-stage ring
+//   warp 15      loads the task's operator (one bulk copy), issues the MMAs
+// Thread 0 fetches tasks and posts one command per order (continue, new task,
+// stop) when the order's field is complete.
+//
+// Every wait is bounded (TC_WAIT_NS): a warp whose wait runs out raises the
+// abort flag and goes on through the same barriers; all roles leave at the next
+// order, record OCRT_ERR_DEVICE and free TMEM.
+#include <cuda.h>
+#include <cstdint>
+#include "kernels.cuh"
+#include "tcgen05.cuh"
+
+using namespace tcg;
+
+#define OR_TS 112                     // levels of a tile
+#define OR_THREADS 512
+#define OR_GRP 16                     // levels per TMEM load
+#define OR_BPIECE (OR_TS * 128)       // bytes of one bf16 piece of a B stage
+#define OR_BSTAGE (3 * OR_BPIECE)
+
+size_t orders_smem_bytes(const Geom &G, int Kmax)
+{
+    const size_t kp = (Kmax + OR_GRP + 3) & ~3;
+    return par_bytes(G) + 2 * (size_t)OR_BSTAGE + 2 * kp * 4 + 2 * 2 * 3 * OR_TS * 4 + 3 * 128 * 4 + 2 * 8 * 8 + 128;
+}
+
+namespace {
+
+__device__ __forceinline__ void or_bar(int id, int n)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+
+// Tile of arrival a of T: 0, T-1, 1, T-2, ...
+__device__ __forceinline__ int or_tile(int a, int T) { return (a & 1) ? T - 1 - (a >> 1) : a >> 1; }
+
+// What a scan thread reads: its row's factors and where its rows lie.
+struct Scan {
+    float T, Ca, Cb;                  // transport weights of a uniform column
+    // The downward source of U is -x (D+ - D-): the sign sg sits in the weights
+    // Ca, Cb and in what the source-only pass writes.
+    float sg;
+    float cm, c0;                     // molecular row factors of xi_A / xi_B and xi_0
+    const float *xs, *ys;             // aerosol / molecular fractions per level
+    const float *wT, *wA, *wB;        // per-layer weights of the slot (non-uniform columns)
+    float *F, *Js;                    // field and source-spill columns
+    int nt, NR;
+    bool st, ok, uni, mol;            // row stored in the field; row valid; uniform column; m <= 2
+};
+// and what it carries along its column: radiance, source of the level before, max |I|
+struct Col { float I, Jp, mi; };
+
+enum { OR_SCAN, OR_SPILL, OR_FROM_J };
+
+// A tile of n levels from k0 in direction H (0: from the bottom up), 16 levels
+// at a time: the source from TMEM at t (D+ at columns 0.., D- at 128..) or
+// (OR_FROM_J) from a tile spilled before, then the recurrence, or (OR_SPILL) the
+// source to J.  Groups that lie wholly inside a uniform column take a form
+// without masks.  There is one copy of this code per direction, and it is kept
+// short: the SM's instruction cache has to hold the loops of all roles (with
+// the cases specialised the kernel was 200 KB and every loop ran at an eighth
+// of its issue rate).
+template <int H, int LDC>
+__device__ __forceinline__ void or_tile_run(const Scan &c, Col &v, int what, uint32_t t, int k0, int n, float ssg,
+                                            const float *xa, const float *x0)
+{
+    const int nt = c.nt, ng = (n + 15) >> 4;
+    const float T0 = c.T, A0 = c.Ca, B0 = c.Cb;
+    float I = v.I, Jp = v.Jp, mi = v.mi;
+#pragma unroll 1
+    for (int q = 0; q < ng; ++q) {
+        // opaque to the compiler: left loop-invariant, these conditions would be
+        // unswitched into a copy of the loop per combination
+        int w = what, mol = c.mol, uni = c.uni;
+        asm volatile("" : "+r"(w), "+r"(mol), "+r"(uni));
+        const int gb = 16 * (H == 0 ? ng - 1 - q : q), kb = k0 + gb, nv = nt - kb;   // levels kb .. kb + min(15, nv) exist
+        float J[16];
+        if (w == OR_FROM_J) {
+            const float *p = c.Js + (size_t)kb * LDC;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) J[i] = c.ok && i <= nv ? p[i * LDC] : 0.f;
+        } else {
+            uint32_t P[16], M[16];
+            tmem_ld16_async(t + gb, P);
+            tmem_ld16_async(t + 128 + gb, M);
+            tmem_ld_wait(P, M);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float pv = __uint_as_float(P[i]), mv = __uint_as_float(M[i]);
+                J[i] = H == 0 ? pv + mv : pv - mv;
+            }
+            if (mol) {
+#pragma unroll
+                for (int i = 0; i < 16; i += 4) {
+                    const float4 x = *reinterpret_cast<const float4 *>(c.xs + kb + i);
+                    const float4 y = *reinterpret_cast<const float4 *>(c.ys + kb + i);
+                    const float4 e = *reinterpret_cast<const float4 *>(xa + gb + i);
+                    const float4 z = *reinterpret_cast<const float4 *>(x0 + gb + i);
+                    J[i] = fmaf(y.x, fmaf(c.cm, e.x, c.c0 * z.x), x.x * J[i]);
+                    J[i + 1] = fmaf(y.y, fmaf(c.cm, e.y, c.c0 * z.y), x.y * J[i + 1]);
+                    J[i + 2] = fmaf(y.z, fmaf(c.cm, e.z, c.c0 * z.z), x.z * J[i + 2]);
+                    J[i + 3] = fmaf(y.w, fmaf(c.cm, e.w, c.c0 * z.w), x.w * J[i + 3]);
+                }
+            }
+        }
+        // the group's values first, then its stores off one base address: a
+        // store still reading its registers would hold up the next level's step
+        float *dst = (w == OR_SPILL ? c.Js : c.F) + (size_t)kb * LDC;
+        int last = c.st ? nv : -1;                         // levels kb .. kb + last are stored
+        if (w == OR_SPILL) {
+            last = c.ok ? nv : -1;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) J[i] *= ssg;
+        } else if (uni && kb > 0 && nv > 15) {
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                const int i = H == 0 ? 15 - r : r;
+                const float j = J[i];
+                I = fmaf(T0, I, fmaf(A0, j, B0 * Jp));
+                Jp = j;
+                mi = fmaxf(mi, fabsf(I));
+                J[i] = I;
+            }
+        } else {
+            // the column's ends (its first level holds the start value, levels
+            // past the last one do not step), or weights by layer (k of level k
+            // upward, k - 1 downward): only the levels lo .. hi of the group step
+            const int lo = H == 1 && kb == 0 ? 1 : 0, hi = H == 0 ? nv - 1 : nv;
+            const int e0 = (H == 0 ? kb : kb - 1) * c.NR;
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                const int i = H == 0 ? 15 - r : r;
+                const bool step = i >= lo && i <= hi;
+                float T = T0, A = A0, Bw = B0;
+                if (!uni && step) {
+                    const int e = e0 + i * c.NR;
+                    T = __ldg(c.wT + e); A = c.sg * __ldg(c.wA + e); Bw = c.sg * __ldg(c.wB + e);
+                }
+                const float j = J[i], In = fmaf(T, I, fmaf(A, j, Bw * Jp));
+                I = step ? In : I;
+                Jp = j;
+                mi = fmaxf(mi, fabsf(I));
+                J[i] = I;
+            }
+        }
+        if (last >= 15) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) dst[i * LDC] = J[i];
+        } else {
+#pragma unroll
+            for (int i = 0; i < 15; ++i)
+                if (i <= last) dst[i * LDC] = J[i];
+        }
+    }
+    v.I = I; v.Jp = Jp; v.mi = mi;
+}
+
+struct Bars { uint64_t *bfull, *bempty, *tfull, *tempty, *order, *op, *fin; volatile int *abort; };
+
+__device__ __noinline__ void or_wait_slow(uint64_t *bar, uint32_t parity, volatile int *abort)
+{
+    if (*abort) return;
+    if (!mbar_wait(bar, parity)) *abort = 1;
+}
+__device__ __forceinline__ void or_wait(const Bars &b, uint64_t *bar, uint32_t parity)
+{
+    if (!mbar_try_wait(bar, parity)) or_wait_slow(bar, parity, b.abort);
+}
+
+// One order of the scan warps of direction H: every tile in arrival order.
+// SRC: the source only, every tile to J.  U: arrivals before this order.  xi:
+// this direction's functional buffers.
+template <int H, bool SRC, int LDC>
+__device__ __forceinline__ Col or_order(const Scan &c, Col v, const Bars &b, uint32_t tmem, int T, int K, uint32_t U,
+                                        float *xi, int f0, int row, int lane, int quad, bool par_odd, bool rowB)
+{
+    int next = H == 0 ? T - 1 : 0, held = -1, a = 0;
+    uint32_t held_slot = 0, nx = 0;                       // nx: functional buffers written
+    const int dir = H == 0 ? -1 : 1;
+    const bool fq = f0 < quad * 32 + 32 && f0 + 3 > quad * 32;            // quadrant holds functional rows
+    const bool rows = quad * 32 < 3 * c.NR;               // quadrant holds output rows
+    const float *xa = xi, *x0 = xi;
+#pragma unroll 1
+    for (;;) {
+        int t, what = OR_SCAN;
+        uint32_t slot = 0;
+        if (held >= 0 && held == next) {
+            t = held; slot = held_slot; held = -1;
+        } else if (a < T) {
+            t = or_tile(a, T);
+            slot = (U + a) & 1;
+            or_wait(b, &b.tfull[slot], ((U + a) >> 1) & 1);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            __syncwarp();
+            ++a;
+            if (SRC || t != next) {
+                if (!SRC && a > T - 2) { held = t; held_slot = slot; continue; }
+                what = OR_SPILL;
+            }
+        } else if (!SRC && next >= 0 && next < T) {
+            t = next;
+            what = OR_FROM_J;
+        } else {
+            break;
+        }
+        const int k0 = t * OR_TS, n = min(OR_TS, K - k0);
+        const uint32_t tb = tmem + slot * 256 + ((uint32_t)(quad * 32) << 16);
+        if (c.mol && what != OR_FROM_J) {
+            // the tile's molecular functionals, to every warp of this direction
+            float *x = xi + (nx & 1) * 3 * OR_TS;
+            ++nx;
+            if (fq) {
+                const int f = row - f0;
+#pragma unroll 1
+                for (int g = 0; g < (n + 7) >> 3; ++g) {
+                    uint32_t z[8], o[8];
+                    tmem_ld8_async(tb + (par_odd ? 128 : 0) + 8 * g, z);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) o[i] = 0;
+                    tmem_ld_wait(z, o);
+                    if (f >= 0 && f < 3) {
+                        uint4 *d = reinterpret_cast<uint4 *>(x + f * OR_TS + 8 * g);
+                        d[0] = make_uint4(z[0], z[1], z[2], z[3]);
+                        d[1] = make_uint4(z[4], z[5], z[6], z[7]);
+                    }
+                }
+            }
+            or_bar(2 + H, 128);
+            xa = x + (rowB ? OR_TS : 0);
+            x0 = x + 2 * OR_TS;
+        }
+        if (rows) or_tile_run<H, LDC>(c, v, what, tb, k0, n, SRC ? c.sg : 1.f, xa, x0);
+        if (what != OR_FROM_J) {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&b.tempty[slot]);
+        }
+        if (what != OR_SPILL) next += dir;
+    }
+    return v;
+}
+
+} // namespace
+
+// SRC = false: every order from the second on, of every task.  SRC = true: the
+// source of the field at hand into J, once per task (the water column's
+// skylight, k_dtop_field).
+template <bool SRC, int LDC>
+__device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &W, const Geom &G, int t0, int nw, int Kmax,
+                                            const unsigned char *popt, const float *molc, int *counter)
+{
+    // the declared alignment keeps the pointers below known as shared memory
+    extern __shared__ __align__(1024) unsigned char or_smem[];
+    unsigned char *base = or_smem;
+    // pitch of the surface rows, round32(3 NR), which the row stride determines
+    constexpr int RP = LDC == 224 ? 128 : LDC >= 160 ? 96 : LDC >= 96 ? 64 : 32;
+    const int N = G.N, NR = G.NR, Rw = par_rows(G), kp = (Kmax + OR_GRP + 3) & ~3;
+    const uint32_t a_tile = (uint32_t)Rw * 128u;
+    unsigned char *sA = base, *sB = base + 9 * a_tile;
+    float *xs = (float *)(sB + 2 * OR_BSTAGE), *ys = xs + kp;
+    float *xi = ys + kp;                                  // [2 directions][2 buffers][3][OR_TS]
+    float *fb = xi + 2 * 2 * 3 * OR_TS;                   // [128] surface-side radiance per row (x quadrature weight)
+    float *bcx = fb + 128;                                // [2 orders][128] boundary values per row
+    float2 *red = (float2 *)(bcx + 256);              // [2 orders][8 warps]
+    Bars b;
+    b.bfull = (uint64_t *)(red + 16);
+    b.bempty = b.bfull + 2; b.tfull = b.bfull + 4; b.tempty = b.bfull + 6;
+    b.order = b.bfull + 8; b.op = b.bfull + 9; b.fin = b.bfull + 10;
+    uint32_t *tslot = (uint32_t *)(b.bfull + 11);
+    b.abort = (volatile int *)(tslot + 1);
+    volatile int *cmd = (volatile int *)(tslot + 2);      // [2]: 2 task + new, or -1
+    volatile int *cur_s = (volatile int *)(tslot + 4);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+    if (warp == 15) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&b.bfull[i], OR_TS / 16);
+            mbar_init(&b.bempty[i], 1);
+            mbar_init(&b.tfull[i], 1);
+            mbar_init(&b.tempty[i], 8);
+        }
+        mbar_init(b.order, 1);
+        mbar_init(b.op, 1);
+        mbar_init(b.fin, 1);
+        *b.abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tslot;
+
+    if (warp < 8) {
+        // ================= scan warps =================
+        const int h = warp >> 2, quad = warp & 3, row = quad * 32 + lane;
+        int s = 0, g = NR;
+        if (row < 3 * N) { s = row / N; g = row - s * N; }
+        else if (row < 3 * NR) { g = N + (row - 3 * N) / 3; s = (row - 3 * N) % 3; }
+        const int c = g < NR ? col_of(G, s, h, g) : 0;
+        const int f0 = 3 * NR;
+        uint32_t U = 0;
+        int step = 0, nxt = 0;
+        if (tid == 0) nxt = atomicAdd(counter, 1);
+        for (;;) {
+            if (tid == 0) {
+                // a task that ends with order 1 needs nothing here
+                while (!SRC && nxt < nw && B.px[B.tasks[t0 + nxt].pix].max_orders <= 1) nxt = atomicAdd(counter, 1);
+                *cur_s = nxt < nw && !*b.abort ? nxt : -1;
+            }
+            or_bar(1, 256);
+            const int tl = *cur_s;
+            if (tid == 0) {
+                cmd[step & 1] = tl < 0 ? -1 : 2 * tl + 1;
+                mbar_arrive(b.order);
+                if (tl >= 0) nxt = atomicAdd(counter, 1);
+            }
+            if (tl < 0) break;
+            const TaskDev &tk = B.tasks[t0 + tl];
+            const PixDev &d = B.px[tk.pix];
+            const int nt = d.nt, K = nt + 1, T = (K + OR_TS - 1) / OR_TS;
+            const bool water = d.medium == 1, mol = tk.m <= 2;
+            const float *lv = B.lvf + 3 * d.lev_off;
+            for (int k = tid; mol && k < K + OR_GRP; k += 256) {
+                xs[k] = k < K ? lv[3 * k] : 0.f;
+                ys[k] = k < K ? lv[3 * k + 1] : 0.f;
+            }
+            Scan sc;
+            sc.ok = g < d.n_ring;
+            sc.st = row < 3 * N;
+            sc.uni = !d.gas && !d.has_dtau;
+            sc.mol = mol;
+            sc.sg = h == 1 && s == 2 ? -1.f : 1.f;
+            sc.xs = xs; sc.ys = ys; sc.nt = nt; sc.NR = NR;
+            sc.F = W.F + tk.fld_off + c;
+            sc.Js = W.J + tk.fld_off + c;
+            const int gc = sc.ok ? g : 0;
+            sc.wT = B.Tc + d.coef_off + gc; sc.wA = B.Ca + d.coef_off + gc; sc.wB = B.Cb + d.coef_off + gc;
+            // equal optical depths (no gas, no layer overrides): every layer has the weights of the first
+            sc.T = sc.wT[0]; sc.Ca = sc.sg * sc.wA[0]; sc.Cb = sc.sg * sc.wB[0];
+            sc.cm = sc.c0 = 0.f;
+            if (mol && sc.ok) {
+                const float par = (tk.m & 1) ? -1.f : 1.f;
+                const float v = molc[(size_t)tl * OR_MOLC + row];
+                // downward: par, and sigma; the latter is in the weights
+                sc.cm = h == 0 ? v : par * v;
+                sc.c0 = s == 0 && tk.m == 0 ? 1.f : 0.f;
+            }
+            // totals at the output levels (double-float) and, where all are
+            // kept, at level 1
+            float *Tot = W.Tot + tk.fld_off + c;
+            float2 t_top = make_float2(0.f, 0.f), t_bot = t_top;
+            float t_one = 0.f;
+            if (sc.ok) {
+                t_top = make_float2(Tot[0], W.Ttl[tot_tail_off(tk, G, 0, c)]);
+                t_bot = make_float2(Tot[(size_t)nt * LDC], W.Ttl[tot_tail_off(tk, G, nt, c)]);
+                if (G.tot_all) t_one = Tot[LDC];
+            }
+            // the boundary is fed by the radiance going down at the bottom
+            // (atmosphere) or going up at the top (under the water surface)
+            const bool src = h == (water ? 0 : 1), dst = !src && (water || d.surf_on);
+            const float pw = row < 3 * N ? B.pw[(tk.m == 0 ? 0 : N) + g] : 0.f;
+            const float *Rm = (water || d.rough) ? W.srf + tk.srf_off + row : nullptr;
+            const float *MF = B.frs + ((size_t)tk.pix * NR + gc) * 9 + s * 3;
+            const bool surf = !SRC && (water || d.surf_on);
+            // The boundary values of the next order, by the threads of the source
+            // direction (they finish first: the other one starts from the boundary
+            // and ends away from it): radiance of this thread's row in, boundary
+            // value of the same row number of the other direction out.
+            auto boundary = [&](int at, float w) {
+                fb[row] = Rm ? pw * w : w;
+                or_bar(2 + h, 128);
+                float a = 0.f;
+                if (Rm) {
+                    float a0 = 0.f, a1 = 0.f;
+                    if (row < 3 * NR)
+#pragma unroll 1
+                        for (int j = 0; j < 3 * N; j += 24) {
+                            float r[24];
+#pragma unroll
+                            for (int q = 0; q < 24; ++q) r[q] = __ldg(Rm + j * RP + q * RP);
+#pragma unroll
+                            for (int q = 0; q < 24; q += 2) {
+                                a0 = fmaf(r[q], fb[j + q], a0);
+                                a1 = fmaf(r[q + 1], fb[j + q + 1], a1);
+                            }
+                        }
+                    a = a0 + a1;
+                } else if (sc.ok) {
+                    a = MF[0] * fb[srf_row(G, g, 0)] + MF[1] * fb[srf_row(G, g, 1)] + MF[2] * fb[srf_row(G, g, 2)];
+                }
+                bcx[at * 128 + row] = a;
+            };
+            if (src && surf) boundary(step & 1, sc.ok ? sc.F[water ? 0 : (size_t)nt * LDC] : 0.f);
+            float resid = 0.f;
+            int it = 2, conv = 0;
+            or_bar(1, 256);
+            for (;; ++it) {
+                const float bc = !SRC && dst && sc.ok ? bcx[(step & 1) * 128 + row] : 0.f;
+                Col v{bc, 0.f, 0.f};
+                float *xh = xi + h * 2 * 3 * OR_TS;
+                const bool odd = tk.m & 1, rb = s != 0;
+                if (h == 0) v = or_order<0, SRC, LDC>(sc, v, b, tmem, T, K, U, xh, f0, row, lane, quad, odd, rb);
+                else v = or_order<1, SRC, LDC>(sc, v, b, tmem, T, K, U, xh, f0, row, lane, quad, odd, rb);
+                U += T;
+                if (SRC) { ++step; break; }
+                // ---- end of the order: totals, surface-side radiance, residual ----
+                float mi = 0.f, mt = 0.f;
+                if (sc.ok) {
+                    t_top = df_add(t_top, h == 0 ? v.I : bc);
+                    t_bot = df_add(t_bot, h == 0 ? bc : v.I);
+                    if (G.tot_all && sc.st) t_one += sc.F[LDC];
+                    mi = v.mi;
+                    mt = fmaxf(fabsf(t_top.x), fabsf(t_bot.x));
+                    if (!isfinite(v.I)) atomicExch(B.err, OCRT_ERR_NONFINITE);
+                }
+                if (src && surf) boundary((step + 1) & 1, sc.ok ? v.I : 0.f);
+                for (int o = 16; o > 0; o >>= 1) {
+                    mi = fmaxf(mi, __shfl_xor_sync(0xffffffffu, mi, o));
+                    mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, o));
+                }
+                if (lane == 0) red[(step & 1) * 8 + warp] = make_float2(mi, mt);
+                or_bar(1, 256);
+#pragma unroll
+                for (int w = 0; w < 8; ++w) {
+                    const float2 v = red[(step & 1) * 8 + w];
+                    mi = fmaxf(mi, v.x);
+                    mt = fmaxf(mt, v.y);
+                }
+                resid = mt > 0.f ? mi / mt : 0.f;
+                conv = (double)resid < d.tol;
+                ++step;
+                if (conv || it >= d.max_orders || *b.abort) break;
+                if (tid == 0) {
+                    cmd[step & 1] = 2 * tl;
+                    mbar_arrive(b.order);
+                }
+            }
+            if (SRC) continue;
+            if (sc.ok) {
+                Tot[0] = t_top.x;
+                Tot[(size_t)nt * LDC] = t_bot.x;
+                W.Ttl[tot_tail_off(tk, G, 0, c)] = t_top.y;
+                W.Ttl[tot_tail_off(tk, G, nt, c)] = t_bot.y;
+                if (G.tot_all && sc.st && nt > 1) Tot[LDC] = t_one;
+            }
+            if (tid == 0) {
+                TaskState st;
+                st.active = 0; st.orders = it; st.converged = conv; st.pad_ = 0; st.resid = (double)resid;
+                B.state[t0 + tl] = st;
+            }
+        }
+    } else if (warp < 8 + OR_TS / 16) {
+        // ================= producers =================
+        const int pw = warp - 8;                          // 16-level block of the tile
+        const int q = lane & 7, l2 = lane >> 3;
+        // rows of iteration x: 4 apart within a warp store, so the two halves
+        // of the swizzle fall on different banks
+        auto r16 = [&](int x) -> int { return 16 * pw + x * 2 + (l2 >> 1) + (l2 & 1) * 4; };
+        const bool qin = 4 * q < N;
+        uint32_t gi = 0;                                  // stages filled
+        int K = 0, T = 0;
+        const float *Fb = nullptr, *lv = nullptr;
+        // half stage j = 2 (3 a + si) + hh of an order: rows of iterations
+        // 2 hh, 2 hh + 1 into registers
+        struct Rows { float4 u[2], v[2]; float x[2]; };
+        auto load = [&](Rows &d, int j) {
+            const int e = j >> 1, a = e / 3, si = e - 3 * a;
+            const int k0 = or_tile(a, T) * OR_TS, nl = min(OR_TS, K - k0);
+            const int rb = r16(0) + 8 * (j & 1);
+            const float *src = Fb + (size_t)(k0 + rb) * LDC + 2 * N * si + 4 * q;
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const bool in = qin && rb + 2 * x < nl;
+                d.x[x] = in && lv ? __ldg(lv + 3 * (k0 + rb + 2 * x)) : 1.f;
+                d.u[x] = in ? *reinterpret_cast<const float4 *>(src + 2 * x * LDC) : make_float4(0.f, 0.f, 0.f, 0.f);
+                d.v[x] = in ? *reinterpret_cast<const float4 *>(src + 2 * x * LDC + N) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        };
+        // F+- of half a stage into its B tile
+        auto fill = [&](const Rows &d, int j, uint32_t st) {
+            const int si = (j >> 1) % 3, rb = r16(0) + 8 * (j & 1);
+            // F+ = up + sigma down: for U the sum is F- and the difference F+
+            unsigned char *tile = sB + st * OR_BSTAGE;
+            const int cs = 4 * q + (si == 2 ? 32 : 0), cd = 4 * q + (si == 2 ? 0 : 32);
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                uint32_t s0[3], s1[3], d0[3], d1[3];
+                const float f = d.x[x];
+                const float4 u = d.u[x], v = d.v[x];
+                split_bf16x3(f * (u.x + v.x), f * (u.y + v.y), s0);
+                split_bf16x3(f * (u.z + v.z), f * (u.w + v.w), s1);
+                split_bf16x3(f * (u.x - v.x), f * (u.y - v.y), d0);
+                split_bf16x3(f * (u.z - v.z), f * (u.w - v.w), d1);
+                unsigned char *ps = tile + par_swz(rb + 2 * x, cs), *pd = tile + par_swz(rb + 2 * x, cd);
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    *reinterpret_cast<uint2 *>(ps + p * OR_BPIECE) = make_uint2(s0[p], s1[p]);
+                    *reinterpret_cast<uint2 *>(pd + p * OR_BPIECE) = make_uint2(d0[p], d1[p]);
+                }
+            }
+        };
+        for (int step = 0;; ++step) {
+            or_wait(b, b.order, step & 1);
+            __syncwarp();
+            if (*b.abort) break;
+            const int cm = cmd[step & 1];
+            if (cm < 0) break;
+            if (cm & 1) {
+                const TaskDev &tk = B.tasks[t0 + (cm >> 1)];
+                K = tk.K;
+                T = (K + OR_TS - 1) / OR_TS;
+                Fb = W.F + tk.fld_off;
+                lv = tk.m <= 2 ? nullptr : B.lvf + 3 * B.px[tk.pix].lev_off;
+            }
+            // the rows of a stage are loaded while the stage before is split
+            Rows ra, rb;
+            load(ra, 0);
+            load(rb, 1);
+#pragma unroll 1
+            for (int j = 0; j < 6 * T; j += 2, ++gi) {
+                const uint32_t st = gi & 1;
+                const bool mine = 16 * pw < min(OR_TS, K - or_tile(j / 6, T) * OR_TS);
+                if (gi >= 2) or_wait(b, &b.bempty[st], ((gi >> 1) - 1) & 1);
+                __syncwarp();
+                if (mine) fill(ra, j, st);
+                if (j + 2 < 6 * T) load(ra, j + 2);
+                if (mine) fill(rb, j + 1, st);
+                if (j + 3 < 6 * T) load(rb, j + 3);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&b.bfull[st]);
+            }
+        }
+    } else if (warp == 15) {
+        // ================= operator load and MMA issue =================
+        // The warp runs converged and one elected lane issues: addresses and
+        // descriptors then stay on the uniform datapath (from a divergent
+        // single lane an MMA took 119 cycles to issue, twice its run time).
+        uint32_t gi = 0, U = 0, nop = 0;
+        int K = 0, T = 0;
+        bool op_out = false;                              // an operator copy in flight
+        const bool two = N > 16;                          // two 16-deep steps per parity
+        const uint32_t sa = smem_u32(sA) >> 4, sb = smem_u32(sB) >> 4, at = a_tile >> 4;
+        const uint64_t dbase = sdesc_sw128(0);            // layout bits; addresses are below 2^18
+        for (int step = 0;; ++step) {
+            or_wait(b, b.order, step & 1);
+            if (__any_sync(0xffffffffu, *b.abort != 0)) break;
+            const int cm = cmd[step & 1];
+            if (cm < 0) break;
+            if (cm & 1) {
+                const int tl = cm >> 1;
+                K = B.tasks[t0 + tl].K;
+                T = (K + OR_TS - 1) / OR_TS;
+                // the operator's shared memory is free: every product of the
+                // task before has been consumed
+                if (lane == 0) {
+                    mbar_expect_tx(b.op, 9 * a_tile);
+                    bulk_g2s(sA, popt + (size_t)tl * par_bytes(G), 9 * a_tile, b.op);
+                }
+                __syncwarp();
+                or_wait(b, b.op, nop & 1);
+                op_out = __any_sync(0xffffffffu, *b.abort != 0);
+                if (op_out) break;
+                ++nop;
+            }
+            bool stop = false;
+#pragma unroll 1
+            for (int a = 0; a < T && !stop; ++a, ++U) {
+                const uint32_t slot = U & 1;
+                const int nl = min(OR_TS, K - or_tile(a, T) * OR_TS), n16 = (nl + 15) & ~15;
+                if (U >= 2) or_wait(b, &b.tempty[slot], ((U >> 1) - 1) & 1);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t idesc = idesc_bf16(128, n16), acc = tmem + slot * 256;
+#pragma unroll 1
+                for (int si = 0; si < 3; ++si, ++gi) {
+                    const uint32_t st = gi & 1;
+                    or_wait(b, &b.bfull[st], (gi >> 1) & 1);
+                    if (__any_sync(0xffffffffu, *b.abort != 0)) { stop = true; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t ta = sa + si * 3 * at, tb = sb + st * (OR_BSTAGE >> 4);
+                    if (elect_one()) {
+                        // pieces (operator, field) of the six products, the small ones
+                        // first: the accumulator is truncated at each step, so the
+                        // fewer steps it takes at full size the better
+                        constexpr int pa[6] = {2, 1, 0, 1, 0, 0}, pb[6] = {0, 1, 2, 0, 1, 0};
+#pragma unroll
+                        for (int pr = 0; pr < 2; ++pr)
+#pragma unroll
+                            for (int e = 0; e < 12; ++e) {
+                                const int q = e >> 1, k = e & 1, off = pr * 4 + k * 2;
+                                if (k && !two) continue;
+                                umma_bf16(acc + pr * 128, dbase | (ta + off + pa[q] * at),
+                                          dbase | (tb + off + pb[q] * (OR_BPIECE >> 4)), idesc, (si > 0 || e > 0) ? 1u : 0u);
+                            }
+                        umma_commit(&b.bempty[st]);
+                        if (si == 2) umma_commit(&b.tfull[slot]);
+                    }
+                    __syncwarp();
+                }
+            }
+            if (stop) break;
+        }
+        // an operator copy still in flight lands, and every MMA completes,
+        // before the CTA leaves
+        if (op_out) (void)mbar_wait(b.op, nop & 1);
+        if (elect_one()) umma_commit(b.fin);
+        __syncwarp();
+        if (!mbar_wait(b.fin, 0)) *b.abort = 1;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (tid == 0 && *b.abort) atomicExch(B.err, OCRT_ERR_DEVICE);
+    if (warp == 15) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
+// The row stride is a template argument: the scan's stores and the producers'
+// loads then take immediate offsets.  Its values for N = 8, 16, 24, 32 with one
+// or four zero-weight slots.
+template <int LDC>
+__global__ void __launch_bounds__(OR_THREADS, 1)
+k_orders(BatchBufs B, WaveBufs W, Geom G, int t0, int nw, int Kmax, const unsigned char *popt, const float *molc,
+         int *counter)
+{
+    orders_body<false, LDC>(B, W, G, t0, nw, Kmax, popt, molc, counter);
+}
+
+template <int LDC>
+__global__ void __launch_bounds__(OR_THREADS, 1)
+k_orders_source(BatchBufs B, WaveBufs W, Geom G, int t0, int nw, int Kmax, const unsigned char *popt, const float *molc,
+                int *counter)
+{
+    orders_body<true, LDC>(B, W, G, t0, nw, Kmax, popt, molc, counter);
+}
+
+// Task counters of a wave's launches.
+__global__ void k_orders_reset(int *counter)
+{
+    if (threadIdx.x < 2) counter[threadIdx.x] = 0;
+}
+
+namespace {
+
+typedef void (*OrdersFn)(BatchBufs, WaveBufs, Geom, int, int, int, const unsigned char *, const float *, int *);
+struct OrdersInst { int ldc; OrdersFn orders, source; };
+const OrdersInst g_orders[] = {{64, k_orders<64>, k_orders_source<64>},    {96, k_orders<96>, k_orders_source<96>},
+                               {128, k_orders<128>, k_orders_source<128>}, {160, k_orders<160>, k_orders_source<160>},
+                               {192, k_orders<192>, k_orders_source<192>}, {224, k_orders<224>, k_orders_source<224>}};
+
+const OrdersInst *orders_inst(int ldc)
+{
+    for (const OrdersInst &o : g_orders)
+        if (o.ldc == ldc) return &o;
+    return nullptr;
+}
+
+} // namespace
+
+// N a multiple of 8 keeps the producers' rows in whole float4s and the surface
+// rows in whole steps of the boundary sum; 3 NR + 3 rows fit one MMA of 128
+// (111 at 32 streams with four zero-weight slots); larger N (48 streams) would need a
+// second M tile and twice the operator, 480 KB, more than an SM has.
+bool orders_supported(const Geom &G, int Kmax)
+{
+    return G.N % 8 == 0 && G.N <= 32 && 3 * G.NR + 3 <= 128 && orders_inst(G.LDC) &&
+           orders_smem_bytes(G, Kmax) <= 227 * 1024;
+}
+
+void orders_launch(bool source, int grid, cudaStream_t st, const BatchBufs &B, const WaveBufs &W, const Geom &G, int t0,
+                   int nw, int Kmax, const unsigned char *popt, const float *molc, int *counter)
+{
+    const OrdersInst *o = orders_inst(G.LDC);
+    (source ? o->source : o->orders)<<<grid, OR_THREADS, orders_smem_bytes(G, Kmax), st>>>(B, W, G, t0, nw, Kmax, popt,
+                                                                                        molc, counter);
+}
+
+cudaError_t orders_init()
+{
+    for (const OrdersInst &o : g_orders)
+        for (OrdersFn f : {o.orders, o.source}) {
+            const cudaError_t e = cudaFuncSetAttribute((const void *)f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       227 * 1024);
+            if (e != cudaSuccess) return e;
+        }
+    return cudaSuccess;
+}

@@ -366,7 +366,8 @@ __global__ void __launch_bounds__(256, 2) k_tables(const TaskDev *tasks, int t0,
                          const double *gw,
                          const double *mb, const double *mg, const double *ma, const double *mz,
                          float *ops, float *pvec, float *fvec, float *opt, int plain,
-                         const float *V, int vp0, long long vstride, const float *sprod)
+                         const float *V, int vp0, long long vstride, const float *sprod, float *molc,
+                         unsigned char *popt)
 {
     const int tl = blockIdx.x;
     if (tl >= nt_tasks) return;
@@ -501,6 +502,24 @@ __global__ void __launch_bounds__(256, 2) k_tables(const TaskDev *tasks, int t0,
     }
     // tables: value at +col = S, at -col = sigma * D with sigma from the column basis
     auto emit = [&](const float *Ea, const float *Oa, int i) {
+        if (popt) {
+            // parity operator of k_orders: the sums themselves, as k_tables_tc lays it out
+            float v0 = Ea[0], v1 = Oa[0];
+            if (Vm) {
+                const float *v = Vm + (size_t)(1 + i) * 2 * G.NR + os;
+                v0 = 0.5f * (v[0] + v[G.NR]);
+                v1 = 0.5f * (v[0] - v[G.NR]);
+            }
+            for (int pr = 0; pr < 2; ++pr) {
+                float c[9];
+                par_coefs(pr ? Oa : Ea, pr ? Ea : Oa, c);
+                c[0] = pr ? v1 : v0;
+                for (int q = 0; q < 9; ++q)
+                    par_put(popt + (size_t)tl * par_bytes(G), G, q % 3, srf_row(G, os, q / 3), 32 * pr + i,
+                            c[q] * (float)gw[i]);
+            }
+            return;
+        }
         float S[13], D[13], c[18];
 #pragma unroll
         for (int q = 0; q < 13; ++q) { S[q] = Ea[q] + Oa[q]; D[q] = Ea[q] - Oa[q]; }
@@ -531,7 +550,25 @@ __global__ void __launch_bounds__(256, 2) k_tables(const TaskDev *tasks, int t0,
     // w_i f(mu_i), f in {1, P2m, R2m, T2m}; U holds the outgoing factors for
     // input block b = 2s + h and functional f at column 4b + f.  The sign
     // pattern is that of the pair contraction in rt_sos_operator.c:387-406.
-    if (Bop && mol) {
+    if (popt && mol && !sprod) {
+        // functional rows of the parity operator (the others were cleared)
+        for (int e = threadIdx.x; e < 3 * N; e += blockDim.x) {
+            const int f = e / N, i = e - f * N;
+            float c[3];
+            par_functional(f, m, d.depol, basis(0, i, 2), basis(1, i, 2), basis(2, i, 2), c);
+            for (int si = 0; si < 3; ++si)
+                par_put(popt + (size_t)tl * par_bytes(G), G, si, 3 * G.NR + f, 32 * (m & 1) + i, c[si] * (float)gw[i]);
+        }
+    }
+    if (molc && mol) {
+        // k_orders: the row factors of the parity form, J_mol = factor x xi
+        // (P for I, R for Q, -T for U of the outgoing slot)
+        for (int e = threadIdx.x; e < 3 * n; e += blockDim.x) {
+            const int o = e / 3, so = e - 3 * o;
+            const float v = basis(so, o, 2);
+            molc[(size_t)tl * OR_MOLC + srf_row(G, o, so)] = so == 2 ? -v : v;
+        }
+    } else if (Bop && mol) {
         for (int e = threadIdx.x; e < n * 6; e += blockDim.x) {
             const int o = e / 6, ob = e - o * 6;
             const float po = basis(0, o, 2), ro = basis(1, o, 2), to = basis(2, o, 2);
@@ -852,7 +889,7 @@ __device__ __forceinline__ void coxmunk_pair(int p, int o, int i, const TaskDev 
                 float sc = m == 0 ? scale0 : scale1;
                 if (m > 0 && (e == 2 || e == 5)) sc = -sc;
                 const TaskDev &tk = tasks[task_first + m];
-                const size_t off = i < N ? ((size_t)os * N + i) * 9 + e : (size_t)G.NR * N * 9 + (size_t)os * 9 + e;
+                const size_t off = i < N ? srf_entry(G, os, i, e) : (size_t)G.srf_sun + (size_t)os * 9 + e;
                 srf[tk.srf_off + off] = acc[a][b] * sc;
                 if (DW) srfW[tk.srf_off + off] = (ca * acc[a][b] + cb * acct[AT == 5 ? a : 0][b]) * sc;
                 if (mirror) {
@@ -860,7 +897,7 @@ __device__ __forceinline__ void coxmunk_pair(int p, int o, int i, const TaskDev 
                     const int et = (e % 3) * 3 + e / 3;
                     float st = m == 0 ? scale0 : scale1;
                     if (m > 0 && (et == 2 || et == 5)) st = -st;
-                    const size_t offt = ((size_t)i * N + os) * 9 + et;
+                    const size_t offt = srf_entry(G, i, os, et);
                     srf[tk.srf_off + offt] = acc[a][b] * st;
                     if (DW) srfW[tk.srf_off + offt] = (ca * acc[a][b] + cb * acct[AT == 5 ? a : 0][b]) * st;
                 }

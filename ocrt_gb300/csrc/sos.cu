@@ -24,7 +24,7 @@
 __device__ inline float rough_seed(const TaskDev &tk, const WaveBufs &W, const BatchBufs &B, const PixDev &d,
                                    const Geom &G, float fs_tdn, int k, int g, int s)
 {
-    const float *Rs = W.srf + tk.srf_off + (size_t)G.NR * G.N * 9;
+    const float *Rs = W.srf + tk.srf_off + G.srf_sun;
     return fs_tdn * B.Eatt[(d.lev_off + k) * G.NR + g] * Rs[g * 9 + s * 3];
 }
 
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(512, 1) k_primary(BatchBufs B, WaveBufs W, Geo
     // rough direct-beam seed (rt_surface_boundary.c:430-493) on upward columns:
     // fs_tdn exp(-(tau-h_k)/mu_g) R_m(mu_g, mu0)[s, I], the attenuation per level from Eatt
     const bool seeded = d.rough && h == 0 && !d.bottom_only;
-    const float rs = seeded ? W.srf[tk.srf_off + (size_t)G.NR * G.N * 9 + g * 9 + s * 3] : 0.f;
+    const float rs = seeded ? W.srf[tk.srf_off + G.srf_sun + g * 9 + s * 3] : 0.f;
     // water column: the skylight's first-scatter source, computed into J by the
     // source pass over the unscattered skylight field (k_dtop_field)
     const float *Jdt = (d.medium == 1 && d.ext_off >= 0 && tk.m <= d.ext_mmax) ? W.J + tk.fld_off : nullptr;
@@ -157,7 +157,7 @@ __device__ __forceinline__ void primary_cols(const BatchBufs &B, const WaveBufs 
     for (int u = 0; u < WD; ++u) {
         faP[u] = d.bottom_only ? 0.f : pv[u];
         fmP[u] = d.bottom_only ? 0.f : pv[G.LDC + u];
-        rs[u] = seeded ? W.srf[tk.srf_off + (size_t)NR * N * 9 + (g + u) * 9 + s * 3] : 0.f;
+        rs[u] = seeded ? W.srf[tk.srf_off + G.srf_sun + (g + u) * 9 + s * 3] : 0.f;
         exv[u] = extb ? (float)B.ext[d.ext_off + ((size_t)tk.m * NR + g + u) * 3 + s] : 0.f;
     }
     const float *Jdt = (d.medium == 1 && d.ext_off >= 0 && tk.m <= d.ext_mmax) ? W.J + tk.fld_off + c : nullptr;

@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1)
 k_tables_tc(const TaskDev *tasks, int t0, int nt_tasks, const PixDev *px, Geom G, int L, const float *GT,
             const float *AT, const float *Bx, const double *gw, const double *mb, const double *mg, const double *ma,
             const double *mz, float *ops, float *opt, int plain, const float *V, int vp0, long long vstride,
-            float *sprod, int *err)
+            float *sprod, int *err, unsigned char *popt, const float *Bp, const float *Br, const float *Bt)
 {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *base = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -356,8 +356,8 @@ k_tables_tc(const TaskDev *tasks, int t0, int nt_tasks, const PixDev *px, Geom G
                         for (int i = 0; i < 32; ++i)
                             if (i < N) {
                                 const float ev = __uint_as_float(e[i]), ov = __uint_as_float(od[i]);
-                                pt[i] = ev + ov;
-                                pt[13 * TT_PS + i] = ev - ov;
+                                pt[i] = popt ? ev : ev + ov;
+                                pt[13 * TT_PS + i] = popt ? ov : ev - ov;
                             }
                     }
                 } else if (role == 1) {
@@ -380,6 +380,68 @@ k_tables_tc(const TaskDev *tasks, int t0, int nt_tasks, const PixDev *px, Geom G
             // ---- operator entries: a warp per outgoing slot, lane = incoming Gauss slot ----
             const float *Vm = (V && d.vk_n > 1) ? V + (size_t)(tk.pix - vp0) * vstride + (size_t)m * (N + 1) * 2 * G.NR
                                                 : nullptr;
+            if (popt) {
+                // ---- parity operator of the fused order kernel ----
+                // The field enters as F+- = F_up +- sigma F_dn (sigma = 1, 1, -1
+                // for I, Q, U), in which the operator is block diagonal; its
+                // entries are the even- and odd-(l + m) sums themselves, so
+                // nothing cancels.  Lane: parity lane >> 4, incoming slots i, i + 1.
+                const int pr = lane >> 4, i0 = 2 * (lane & 15), Rw = par_rows(G), n3 = 3 * n;
+                unsigned char *Pt = popt + (size_t)tl * par_bytes(G);
+                const float w0 = i0 < N ? (float)gw[i0] : 0.f, w1 = i0 + 1 < N ? (float)gw[i0 + 1] : 0.f;
+                auto put = [&](int si, int row, float a, float b) {
+                    uint32_t pc[3];
+                    split_bf16x3(i0 < N ? a * w0 : 0.f, i0 + 1 < N ? b * w1 : 0.f, pc);
+                    unsigned char *dst = Pt + (size_t)si * 3 * Rw * 128 + par_swz(row, 32 * pr + i0);
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) *reinterpret_cast<uint32_t *>(dst + (size_t)q * Rw * 128) = pc[q];
+                };
+                for (int item = ew; item < n3; item += TT_EW) {
+                    const int o = item / 3, so = item - 3 * o, row = srf_row(G, o, so);
+                    // X: the sums of this lane's parity, Y: of the other one
+                    const float *X = ptab + (size_t)o * 26 * TT_PS + (pr ? 13 * TT_PS : 0) + i0;
+                    const float *Y = ptab + (size_t)o * 26 * TT_PS + (pr ? 0 : 13 * TT_PS) + i0;
+                    // entries of this outgoing component from its three incoming ones
+                    auto pair = [&](int u, float *c9) {
+                        float x[13], y[13];
+#pragma unroll
+                        for (int q = 0; q < 13; ++q) { x[q] = X[q * TT_PS + u]; y[q] = Y[q * TT_PS + u]; }
+                        par_coefs(x, y, c9);
+                        if (Vm && i0 + u < N) {                      // the value kernel's table instead
+                            const float *v = Vm + (size_t)(1 + i0 + u) * 2 * G.NR + o;
+                            c9[0] = 0.5f * (v[0] + (pr ? -v[G.NR] : v[G.NR]));
+                        }
+                    };
+                    float ca[9], cb[9];
+                    pair(0, ca);
+                    pair(1, cb);
+#pragma unroll
+                    for (int si = 0; si < 3; ++si)
+                        put(si, row, so == 0 ? ca[si] : so == 1 ? ca[3 + si] : ca[6 + si],
+                            so == 0 ? cb[si] : so == 1 ? cb[3 + si] : cb[6 + si]);
+                }
+                // rows of unused zero-weight slots, the molecular functionals
+                // and the padding rows
+                for (int row = 3 * n + ew; row < Rw; row += TT_EW) {
+                    const int f = row - 3 * G.NR;
+                    const bool on = m <= 2 && f >= 0 && f < 3 && pr == (m & 1);
+                    float v[3][2] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+                    if (on) {
+                        const size_t gb = ((size_t)m * (L + 1) + 2) * N;
+#pragma unroll
+                        for (int u = 0; u < 2; ++u)
+                            if (i0 + u < N) {
+                                float c[3];
+                                par_functional(f, m, d.depol, Bp[gb + i0 + u], Br[gb + i0 + u], Bt[gb + i0 + u], c);
+                                v[0][u] = c[0]; v[1][u] = c[1]; v[2][u] = c[2];
+                            }
+                    }
+#pragma unroll
+                    for (int si = 0; si < 3; ++si) put(si, row, v[si][0], v[si][1]);
+                }
+                tt_bar(1, TT_EW * 32);                               // table reads done
+                continue;
+            }
             float *Aop = ops + tk.op_off;
             float *Atile = opt ? opt + 2 * tk.op_off : nullptr;
             if (lane < N) {
@@ -471,9 +533,9 @@ size_t tables_tc_gt_floats(int N, int M, int L) { return (size_t)(M + 1) * 3 * N
 
 size_t tables_tc_at_floats(int M, int L) { return (size_t)(M + 1) * (tt_kpad(L) / TT_KC) * 2 * TT_AG_FLOATS; }
 
-bool tables_tc_supported(const Geom &G, int L)
+bool tables_tc_supported(const Geom &G, int L, bool parity)
 {
-    return G.N <= 32 && 3 * (G.E + 1) <= 32 && G.CIN % 32 == 0 && tables_tc_smem_bytes(G, L) <= 227 * 1024;
+    return G.N <= 32 && 3 * (G.E + 1) <= 32 && (parity || G.CIN % 32 == 0) && tables_tc_smem_bytes(G, L) <= 227 * 1024;
 }
 
 int tables_tc_threads() { return TT_THREADS; }

@@ -1,0 +1,47 @@
+"""All orders of a task in one CTA (k_orders: N = 8, 16, 24, 32, forward solves)
+at the edges of its shape: tiles of 112 levels (one tile, a tile of one level,
+two, three and four tiles, so kept, spilled and reloaded ones), groups of 16
+levels, the smallest column, every surface, layers of unequal optical depth,
+molecules alone, the view as an inserted slot and as a Gauss node.
+
+Against the FP64 oracle at the parity bar, and against the separate passes
+(OCRT_GB_SOURCE_KERNEL=simt) at 1e-5 relative in I and 1e-6 absolute in Q and U:
+an order is an FP32 recurrence over at most 400 levels, about sqrt(400) x 6e-8
+= 1.2e-6 of the field per path, the operators differ by the same FP32 rounding,
+and a mode may stop one order earlier (tolerance 1e-7)."""
+import numpy as np
+import pytest
+
+from _helpers import assert_parity
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("layers", [2, 14, 111, 112, 128, 223, 224, 336, 400])
+@pytest.mark.parametrize("N", [8, 16, 24, 32])
+def test_orders_match_oracle_and_separate_passes(gpu, oracle, monkeypatch, N, layers):
+    from ocrt_gb300 import _abi as A
+    from synthetic import hg_aerosol_moments
+    rng = np.random.default_rng(1000 * N + layers)
+    mom = hg_aerosol_moments(0.7, 40)
+    cases, aers, ly = [], [], []
+    for surface, aerosol, uneven in (("black_fresnel_ocean", True, False), ("black", True, True), ("flat", False, False),
+                                     ("black_fresnel_ocean", False, True)):
+        cases.append(A.default_case(surface=surface, sza_deg=rng.uniform(5, 70), vza_deg=rng.uniform(0, 60),
+                                    raa_deg=rng.uniform(0, 180), wind_speed=rng.uniform(1, 10),
+                                    wavelength_nm=float(rng.choice([443.0, 865.0]))))
+        aers.append(A.AerosolHolder(rng.uniform(0.05, 0.4) if aerosol else 0.0, rng.uniform(0.85, 0.99), *mom))
+        dt = rng.uniform(0.5, 1.5, layers) * 0.3 / layers if uneven else None
+        ly.append(A.LayersHolder(layers, dt, None))
+    o = A.default_opts(n_mu=N, n_layers=layers, fourier_m_max=4, max_orders=300, tolerance=1e-7,
+                       view_as_node=int(layers % 2))
+    monkeypatch.delenv("OCRT_GB_SOURCE_KERNEL", raising=False)
+    got, _ = gpu.solve_batch_adjoint(cases, o, aers, ly, None)
+    monkeypatch.setenv("OCRT_GB_SOURCE_KERNEL", "simt")
+    sep, _ = gpu.solve_batch_adjoint(cases, o, aers, ly, None)
+    np.testing.assert_allclose(got["rho_I"], sep["rho_I"], rtol=1e-5, atol=0)
+    for k in ("rho_Q", "rho_U"):
+        np.testing.assert_allclose(got[k], sep[k], rtol=0, atol=1e-6)
+    for i, c in enumerate(cases):
+        ref = oracle.solve_layers(c, o, aers[i], ly[i].dtau, None)
+        assert_parity({k: got[k][i] for k in ("rho_I", "rho_Q", "rho_U")}, ref, f"N={N} layers={layers} pixel {i}")
