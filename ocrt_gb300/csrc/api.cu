@@ -901,10 +901,9 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
     CK(cudaMemsetAsync(g.err, 0, 2 * sizeof(int), st));
     LAUNCH(plan, KC_SETUP, k_gauss<<<1, 64, 0, st>>>(g.N, g.gmu, g.gw, g.pw));
     LAUNCH(plan, KC_SETUP, k_pixel_setup<<<(P + 127) / 128, 128, 0, st>>>(g.px, P, g.N, g.gmu));
-    LAUNCH(plan, KC_SETUP, k_levels<<<dim3(2, P), 256, 0, st>>>(g.px, P, g.h, g.ch, g.xd, g.yd, g.z));
+    LAUNCH(plan, KC_SETUP, k_levels<<<dim3(lev_blocks(g.ntmax), P), LEV_B, 0, st>>>(g.px, P, g.h, g.ch, g.xd, g.yd, g.z));
     if (g.any_water)
         LAUNCH(plan, KC_SETUP, k_levels_water<<<dim3(2, P), 256, 0, st>>>(g.px, P, g.h, g.ch, g.xd, g.yd, g.z));
-    LAUNCH(plan, KC_SETUP, k_level_mix<<<dim3(2, P), 256, 0, st>>>(g.px, P, g.z, g.xd, g.yd));
     if (g.any_gas)
         LAUNCH(plan, KC_SETUP, k_gas_apply<<<P, 256, 0, st>>>(g.px, P, g.h, g.ch, g.xd, g.yd, g.z, g.tabs));
     if (g.any_layers)
@@ -994,7 +993,7 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
         CK(cudaMemsetAsync(g.mol_cnt, 0, sizeof(int) * ((size_t)g.max_orders + 2), st));
         CK(cudaMemsetAsync(g.work, 0, sizeof(int) * 4 * ((size_t)g.max_orders + 2), st));
         CK(cudaMemsetAsync(g.aflag, 0, (size_t)nw, st));
-        LAUNCH(plan, KC_TABLES, k_basis_pix<<<(nw + 128 / (1 + G.E) - 1) / (128 / (1 + G.E)), 128, 0, st>>>(
+        LAUNCH(plan, KC_TABLES, k_basis_pix<<<(nw + 32 / (1 + G.E) - 1) / (32 / (1 + G.E)), 32, 0, st>>>(
                    g.tasks, w.t0, nw, g.px, g.Lmax, G.E, g.Bx, g.gcoef));
         if (g.any_vk)
             LAUNCH(plan, KC_TABLES, k_value_pfm<<<dim3(((G.N + 1) * 2 * G.NR + 127) / 128, w.p1 - w.p0), 128,
@@ -1779,8 +1778,7 @@ int level_profile(const ocrt_case *cs, const ocrt_opts *opts, const ocrt_aerosol
         h.assign(nt + 1, 0.0); zk.assign(nt + 1, 0.0); ta.assign(nt + 1, 0.0); w.assign(nt, 0.0);
         k_gauss<<<1, 64, 0, st>>>(g.N, g.gmu, g.gw, g.pw);
         k_pixel_setup<<<1, 128, 0, st>>>(g.px, 1, g.N, g.gmu);
-        k_levels<<<dim3(2, 1), 256, 0, st>>>(g.px, 1, g.h, g.ch, g.xd, g.yd, g.z);
-        k_level_mix<<<dim3(2, 1), 256, 0, st>>>(g.px, 1, g.z, g.xd, g.yd);
+        k_levels<<<dim3(lev_blocks(nt), 1), LEV_B, 0, st>>>(g.px, 1, g.h, g.ch, g.xd, g.yd, g.z);
         if (g.any_gas) k_gas_apply<<<1, 256, 0, st>>>(g.px, 1, g.h, g.ch, g.xd, g.yd, g.z, g.tabs);
         const size_t lb = sizeof(double) * (nt + 1);
         if (cudaGetLastError() != cudaSuccess ||

@@ -8,9 +8,10 @@
 // setup.cu
 __global__ void k_gauss(int N, double *mu, double *w, float *pw);
 __global__ void k_pixel_setup(PixDev *px, int P, int N, const double *gmu);
+#define LEV_B 64        // threads of k_levels; a block holds LEV_B - 1 levels
+static inline int lev_blocks(int nt) { return (nt + LEV_B - 1) / (LEV_B - 1); }
 __global__ void k_levels(const PixDev *px, int P, double *h, double *ch, double *xd, double *yd, double *z);
 __global__ void k_levels_water(const PixDev *px, int P, double *h, double *ch, double *xd, double *yd, double *z);
-__global__ void k_level_mix(const PixDev *px, int P, const double *z, double *xd, double *yd);
 __global__ void k_coef(const PixDev *px, int P, int N, int NR, const double *gmu, const double *h,
                        float *Tc, float *Ca, float *Cb);
 __global__ void k_coef_quads(const PixDev *px, int P, int N, int NR, const float *Tc, const float *Ca, const float *Cb,

@@ -36,127 +36,131 @@ __host__ __device__ inline double bodhaine_tau(double wl_nm, double p_hpa)
 }
 
 // ---- altitude mapping (rt_molecular_profile.c:9-105, rt_atm.c:44-51) ----
-__device__ inline double us62_pressure(double z)
-{
-    const double Z[8] = {0.0, 11.0, 20.0, 32.0, 47.0, 51.0, 71.0, 84.852};
-    const double P[8] = {101325.0, 22632.1, 5474.89, 868.019, 110.906, 66.9389, 3.95642, 0.3734};
-    if (z <= Z[0]) return P[0];
-    if (z >= Z[7]) return P[7];
-    int lo = 0, hi = 7;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (z < Z[mid]) hi = mid; else lo = mid;
-    }
-    const double t = (z - Z[lo]) / (Z[hi] - Z[lo]);
-    const double a = log(P[lo]), b = log(P[hi]);
-    return exp(a + t * (b - a));
-}
-
 __device__ inline double clamp01d(double x) { return x <= 0.0 ? 0.0 : (x >= 1.0 ? 1.0 : x); }
 
-__device__ inline double us62_raw(double z)
-{
-    if (z <= 0.0) return 1.0;
-    const double g0 = gravity_wgs84(45.0, 0.0);
-    if (z >= 84.852) return clamp01d((0.3734 / gravity_wgs84(45.0, 84852.0)) / (101325.0 / g0));
-    return clamp01d((us62_pressure(z) / gravity_wgs84(45.0, z * 1000.0)) / (101325.0 / g0));
-}
-
-__device__ inline double us62_grid_above(double z)
-{
-    if (z <= 0.0) return 1.0;
-    if (z >= 84.852) return 0.0;
-    const double ft = us62_raw(84.852);
-    return clamp01d((us62_raw(z) - ft) / (1.0 - ft));
-}
-
-__device__ inline double exp_above(double z, double ztop, double h)
-{
-    if (z <= 0.0) return 1.0;
-    if (z >= ztop) return 0.0;
-    const double et = exp(-ztop / h);
-    return (exp(-z / h) - et) / (1.0 - et);
-}
-
-__device__ inline double ray_above(double z, int profile, double h)
-{
-    return profile == 1 ? exp_above(z, OCRT_ZTOP_KM, h) : us62_grid_above(z);
-}
-
-// The same column fractions with their altitude-independent parts evaluated
-// once per thread (the table logarithms, the 45-degree gravity term, the US62
-// fraction at 84.852 km, exp(-ztop / h)), for the 64-step level bisection.
+// Fractions of the molecular (US62 table or exponential) and aerosol column
+// above an altitude.  What does not depend on the altitude (the table
+// logarithms, the 45-degree gravity term, the US62 fraction at 84.852 km,
+// exp(-ztop / h)) is evaluated once per block into shared memory, with FP32
+// copies for the search.
 struct AboveEval {
     int prof;
     double rh, ah, et_r, et_a;
-    double lp[8], a45, q0, ft;
+    double z[8], lp[8], a45, q0, ft;
+    float rh_f, ah_f, et_r_f, et_a_f, z_f[8], lp_f[8], a45_f, q0_f, ft_f;
 };
 
-__device__ inline double above_g45(const AboveEval &E, double z_m) { return E.a45 - 3.086e-6 * z_m; }
+__device__ inline double above_g45(double a45, double z_m) { return a45 - 3.086e-6 * z_m; }
 
-__device__ inline void above_init(AboveEval &E, int prof, double ray_h, double aer_h)
+// By the first 11 threads of a block; a barrier follows.
+__device__ inline void above_init(AboveEval &E, int prof, double ray_h, double aer_h, int tid)
 {
+    const double Z[8] = {0.0, 11.0, 20.0, 32.0, 47.0, 51.0, 71.0, 84.852};
     const double P[8] = {101325.0, 22632.1, 5474.89, 868.019, 110.906, 66.9389, 3.95642, 0.3734};
-    E.prof = prof; E.rh = ray_h; E.ah = aer_h;
-    E.et_r = exp(-OCRT_ZTOP_KM / ray_h);
-    E.et_a = exp(-OCRT_ZTOP_KM / aer_h);
-    for (int i = 0; i < 8; ++i) E.lp[i] = log(P[i]);
-    const double lat = 45.0 * OCRT_PI / 180.0;
-    const double s1 = sin(lat) * sin(lat), s2 = sin(2.0 * lat) * sin(2.0 * lat);
-    E.a45 = 9.780327 * (1.0 + 0.0053024 * s1 - 0.0000058 * s2);
-    E.q0 = 101325.0 / above_g45(E, 0.0);
-    E.ft = clamp01d((0.3734 / above_g45(E, 84852.0)) / E.q0);     // us62_raw(84.852)
+    if (tid < 8) {
+        double zi = 0.0, pi = 1.0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (i == tid) { zi = Z[i]; pi = P[i]; }
+        E.z[tid] = zi;
+        E.lp[tid] = log(pi);
+        E.z_f[tid] = (float)zi;
+        E.lp_f[tid] = (float)E.lp[tid];
+    } else if (tid == 8 || tid == 9) {
+        const double hh = tid == 8 ? ray_h : aer_h, et = exp(-OCRT_ZTOP_KM / hh);
+        if (tid == 8) { E.rh = hh; E.et_r = et; E.rh_f = (float)hh; E.et_r_f = (float)et; }
+        else { E.ah = hh; E.et_a = et; E.ah_f = (float)hh; E.et_a_f = (float)et; }
+    } else if (tid == 10) {
+        E.prof = prof;
+        const double lat = 45.0 * OCRT_PI / 180.0;
+        const double s1 = sin(lat) * sin(lat), s2 = sin(2.0 * lat) * sin(2.0 * lat);
+        E.a45 = 9.780327 * (1.0 + 0.0053024 * s1 - 0.0000058 * s2);
+        E.q0 = 101325.0 / above_g45(E.a45, 0.0);
+        E.ft = clamp01d((0.3734 / above_g45(E.a45, 84852.0)) / E.q0);
+        E.a45_f = (float)E.a45; E.q0_f = (float)E.q0; E.ft_f = (float)E.ft;
+    }
 }
 
-__device__ inline double above_exp(double z, double h, double et)
+// slope, where given: d/dz in FP32
+__device__ inline double above_exp(double z, double h, double et, float *slope = nullptr)
 {
+    if (slope) *slope = 0.f;
     if (z <= 0.0) return 1.0;
     if (z >= OCRT_ZTOP_KM) return 0.0;
-    return (exp(-z / h) - et) / (1.0 - et);
+    const double e = exp(-z / h);
+    if (slope) *slope = -(float)e / ((float)h * (1.f - (float)et));
+    return (e - et) / (1.0 - et);
 }
 
-__device__ inline double above_ray(const AboveEval &E, double z)
+__device__ inline double above_ray(const AboveEval &E, double z, float *slope = nullptr)
 {
-    if (E.prof == 1) return above_exp(z, E.rh, E.et_r);
+    if (E.prof == 1) return above_exp(z, E.rh, E.et_r, slope);
+    if (slope) *slope = 0.f;
     if (z <= 0.0) return 1.0;
     if (z >= 84.852) return 0.0;
-    const double Z[8] = {0.0, 11.0, 20.0, 32.0, 47.0, 51.0, 71.0, 84.852};
-    int lo = 0, hi = 7;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (z < Z[mid]) hi = mid; else lo = mid;
-    }
-    const double t = (z - Z[lo]) / (Z[hi] - Z[lo]);
-    const double a = E.lp[lo], b = E.lp[hi];
-    const double raw = clamp01d((exp(a + t * (b - a)) / above_g45(E, z * 1000.0)) / E.q0);
+    int lo = 0;
+#pragma unroll
+    for (int i = 1; i < 7; ++i) lo += z >= E.z[i];
+    const double dz = E.z[lo + 1] - E.z[lo], dp = E.lp[lo + 1] - E.lp[lo];
+    const double t = (z - E.z[lo]) / dz;
+    const double g = above_g45(E.a45, z * 1000.0);
+    const double raw = clamp01d((exp(E.lp[lo] + t * dp) / g) / E.q0);
+    if (slope) *slope = (float)raw * ((float)dp / (float)dz + 3.086e-3f / (float)g) / (1.f - E.ft_f);
     return clamp01d((raw - E.ft) / (1.0 - E.ft));
 }
 
+// the same to FP32 accuracy
+__device__ inline float above_exp_f(float z, float h, float et) { return (__expf(-z / h) - et) / (1.f - et); }
+
+__device__ inline float above_ray_f(const AboveEval &E, float z)
+{
+    if (E.prof == 1) return above_exp_f(z, E.rh_f, E.et_r_f);
+    if (z >= 84.852f) return 0.f;
+    int lo = 0;
+#pragma unroll
+    for (int i = 1; i < 7; ++i) lo += z >= E.z_f[i];
+    const float t = __fdividef(z - E.z_f[lo], E.z_f[lo + 1] - E.z_f[lo]);
+    const float raw = __expf(E.lp_f[lo] + t * (E.lp_f[lo + 1] - E.lp_f[lo])) / ((E.a45_f - 3.086e-3f * z) * E.q0_f);
+    return (raw - E.ft_f) / (1.f - E.ft_f);
+}
+
 // ---- generalized spherical functions (rt_angular_basis.c:19-124) ----
+__host__ __device__ inline double gsf_diag_factor(int i, int m) { return sqrt((double)(i + m) / (double)i) * 0.5; }
+
 __host__ __device__ inline double gsf_diag_norm(int m)
 {
     double v = 1.0;
-    for (int i = 1; i <= m; ++i) v *= sqrt((double)(i + m) / (double)i) * 0.5;
+    for (int i = 1; i <= m; ++i) v *= gsf_diag_factor(i, m);
     return v;
 }
 
-// The x-independent coefficients of the step l -> l + 1 (l >= max(2, m)):
-// c = {f, b, sc, dc, cc} of the scalar and spin-2 three-term recurrences.
+// Norms of the start values (m >= 2): of P, and of R and T, from dn = gsf_diag_norm(m).
+__host__ __device__ inline void gsf_start_norms(int m, double dn, double *c)
+{
+    c[0] = dn;
+    c[1] = dn * sqrt((double)m / (double)(m + 1)) * sqrt((double)(m - 1) / (double)(m + 2));
+}
+
+// The x-independent coefficients of the step l -> l + 1 (l >= max(2, m)) of the
+// scalar and spin-2 three-term recurrences
+//   p2 = f x p1 - fb p0,   r2 = sc x r1 - scc t1 - sdc r0,   t2 = sc x t1 - scc r1 - sdc t0:
+// c = {f, fb, sc, sdc, scc}.
 __host__ __device__ inline void gsf_step_coefs(int l, int m, double *c)
 {
     c[0] = (2.0 * l + 1.0) / sqrt((double)(l + m + 1) * (double)(l - m + 1));
-    c[1] = sqrt((double)(l + m) * (double)(l - m)) / (2.0 * l + 1.0);
+    c[1] = c[0] * sqrt((double)(l + m) * (double)(l - m)) / (2.0 * l + 1.0);
     c[2] = (double)(l + 1) * (double)(2 * l + 1) /
            sqrt((double)(l + 3) * (double)(l - 1) * (double)(l + m + 1) * (double)(l - m + 1));
-    c[3] = sqrt((double)(l + 2) * (double)(l - 2) * (double)(l + m) * (double)(l - m)) /
+    c[3] = c[2] * sqrt((double)(l + 2) * (double)(l - 2) * (double)(l + m) * (double)(l - m)) /
            ((double)l * (double)(2 * l + 1));
-    c[4] = 2.0 * (double)m / ((double)l * (double)(l + 1));
+    c[4] = c[2] * (2.0 * (double)m / ((double)l * (double)(l + 1)));
 }
 
 // Runs the scalar and spin-2 recurrences for one direction cosine x and
 // hands every degree l = 0..L to sink(l, P, R, T).  ctab, when given, holds
-// gsf_step_coefs(l, m) at ctab[5 l] (k_gsf_coefs), so the steps need no
-// square root or division.
+// gsf_step_coefs(l, m) at ctab[5 l] and gsf_start_norms(m) at ctab[0]
+// (k_gsf_coefs), so the steps need no square root or division; the
+// coefficients of four steps are loaded ahead.
 template <class Sink>
 __device__ inline void gsf_recur(int L, int m, double x, Sink sink, const double *ctab = nullptr)
 {
@@ -180,29 +184,48 @@ __device__ inline void gsf_recur(int L, int m, double x, Sink sink, const double
         r0 = 0.0; r1 = -x * s * 0.5;
         t0 = 0.0; t1 = -s * 0.5;
     } else {
-        const double dn = gsf_diag_norm(m);
-        p0 = 0.0; p1 = dn * pow(1.0 - x * x, 0.5 * (double)m);
-        const double sn = dn * sqrt((double)m / (double)(m + 1)) * sqrt((double)(m - 1) / (double)(m + 2));
-        const double env = pow(1.0 - x * x, 0.5 * (double)m - 1.0);
-        r0 = 0.0; r1 = sn * (1.0 + x * x) * env;
-        t0 = 0.0; t1 = sn * 2.0 * x * env;
+        double nrm[2];
+        if (ctab) { nrm[0] = __ldg(ctab); nrm[1] = __ldg(ctab + 1); }
+        else gsf_start_norms(m, gsf_diag_norm(m), nrm);
+        const double s2 = 1.0 - x * x, env = pow(s2, 0.5 * (double)m - 1.0);
+        p0 = 0.0; p1 = nrm[0] * env * s2;
+        r0 = 0.0; r1 = nrm[1] * (1.0 + x * x) * env;
+        t0 = 0.0; t1 = nrm[1] * 2.0 * x * env;
     }
     if (l0 - 1 <= L) sink(l0 - 1, p0, r0, t0);
     if (l0 <= L) sink(l0, p1, r1, t1);
-    for (int l = l0; l < L; ++l) {
-        double k[5];
-        if (ctab) {
-#pragma unroll
-            for (int q = 0; q < 5; ++q) k[q] = ctab[5 * l + q];
-        } else {
-            gsf_step_coefs(l, m, k);
-        }
-        const double f = k[0], b = k[1], sc = k[2], dc = k[3], cc = k[4];
-        const double p2 = f * (x * p1 - b * p0);
-        const double r2 = sc * (x * r1 - cc * t1 - dc * r0);
-        const double t2 = sc * (x * t1 - cc * r1 - dc * t0);
+    // the terms in degree l - 1 first: a dependent FP64 operation takes ~100
+    // cycles, and two of them are a step's chain
+    auto step = [&](int l, const double *k) {
+        const double fx = k[0] * x, sx = k[2] * x;
+        const double p2 = fma(fx, p1, -(k[1] * p0));
+        const double r2 = fma(sx, r1, fma(-k[4], t1, -(k[3] * r0)));
+        const double t2 = fma(sx, t1, fma(-k[4], r1, -(k[3] * t0)));
         p0 = p1; p1 = p2; r0 = r1; r1 = r2; t0 = t1; t1 = t2;
         sink(l + 1, p2, r2, t2);
+    };
+    if (!ctab) {
+        for (int l = l0; l < L; ++l) {
+            double k[5];
+            gsf_step_coefs(l, m, k);
+            step(l, k);
+        }
+        return;
+    }
+    double kn[20];
+    auto load = [&](int l) {
+#pragma unroll
+        for (int q = 0; q < 20; ++q) kn[q] = __ldg(ctab + min(5 * l + q, 5 * L - 1));
+    };
+    if (l0 < L) load(l0);
+    for (int l = l0; l < L; l += 4) {
+        double k[20];
+#pragma unroll
+        for (int q = 0; q < 20; ++q) k[q] = kn[q];
+        if (l + 4 < L) load(l + 4);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (l + i < L) step(l + i, k + 5 * i);
     }
 }
 

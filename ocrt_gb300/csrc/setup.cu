@@ -14,25 +14,39 @@
 #include "physics.cuh"
 #include "tables.cuh"
 
+// One thread per node; one block.  A chain of dependent FP64 operations: with
+// the step P_{q+1} = t P_q + q/(q+1) (t P_q - P_{q-1}) and its ratios tabulated
+// first it is two operations long instead of a division's dozens, and from the
+// second-order start below Newton ends after two or three passes.  The error of
+// the nodes (1.5e-16) and weights is that of the three-term form with divisions.
+// 32 streams: 33 us, 155 us before.
 __global__ void k_gauss(int N, double *mu, double *w, float *pw)
 {
+    __shared__ double ratio[2 * 64];
+    const int order = 2 * N;
+    for (int q = threadIdx.x; q < order; q += blockDim.x) ratio[q] = (double)q / (double)(q + 1);
+    __syncthreads();
     const int k = threadIdx.x + 1;               // 1..N (largest root first)
     if (k > N) return;
-    const int order = 2 * N;
-    double t = cos(OCRT_PI * ((double)k - 0.25) / ((double)order + 0.5));
-    double pn = 0, pm = 0, dp = 1;
+    const double no = (double)order;
+    double t = cos(OCRT_PI * ((double)k - 0.25) / (no + 0.5)) * (1.0 - (1.0 - 1.0 / no) / (8.0 * no * no));
+    double a, b;
+    auto legendre = [&]() {
+        a = 1.0; b = t;
+        for (int q = 1; q < order; ++q) {
+            const double tb = t * b, c = fma(ratio[q], fma(t, b, -a), tb);
+            a = b; b = c;
+        }
+    };
     for (int it = 0; it < 100; ++it) {
-        double a = 1.0, b = t;
-        for (int q = 1; q < order; ++q) { const double c = ((2.0 * q + 1.0) * t * b - (double)q * a) / (double)(q + 1); a = b; b = c; }
-        pn = b; pm = a;
-        dp = (double)order * (t * pn - pm) / (t * t - 1.0);
-        const double step = -pn / dp;
+        legendre();
+        const double step = -b * (t * t - 1.0) / (no * (t * b - a));
         t += step;
-        if (fabs(step) < 1.0e-15 * (fabs(t) + 1.0)) break;
+        // what is left is about step^2 t / (1 - t^2), below 1e-17 from here
+        if (fabs(step) < 1.0e-10) break;
     }
-    double a = 1.0, b = t;
-    for (int q = 1; q < order; ++q) { const double c = ((2.0 * q + 1.0) * t * b - (double)q * a) / (double)(q + 1); a = b; b = c; }
-    dp = (double)order * (t * b - a) / (t * t - 1.0);
+    legendre();
+    const double dp = no * (t * b - a) / (t * t - 1.0);
     mu[N - k] = t;
     w[N - k] = 2.0 / ((1.0 - t * t) * dp * dp);
     // surface-operator weights (2 pi or pi) mu w, rounded once (rt_surface_boundary.c:137-208)
@@ -79,75 +93,93 @@ __global__ void k_pixel_setup(PixDev *px, int P, int N, const double *gmu)
     d.rough = d.surf_on && !d.flat;
 }
 
-// One thread per (pixel, level).  Altitude of each level by 64-step
-// bisection on the column above (rt_molecular_profile.c:84-105, rt_atm.c:313-355);
-// every level brackets [0, 100 km] independently.
-__global__ void k_levels(const PixDev *px, int P, double *h, double *ch, double *xd, double *yd, double *z)
+// Altitude of each level, the root of (column above z) = its optical depth
+// (rt_molecular_profile.c:84-105, rt_atm.c:313-355), then the scattering
+// fractions of the layer above it; one thread per (pixel, level).  FP64 runs at
+// two lanes a clock and SM, so the count of FP64 evaluations of the column is
+// what costs: an FP32 bisection finds the root to ~1e-5 km, and Newton steps of
+// the FP64 column (derivative in FP32, bracketed) take it to rounding in two or
+// three evaluations where a bisection down to adjacent doubles takes 26.  A block
+// takes LEV_B - 1 levels and, for the layer differences, redoes the level above
+// its first; small blocks put even one pixel's levels on several SMs.
+// 192 pixels x 200 levels: 148 us, 1700 + 127 us before (levels and fractions);
+// one pixel at 400: 34 us, 430 + 34 us before.
+__global__ void __launch_bounds__(LEV_B) k_levels(const PixDev *px, int P, double *h, double *ch, double *xd, double *yd, double *z)
 {
+    __shared__ AboveEval E;
+    __shared__ double sray[LEV_B], saer[LEV_B];
     const int p = blockIdx.y;
     if (p >= P) return;
     const PixDev &d = px[p];
     if (d.medium == 1) return;
-    const int nt = d.nt;
+    const int nt = d.nt, tid = threadIdx.x;
+    const int k = blockIdx.x * (LEV_B - 1) + tid - 1;
+    if ((int)blockIdx.x * (LEV_B - 1) > nt) return;
     const double tau = d.tau_total, tr = d.tau_r;
-    const int aer = d.mom_off >= 0 && d.tau_a > 0.0;
+    const bool aer = d.mom_off >= 0 && d.tau_a > 0.0;
     const double ta = aer ? d.tau_a : 0.0;
     const double ah = d.aer_h_km > 0.0 ? d.aer_h_km : 2.0;
-    AboveEval E;
-    above_init(E, d.profile, d.ray_h_km, ah);
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k <= nt; k += gridDim.x * blockDim.x) {
+    above_init(E, d.profile, d.ray_h_km, ah, tid);
+    __syncthreads();
+    const bool in = k >= 0 && k <= nt;
+    if (in) {
         const long long o = d.lev_off + k;
         const double hk = (double)k * tau / (double)nt;
-        h[o] = hk;
-        ch[o] = 0.5 * exp(-hk / d.mu0);
         double zk;
         if (k == 0) zk = OCRT_ZTOP_KM;
         else if (k == nt && aer) zk = 0.0;
         else {
-            const double ztop = (!aer && d.profile == 0) ? 84.852 : OCRT_ZTOP_KM;
+            const double top = (!aer && d.profile == 0) ? 84.852 : OCRT_ZTOP_KM;
             const double f = hk / tau;
             if (!aer && f >= 1.0) zk = 0.0;
             else {
-                double lo = 0.0, hi = aer ? OCRT_ZTOP_KM : ztop;
-                const double target = aer ? hk : f;
-                auto above_at = [&](double zz) {
-                    return aer ? tr * above_ray(E, zz) + ta * above_exp(zz, ah, E.et_a) : above_ray(E, zz);
-                };
-                // Illinois steps (regula falsi that halves the value of an end
-                // kept twice) narrow the bracket while keeping the bisection's
-                // invariant above(lo) > target >= above(hi), until it is ~1e-12
-                // wide relative; the bisection below then ends, as a full
-                // 64-step bisection from [0, top] does, on the two adjacent
-                // doubles around the crossing, in ~26 evaluations of the
-                // column fraction instead of ~58.  Where the computed fraction
-                // is not monotone in its last bits the two can end a few ulps
-                // apart (1.2e-15 relative at most over 60k levels of random
-                // profiles, 99.5% identical).
-                double flo = above_at(lo) - target, fhi = above_at(hi) - target;
-                int side = 0;
-                for (int it = 0; it < 40 && hi - lo > 1e-12 * hi; ++it) {
-                    double c = hi - fhi * (hi - lo) / (fhi - flo);
-                    if (!(c > lo && c < hi)) c = 0.5 * (lo + hi);
-                    const double fc = above_at(c) - target;
-                    if (fc > 0.0) { lo = c; flo = fc; if (side < 0) fhi *= 0.5; side = -1; }
-                    else { hi = c; fhi = fc; if (side > 0) flo *= 0.5; side = 1; }
+                // above(z) = wr ray(z) + wa exp(z); decreasing, above(0) > target >= above(top)
+                const double target = aer ? hk : f, wr = aer ? tr : 1.0, wa = aer ? ta : 0.0;
+                const float ft = (float)target, fr = (float)wr, fa = (float)wa;
+                float zlo = 0.f, zhi = (float)top;
+                for (int it = 0; it < 22; ++it) {
+                    const float c = 0.5f * (zlo + zhi);
+                    if (fr * above_ray_f(E, c) + fa * above_exp_f(c, E.ah_f, E.et_a_f) > ft) zlo = c; else zhi = c;
                 }
-                // Once the midpoint equals an end, every later step leaves
-                // 0.5 (lo + hi) at that midpoint, so the loop can stop there.
-                zk = 0.5 * (lo + hi);
+                double lo = 0.0, hi = top;
+                zk = 0.5 * ((double)zlo + (double)zhi);
                 for (int it = 0; it < 64; ++it) {
-                    const double mid = 0.5 * (lo + hi);
-                    zk = mid;
-                    if (mid == lo || mid == hi) break;
-                    if (above_at(mid) > target) lo = mid; else hi = mid;
-                    zk = 0.5 * (lo + hi);
+                    float sr, sa;
+                    const double v = (wr != 0.0 ? wr * above_ray(E, zk, &sr) : (sr = 0.f, 0.0)) +
+                                     (wa != 0.0 ? wa * above_exp(zk, ah, E.et_a, &sa) : (sa = 0.f, 0.0));
+                    const double df = v - target;
+                    if (df > 0.0) lo = zk; else hi = zk;
+                    double zn = zk - df / (double)(fr * sr + fa * sa);
+                    if (!(zn >= lo && zn <= hi)) zn = 0.5 * (lo + hi);
+                    const double step = fabs(zn - zk);
+                    zk = zn;
+                    // the next step would be ~1e-6 of this one (FP32 derivative) or its square
+                    if (step <= 1e-10 * zk) break;
                 }
             }
         }
-        z[o] = zk;
-        double x = 0.0, y = 1.0;
         if (aer) {
-            if (k == 0) { x = tr == 0.0 ? d.ssa_a : 0.0; y = tr == 0.0 ? 0.0 : 1.0; }
+            sray[tid] = tr * above_ray(E, zk);
+            saer[tid] = ta * above_exp(zk, ah, E.et_a);
+        }
+        if (tid > 0) {
+            z[o] = zk;
+            h[o] = hk;
+            ch[o] = 0.5 * exp(-hk / d.mu0);
+        }
+    }
+    __syncthreads();
+    if (in && tid > 0) {
+        const long long o = d.lev_off + k;
+        double x = 0.0, y = 1.0;
+        if (aer && k == 0) {
+            x = tr == 0.0 ? d.ssa_a : 0.0;
+            y = tr == 0.0 ? 0.0 : 1.0;
+        } else if (aer) {
+            const double dr = sray[tid] - (k == 1 ? 0.0 : sray[tid - 1]);
+            const double da = saer[tid] - (k == 1 ? 0.0 : saer[tid - 1]), dt = dr + da;
+            if (dt > 0.0) { x = da * d.ssa_a / dt; y = dr / dt; }
+            else { x = 0.0; y = tr > 0.0 ? 1.0 : 0.0; }
         }
         xd[o] = x;
         yd[o] = y;
@@ -171,27 +203,6 @@ __global__ void k_levels_water(const PixDev *px, int P, double *h, double *ch, d
         xd[o] = d.w_omega_p;
         yd[o] = d.w_omega_w;
         z[o] = 0.0;
-    }
-}
-
-// Layer scattering fractions once every level altitude is known.
-__global__ void k_level_mix(const PixDev *px, int P, const double *z, double *xd, double *yd)
-{
-    const int p = blockIdx.y;
-    if (p >= P) return;
-    const PixDev &d = px[p];
-    if (d.medium == 1 || !(d.mom_off >= 0 && d.tau_a > 0.0)) return;
-    const double tr = d.tau_r, ta = d.tau_a, ah = d.aer_h_km > 0.0 ? d.aer_h_km : 2.0;
-    for (int k = 1 + blockIdx.x * blockDim.x + threadIdx.x; k <= d.nt; k += gridDim.x * blockDim.x) {
-        const long long o = d.lev_off + k;
-        const double zj = z[o], zp = z[o - 1];
-        const double rj = tr * ray_above(zj, d.profile, d.ray_h_km);
-        const double aj = ta * exp_above(zj, OCRT_ZTOP_KM, ah);
-        const double rp = k == 1 ? 0.0 : tr * ray_above(zp, d.profile, d.ray_h_km);
-        const double ap = k == 1 ? 0.0 : ta * exp_above(zp, OCRT_ZTOP_KM, ah);
-        const double dr = rj - rp, da = aj - ap, dt = dr + da;
-        if (dt > 0.0) { xd[o] = da * d.ssa_a / dt; yd[o] = dr / dt; }
-        else { xd[o] = 0.0; yd[o] = tr > 0.0 ? 1.0 : 0.0; }
     }
 }
 
@@ -243,11 +254,10 @@ __global__ void k_coef_quads(const PixDev *px, int P, int N, int NR, const float
     }
 }
 
-// GSF basis at the Gauss nodes for every mode: B[(m*(L+1) + l)*N + g], 3 arrays.
 // Per-layer overrides (ocrt_layers): optical depths replace the uniform level
 // grid (prefix sum in FP64, one thread per pixel) and the layer albedos
 // rescale the scattering fractions of the layer's bottom level.  Runs after
-// k_level_mix, so the mixing fractions stay those of the uniform grid.
+// k_levels, so the mixing fractions stay those of the uniform grid.
 __global__ void k_layers_apply(PixDev *px, int P, const double *ldt, const double *lss, double *h, double *ch,
                                double *xd, double *yd, int *err)
 {
@@ -310,6 +320,7 @@ __global__ void k_coef_deriv(const PixDev *px, int P, int N, const double *gmu, 
     }
 }
 
+// GSF basis at the Gauss nodes for every mode: B[(m*(L+1) + l)*N + g], 3 arrays.
 __global__ void k_basis_gauss(int N, int M, int L, const double *gmu, float *Bp, float *Br, float *Bt,
                               const double *gcoef)
 {
@@ -324,19 +335,33 @@ __global__ void k_basis_gauss(int N, int M, int L, const double *gmu, float *Bp,
 }
 
 // Step coefficients of the GSF recurrences for every (m, l) of a group:
-// gcoef[(m * (L + 1) + l) * 5 ..] = gsf_step_coefs(l, m) for max(2, m) <= l < L.
-__global__ void k_gsf_coefs(int M, int L, double *gcoef)
+// gcoef[(m * (L + 1) + l) * 5 ..] = gsf_step_coefs(l, m) for max(2, m) <= l < L,
+// and the start values' norms gsf_start_norms(m) at l = 0 (a product over
+// 1..m, here by a block: as a loop of each basis thread it was the longer part
+// of their time at high m).
+__global__ void __launch_bounds__(128) k_gsf_coefs(int M, int L, double *gcoef)
 {
-    const int m = blockIdx.x;
+    __shared__ double part[128];
+    const int m = blockIdx.x, tid = threadIdx.x;
     if (m > M) return;
+    double *c = gcoef + (size_t)m * (L + 1) * 5;
     const int l0 = m < 2 ? 2 : m;
-    for (int l = l0 + threadIdx.x; l < L; l += blockDim.x)
-        gsf_step_coefs(l, m, gcoef + ((size_t)m * (L + 1) + l) * 5);
+    for (int l = l0 + tid; l < L; l += blockDim.x) gsf_step_coefs(l, m, c + 5 * l);
+    double v = 1.0;
+    for (int i = 1 + tid; i <= m; i += blockDim.x) v *= gsf_diag_factor(i, m);
+    part[tid] = v;
+    for (int k = 64; k >= 1; k >>= 1) {
+        __syncthreads();
+        if (tid < k) part[tid] *= part[tid + k];
+    }
+    if (tid == 0 && m >= 2) gsf_start_norms(m, part[0], c);
 }
 
 // GSF basis at the solar direction (-mu0) and at the E zero-weight slots for
 // every task of a wave: Bx[((t*(1+E) + which)*3 + comp)*(L+1) + l], which 0 =
-// sun, 1 + e = slot N + e.
+// sun, 1 + e = slot N + e.  A serial FP64 recurrence per thread, bound by the
+// FP64 issue rate of an SM: blocks of one warp spread a few tasks over many SMs.
+// One pixel, 17 modes, L = 120: 67 us, 155 us before; 3264 tasks 101 us, 252 before.
 __global__ void k_basis_pix(const TaskDev *tasks, int t0, int nt_tasks, const PixDev *px, int L, int E, float *Bx,
                             const double *gcoef)
 {
@@ -349,7 +374,7 @@ __global__ void k_basis_pix(const TaskDev *tasks, int t0, int nt_tasks, const Pi
     const PixDev &d = px[tk.pix];
     const double x = which == 0 ? -d.mu0 : d.xmu[which - 1];
     float *dst = Bx + ((size_t)tl * W + which) * 3 * (L + 1);
-    for (int l = 0; l <= L; ++l) { dst[l] = 0.f; dst[L + 1 + l] = 0.f; dst[2 * (L + 1) + l] = 0.f; }
+    for (int l = d.L + 1; l <= L; ++l) { dst[l] = 0.f; dst[L + 1 + l] = 0.f; dst[2 * (L + 1) + l] = 0.f; }
     gsf_recur(d.L, tk.m, x, [&](int l, double P, double R, double T) {
         dst[l] = (float)P; dst[L + 1 + l] = (float)R; dst[2 * (L + 1) + l] = (float)T;
     }, gcoef ? gcoef + (size_t)tk.m * (L + 1) * 5 : nullptr);
