@@ -622,7 +622,7 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
         (rc = alloc(g.h, g.nlev)) || (rc = alloc(g.ch, g.nlev)) || (rc = alloc(g.xd, g.nlev)) ||
         (rc = alloc(g.yd, g.nlev)) || (rc = alloc(g.z, g.nlev)) || (rc = alloc(g.tabs, g.any_gas ? g.nlev : 1)) ||
         (rc = alloc(g.Tc, g.ncoef)) || (rc = alloc(g.Ca, g.ncoef)) || (rc = alloc(g.Cb, g.ncoef)) ||
-        (scan4_allowed(g.N) && (rc = alloc(g.Cq, g.ncoef / G.NR * (size_t)coef_quad_width(G.NR)))) ||
+        (!g.fused && scan4_allowed(g.N) && (rc = alloc(g.Cq, g.ncoef / G.NR * (size_t)coef_quad_width(G.NR)))) ||
         (rc = alloc(g.Bp, (size_t)(g.Mmax + 1) * (g.Lmax + 1) * g.N)) ||
         (rc = alloc(g.Br, (size_t)(g.Mmax + 1) * (g.Lmax + 1) * g.N)) ||
         (rc = alloc(g.Bt, (size_t)(g.Mmax + 1) * (g.Lmax + 1) * g.N)) ||
@@ -908,7 +908,8 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
         LAUNCH(plan, KC_SETUP, k_gas_apply<<<P, 256, 0, st>>>(g.px, P, g.h, g.ch, g.xd, g.yd, g.z, g.tabs));
     if (g.any_layers)
         LAUNCH(plan, KC_SETUP, k_layers_apply<<<P, 256, 0, st>>>(g.px, P, g.ldt, g.lss, g.h, g.ch, g.xd, g.yd, g.err));
-    LAUNCH(plan, KC_SETUP, k_coef<<<dim3(16, P), 256, 0, st>>>(g.px, P, g.N, G.NR, g.gmu, g.h, g.Tc, g.Ca, g.Cb));
+    LAUNCH(plan, KC_SETUP, k_coef<<<dim3(16, P), 256, 0, st>>>(g.px, P, g.N, G.NR, g.gmu, g.h, g.Tc, g.Ca, g.Cb,
+                                                             g.fused ? 1 : 0));
     if (g.Cq)
         LAUNCH(plan, KC_SETUP, k_coef_quads<<<dim3(16, P), 256, 0, st>>>(g.px, P, g.N, G.NR, g.Tc, g.Ca, g.Cb, g.Cq));
     LAUNCH(plan, KC_SETUP, k_gsf_coefs<<<g.Mmax + 1, 128, 0, st>>>(g.Mmax, g.Lmax, g.gcoef));
@@ -948,7 +949,7 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
     const int poll = 4;
     // ---- transport-scan implementation: forced, tuned, or being tuned ----
     std::vector<int> scan_cands;
-    if (!g.Cq || g.fused) {
+    if (!g.Cq) {
         scan_cands.push_back(SK_COLUMN);
     } else {
         scan_cands.push_back(SK_QUAD);
@@ -1091,14 +1092,15 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
             CK(cudaMemsetAsync(g.active_cnt + (itd - 1), 0, sizeof(int), st));
             CK(cudaMemsetAsync(g.mol_cnt + (itd - 1), 0, sizeof(int), st));
         }
-        if (g.Cq && !w.any_flat && !primary_column())
-            LAUNCH(plan, KC_PRIMARY, k_primary4<<<nw, scan4_threads(G), 0, st>>>(B, W, G, w.t0));
-        else
-            LAUNCH(plan, KC_PRIMARY, k_primary<<<nw, scan_threads, 0, st>>>(B, W, G, w.t0));
-        if (g.fused)
+        if (g.fused) {
             LAUNCH(plan, KC_SOURCE_TC, orders_launch(false, or_grid, st, B, W, G, w.t0, nw, w.Kmax, g.popt, g.molc, g.ocnt + 1));
-        else
+        } else {
+            if (g.Cq && !w.any_flat && !primary_column())
+                LAUNCH(plan, KC_PRIMARY, k_primary4<<<nw, scan4_threads(G), 0, st>>>(B, W, G, w.t0));
+            else
+                LAUNCH(plan, KC_PRIMARY, k_primary<<<nw, scan_threads, 0, st>>>(B, W, G, w.t0));
             LAUNCH(plan, KC_PRIMARY, k_compact<<<1, COMPACT_THREADS, 0, st>>>(B, w.t0, nw, 2));
+        }
         for (int it = 2; !g.fused && it <= g.max_orders; ++it) {
             if (w.n_simt)
                 LAUNCH(plan, KC_SOURCE, k_source_simt<<<sgrid, 256, 0, st>>>(B, W, G, w.t0, it));

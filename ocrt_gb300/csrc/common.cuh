@@ -68,7 +68,10 @@ struct PixDev {
     double mu0, mu_view, tau_r, tau_total;
     int n_ring, view_slot;  // view_slot: ring slot holding mu_view, -1 = interpolate
     int flat, rough, surf_on;
-    int pad_;
+    // order 1 (k_level_float): surface seed pi mu0 exp(-tau / mu0); flat surface's
+    // Fresnel factors and 0.5 exp(-2 tau / mu0) of the reflected beam
+    float seed0;
+    double beam_RI, beam_RQ, beam_sb;
 };
 
 struct TaskDev {

@@ -13,7 +13,7 @@ static inline int lev_blocks(int nt) { return (nt + LEV_B - 1) / (LEV_B - 1); }
 __global__ void k_levels(const PixDev *px, int P, double *h, double *ch, double *xd, double *yd, double *z);
 __global__ void k_levels_water(const PixDev *px, int P, double *h, double *ch, double *xd, double *yd, double *z);
 __global__ void k_coef(const PixDev *px, int P, int N, int NR, const double *gmu, const double *h,
-                       float *Tc, float *Ca, float *Cb);
+                       float *Tc, float *Ca, float *Cb, int first = 0);
 __global__ void k_coef_quads(const PixDev *px, int P, int N, int NR, const float *Tc, const float *Ca, const float *Cb,
                              float *Cq);
 // gcoef (k_gsf_coefs, (M + 1) (L + 1) 5 doubles) or nullptr: the recurrences'
@@ -125,7 +125,7 @@ __global__ void k_coef_deriv(const PixDev *px, int P, int N, const double *gmu, 
 __global__ void k_cs_table(int M, int nphi, float *cs);
 __global__ void k_flat_fresnel(const PixDev *px, int P, int N, const double *gmu, float *frs);
 __global__ void k_seed_att(const PixDev *px, int P, int N, const double *gmu, const double *h, float *E);
-__global__ void k_level_float(const PixDev *px, int P, const double *xd, const double *yd, const double *ch, float *lvf);
+__global__ void k_level_float(PixDev *px, int P, const double *xd, const double *yd, const double *ch, float *lvf);
 
 // sos.cu
 #define ST_M_TILE 64

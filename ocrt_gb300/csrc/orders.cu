@@ -49,13 +49,14 @@
 //
 // Roles (16 warps, one CTA per SM; four warps per scheduler, so 128 registers a
 // thread):
-//   warps 0-3    upward scan (TMEM lane quadrant = warp), boundary condition
-//   warps 4-7    downward scan
+//   warps 0-3    order 1 and upward scan (TMEM lane quadrant = warp)
+//                (the direction that ends at the surface sums its boundary condition)
+//   warps 4-7    the same downward
 //   warps 8-14   producers, 16 levels each: field rows of a tile and one incoming Stokes
 //                component (loaded a stage ahead) -> F+-, split, swizzled
 //                K-major B tile (128-byte rows: [F+ 32 | F- 32]) of a 2-stage ring
-//   warp 15      loads the task's operator (one bulk copy), issues the MMAs
-// Thread 0 fetches tasks and posts one command per order (continue, new task,
+//   warp 15      issues the MMAs
+// Thread 0 fetches tasks, starts the copy of a task's operator and posts one command per order (continue, new task,
 // stop) when the order's field is complete.
 //
 // Every wait is bounded (TC_WAIT_NS): a warp whose wait runs out raises the
@@ -211,6 +212,112 @@ __device__ __forceinline__ void or_tile_run(const Scan &c, Col &v, int what, uin
     v.I = I; v.Jp = Jp; v.mi = mi;
 }
 
+// Order 1 of a row: what its source, surface seed and outside source are made of.
+struct Prim {
+    float fa, fm;                     // aerosol and molecular factors of the direct-beam source
+    double fA, fM, sb;                // and of the beam a flat surface reflects, 0.5 exp(-2 tau / mu0)
+    float tdn, rs, ex;                // seed factors (rough surface), bottom source
+    const float *ea;                  // attenuation of the surface's light per level, or null
+    const float *lv;                  // level fractions and direct beam
+    const double *hh;                 // level optical depths
+    double mu0;
+    bool flat, jd;                    // reflected beam; skylight source in J
+};
+
+// Order 1: direct beam (rt_primary_source.c:17-198), its reflection by a flat
+// surface, the water column's skylight source, then the recurrence, and on top
+// of the upward radiance the seeds of the direct beam off a rough surface
+// (rt_surface_boundary.c:430-493) and of an outside bottom source (495-527).
+// Tile by tile in the order of the recurrence, the level constants staged in
+// shared memory (pc, 6 OR_TS floats of this direction; pe, the attenuations of
+// the upward one, NR per level), eight levels at a time.  Like or_tile_run one short code
+// for both directions and every case: a level that does not step (the column's
+// first, those past its end) has the weights of a step that changes nothing.
+template <int LDC>
+__device__ __forceinline__ float or_first(const Scan &c, const Prim &p, int h, int T, float *pc, float *pe, int tid,
+                                          int g)
+{
+    const int nt = c.nt, K = nt + 1, dk = h == 0 ? -1 : 1;
+    float *plc = pc, *plx = pc + OR_TS, *ply = pc + 2 * OR_TS;
+    double *pbm = reinterpret_cast<double *>(pc + 4 * OR_TS);
+    const float T0 = c.T, A0 = c.sg * c.Ca, B0 = c.sg * c.Cb;      // the source carries its own sign here
+    float I = 0.f, Jp = 0.f;
+#pragma unroll 1
+    for (int q = 0; q < T; ++q) {
+        const int k0 = (h == 0 ? T - 1 - q : q) * OR_TS, n = min(OR_TS, K - k0);
+        or_bar(2 + h, 128);
+        if (tid < n) {
+            const float *l = p.lv + 3 * (k0 + tid);
+            plx[tid] = l[0]; ply[tid] = l[1]; plc[tid] = l[2];
+            if (p.flat) pbm[tid] = p.sb * exp(p.hh[k0 + tid] / p.mu0);
+        }
+        if (p.ea) {
+            const float *s = p.ea + (size_t)k0 * c.NR;
+#pragma unroll 8
+            for (int x = tid; x < n * c.NR; x += 128) pe[x] = __ldg(s + x);
+        }
+        or_bar(2 + h, 128);
+        if (!c.ok) continue;
+#pragma unroll 1
+        for (int x0 = 0; x0 < n;) {
+            int plain = c.uni && !p.jd && !p.flat, lit = p.ea != nullptr;
+            asm volatile("" : "+r"(plain), "+r"(lit));
+            const int i0 = h == 0 ? n - 1 - x0 : x0, kb = k0 + i0;
+            float *dst = c.F + (size_t)kb * LDC;
+            if (plain && x0 + 8 <= n && q + x0 > 0) {
+                // eight levels of a uniform column that all step
+                float v[8];
+#pragma unroll
+                for (int r = 0; r < 8; ++r) v[r] = lit ? pe[(i0 + dk * r) * c.NR + g] : 0.f;
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const int i = i0 + dk * r;
+                    const float j = prim_source(plc[i], plx[i], ply[i], p.fa, p.fm);
+                    I = prim_step(T0, I, A0, j, B0, Jp);
+                    Jp = j;
+                    v[r] = I + __fmul_rn(__fmul_rn(p.tdn, v[r]), p.rs) + __fmul_rn(p.ex, v[r]);
+                }
+                if (c.st) {
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) dst[dk * r * LDC] = v[r];
+                }
+                x0 += 8;
+                continue;
+            }
+            // up to four levels of any column; the column's first level holds the
+            // start value, and a step past the end changes nothing
+            const int cnt = min(4, n - x0), w0 = (h == 0 ? kb : kb - 1) * c.NR;
+            const bool first = q + x0 == 0;
+            float J[4], wT[4], wA[4], wB[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const bool step = r < cnt && !(first && r == 0);
+                J[r] = p.jd && r < cnt ? c.Js[(size_t)(kb + dk * r) * LDC] : 0.f;
+                wT[r] = step ? T0 : 1.f; wA[r] = step ? A0 : 0.f; wB[r] = step ? B0 : 0.f;
+                if (!c.uni && step) {
+                    const int w = w0 + dk * r * c.NR;
+                    wT[r] = __ldg(c.wT + w); wA[r] = __ldg(c.wA + w); wB[r] = __ldg(c.wB + w);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                if (r < cnt) {
+                    const int i = i0 + dk * r;
+                    float j = __fadd_rn(prim_source(plc[i], plx[i], ply[i], p.fa, p.fm), J[r]);
+                    if (p.flat && !(first && r == 0))
+                        j += (float)(pbm[i] * ((double)plx[i] * p.fA + (double)ply[i] * p.fM));
+                    I = prim_step(wT[r], I, wA[r], j, wB[r], Jp);
+                    Jp = j;
+                    const float e = lit ? pe[i * c.NR + g] : 0.f;
+                    if (c.st) dst[dk * r * LDC] = I + __fmul_rn(__fmul_rn(p.tdn, e), p.rs) + __fmul_rn(p.ex, e);
+                }
+            }
+            x0 += cnt;
+        }
+    }
+    return I;
+}
+
 struct Bars { uint64_t *bfull, *bempty, *tfull, *tempty, *order, *op, *fin; volatile int *abort; };
 
 __device__ __noinline__ void or_wait_slow(uint64_t *bar, uint32_t parity, volatile int *abort)
@@ -298,7 +405,7 @@ __device__ __forceinline__ Col or_order(const Scan &c, Col v, const Bars &b, uin
 
 } // namespace
 
-// SRC = false: every order from the second on, of every task.  SRC = true: the
+// SRC = false: every order of every task.  SRC = true: the
 // source of the field at hand into J, once per task (the water column's
 // skylight, k_dtop_field).
 template <bool SRC, int LDC>
@@ -361,26 +468,35 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
         const int c = g < NR ? col_of(G, s, h, g) : 0;
         const int f0 = 3 * NR;
         uint32_t U = 0;
-        int step = 0, nxt = 0;
+        int step = 0, nxt = 0, nop = 0;
         if (tid == 0) nxt = atomicAdd(counter, 1);
         for (;;) {
-            if (tid == 0) {
-                // a task that ends with order 1 needs nothing here
-                while (!SRC && nxt < nw && B.px[B.tasks[t0 + nxt].pix].max_orders <= 1) nxt = atomicAdd(counter, 1);
-                *cur_s = nxt < nw && !*b.abort ? nxt : -1;
-            }
+            if (tid == 0) *cur_s = nxt < nw && !*b.abort ? nxt : -1;
             or_bar(1, 256);
             const int tl = *cur_s;
-            if (tid == 0) {
-                cmd[step & 1] = tl < 0 ? -1 : 2 * tl + 1;
-                mbar_arrive(b.order);
-                if (tl >= 0) nxt = atomicAdd(counter, 1);
+            if (tl < 0) {
+                if (tid == 0) {
+                    cmd[step & 1] = -1;
+                    mbar_arrive(b.order);
+                    // an operator copy in flight lands before the CTA leaves
+                    if (nop && !mbar_wait(b.op, (nop - 1) & 1)) *b.abort = 1;
+                }
+                break;
             }
-            if (tl < 0) break;
             const TaskDev &tk = B.tasks[t0 + tl];
             const PixDev &d = B.px[tk.pix];
             const int nt = d.nt, K = nt + 1, T = (K + OR_TS - 1) / OR_TS;
-            const bool water = d.medium == 1, mol = tk.m <= 2;
+            const bool water = d.medium == 1, mol = tk.m <= 2, more = SRC || d.max_orders > 1;
+            if (tid == 0) {
+                nxt = atomicAdd(counter, 1);
+                if (more) {
+                    // the task's operator, behind order 1; its shared memory is
+                    // free, every product of the task before has been consumed
+                    mbar_expect_tx(b.op, 9 * a_tile);
+                    bulk_g2s(sA, popt + (size_t)tl * par_bytes(G), 9 * a_tile, b.op);
+                    ++nop;
+                }
+            }
             const float *lv = B.lvf + 3 * d.lev_off;
             for (int k = tid; mol && k < K + OR_GRP; k += 256) {
                 xs[k] = k < K ? lv[3 * k] : 0.f;
@@ -412,11 +528,6 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
             float *Tot = W.Tot + tk.fld_off + c;
             float2 t_top = make_float2(0.f, 0.f), t_bot = t_top;
             float t_one = 0.f;
-            if (sc.ok) {
-                t_top = make_float2(Tot[0], W.Ttl[tot_tail_off(tk, G, 0, c)]);
-                t_bot = make_float2(Tot[(size_t)nt * LDC], W.Ttl[tot_tail_off(tk, G, nt, c)]);
-                if (G.tot_all) t_one = Tot[LDC];
-            }
             // the boundary is fed by the radiance going down at the bottom
             // (atmosphere) or going up at the top (under the water surface)
             const bool src = h == (water ? 0 : 1), dst = !src && (water || d.surf_on);
@@ -452,11 +563,54 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
                 }
                 bcx[at * 128 + row] = a;
             };
-            if (src && surf) boundary(step & 1, sc.ok ? sc.F[water ? 0 : (size_t)nt * LDC] : 0.f);
+            if (!SRC) {
+                Prim p;
+                const float *pv = W.pvec + (size_t)tl * 2 * LDC + c;
+                // an atmosphere driven only by a bottom source has no solar primary and no
+                // surface seeds (rt_solver.c:949-954, rt_surface_boundary.c:553-569)
+                const bool sun = sc.ok && !d.bottom_only, ext = d.ext_off >= 0 && tk.m <= d.ext_mmax;
+                p.fa = sun ? pv[0] : 0.f;
+                p.fm = sun ? pv[LDC] : 0.f;
+                p.flat = d.flat && !d.bottom_only;
+                p.fA = p.fM = 0.0;
+                if (p.flat && sc.ok) {
+                    // Stokes s of the reflected beam uses kernel components (s, s + 3)
+                    const float *fa = W.fvec + ((size_t)tl * 4 + 2 * h) * 6 * NR, *fm = fa + 6 * NR;
+                    p.fA = d.beam_RI * fa[s * NR + g] + d.beam_RQ * fa[(s + 3) * NR + g];
+                    p.fM = d.beam_RI * fm[s * NR + g] + d.beam_RQ * fm[(s + 3) * NR + g];
+                }
+                p.sb = d.beam_sb;
+                const bool seed = d.rough && h == 0 && sun, extb = d.medium == 0 && ext && h == 0 && sc.ok;
+                p.tdn = p.rs = p.ex = 0.f;
+                if (seed) {
+                    p.tdn = (tk.m == 0 ? 1.f : 0.5f) * d.seed0;
+                    p.rs = W.srf[tk.srf_off + G.srf_sun + g * 9 + s * 3];
+                }
+                if (extb) p.ex = (float)B.ext[d.ext_off + ((size_t)tk.m * NR + g) * 3 + s];
+                p.ea = (d.rough && !d.bottom_only || d.medium == 0 && ext) && h == 0 ? B.Eatt + d.lev_off * NR : nullptr;
+                p.lv = lv; p.hh = B.h + d.lev_off; p.mu0 = d.mu0;
+                p.jd = water && ext;
+                const float I1 = or_first<LDC>(sc, p, h, T, xi + h * 2 * 3 * OR_TS, reinterpret_cast<float *>(sB), tid & 127, gc);
+                if (!isfinite(I1)) atomicExch(B.err, OCRT_ERR_NONFINITE);
+                // totals at the two ends: the column's start value 0 and its end value, and the seeds
+                auto lit = [&](float I, int k) {
+                    const float e = p.ea ? __ldg(p.ea + (size_t)k * NR + gc) : 0.f;
+                    return df_add(df_add(make_float2(I, 0.f), __fmul_rn(__fmul_rn(p.tdn, e), p.rs)), __fmul_rn(p.ex, e));
+                };
+                t_top = lit(h == 0 ? I1 : 0.f, 0);
+                t_bot = lit(h == 0 ? 0.f : I1, nt);
+                if (G.tot_all && sc.ok && sc.st) t_one = sc.F[LDC];
+                if (src && surf && more) boundary(step & 1, sc.ok ? I1 : 0.f);
+            }
             float resid = 0.f;
             int it = 2, conv = 0;
+            if (!more) { it = 1; conv = 1; }
             or_bar(1, 256);
-            for (;; ++it) {
+            if (more && tid == 0) {
+                cmd[step & 1] = 2 * tl + 1;
+                mbar_arrive(b.order);
+            }
+            for (; more; ++it) {
                 const float bc = !SRC && dst && sc.ok ? bcx[(step & 1) * 128 + row] : 0.f;
                 Col v{bc, 0.f, 0.f};
                 float *xh = xi + h * 2 * 3 * OR_TS;
@@ -600,7 +754,6 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
         // single lane an MMA took 119 cycles to issue, twice its run time).
         uint32_t gi = 0, U = 0, nop = 0;
         int K = 0, T = 0;
-        bool op_out = false;                              // an operator copy in flight
         const bool two = N > 16;                          // two 16-deep steps per parity
         const uint32_t sa = smem_u32(sA) >> 4, sb = smem_u32(sB) >> 4, at = a_tile >> 4;
         const uint64_t dbase = sdesc_sw128(0);            // layout bits; addresses are below 2^18
@@ -610,19 +763,10 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
             const int cm = cmd[step & 1];
             if (cm < 0) break;
             if (cm & 1) {
-                const int tl = cm >> 1;
-                K = B.tasks[t0 + tl].K;
+                K = B.tasks[t0 + (cm >> 1)].K;
                 T = (K + OR_TS - 1) / OR_TS;
-                // the operator's shared memory is free: every product of the
-                // task before has been consumed
-                if (lane == 0) {
-                    mbar_expect_tx(b.op, 9 * a_tile);
-                    bulk_g2s(sA, popt + (size_t)tl * par_bytes(G), 9 * a_tile, b.op);
-                }
-                __syncwarp();
                 or_wait(b, b.op, nop & 1);
-                op_out = __any_sync(0xffffffffu, *b.abort != 0);
-                if (op_out) break;
+                if (__any_sync(0xffffffffu, *b.abort != 0)) break;
                 ++nop;
             }
             bool stop = false;
@@ -662,9 +806,7 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
             }
             if (stop) break;
         }
-        // an operator copy still in flight lands, and every MMA completes,
-        // before the CTA leaves
-        if (op_out) (void)mbar_wait(b.op, nop & 1);
+        // every MMA completes before the CTA leaves
         if (elect_one()) umma_commit(b.fin);
         __syncwarp();
         if (!mbar_wait(b.fin, 0)) *b.abort = 1;

@@ -211,12 +211,13 @@ __global__ void k_levels_water(const PixDev *px, int P, double *h, double *ch, d
 // (the reference's slope/intercept form of rt_layer_transport.c:89-99 expanded,
 // which keeps every weight non-negative).  Computed in FP64, stored FP32.
 __global__ void k_coef(const PixDev *px, int P, int N, int NR, const double *gmu, const double *h,
-                       float *Tc, float *Ca, float *Cb)
+                       float *Tc, float *Ca, float *Cb, int first)
 {
     const int p = blockIdx.y;
     if (p >= P) return;
     const PixDev &d = px[p];
-    const int total = d.nt * NR;
+    // layers of equal depth have the weights of the first: all that k_orders reads
+    const int total = (first && !d.gas && !d.has_dtau ? 1 : d.nt) * NR;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
         const int layer = e / NR, g = e - layer * NR;
         const long long o = d.coef_off + e;
@@ -1015,12 +1016,21 @@ __global__ void k_seed_att(const PixDev *px, int P, int N, const double *gmu, co
 }
 
 // FP32 copies of the per-level scattering fractions and direct beam, read at
-// every (level, column) by the order-loop kernels.
-__global__ void k_level_float(const PixDev *px, int P, const double *xd, const double *yd, const double *ch, float *lvf)
+// every (level, column) by the order-loop kernels, and the pixel's constants of
+// order 1, once the column's depth is final.
+__global__ void k_level_float(PixDev *px, int P, const double *xd, const double *yd, const double *ch, float *lvf)
 {
     const int p = blockIdx.y;
     if (p >= P) return;
-    const PixDev &d = px[p];
+    PixDev &d = px[p];
+    if (blockIdx.x == 0 && threadIdx.x == 0 && d.medium == 0) {
+        const double n2 = d.n_water * d.n_water, mu0 = d.mu0, tn = sqrt(n2 - 1.0 + mu0 * mu0);
+        const double rp = (n2 * mu0 - tn) / (n2 * mu0 + tn), rs = (mu0 - tn) / (mu0 + tn);
+        d.seed0 = (float)(OCRT_PI * mu0 * exp(-d.tau_total / mu0));
+        d.beam_RI = (rp * rp + rs * rs) / 2.0;
+        d.beam_RQ = d.q_conv == 1 ? (rp * rp - rs * rs) / 2.0 : (rs * rs - rp * rp) / 2.0;
+        d.beam_sb = 0.5 * exp(-2.0 * d.tau_total / mu0);
+    }
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k <= d.nt; k += gridDim.x * blockDim.x) {
         const long long o = d.lev_off + k;
         lvf[3 * o + 0] = (float)xd[o];

@@ -45,3 +45,33 @@ def test_orders_match_oracle_and_separate_passes(gpu, oracle, monkeypatch, N, la
     for i, c in enumerate(cases):
         ref = oracle.solve_layers(c, o, aers[i], ly[i].dtau, None)
         assert_parity({k: got[k][i] for k in ("rho_I", "rho_Q", "rho_U")}, ref, f"N={N} layers={layers} pixel {i}")
+
+
+@pytest.mark.parametrize("layers", [2, 7, 8, 112, 113, 226])
+@pytest.mark.parametrize("max_orders", [1, 2])
+def test_first_order(gpu, oracle, monkeypatch, max_orders, layers):
+    """Order 1 inside the kernel (eight levels at a time, and up to four where a
+    column starts, ends or is not plain): tasks that end with it or go one order
+    on, every surface over even and uneven layers, same bounds."""
+    from ocrt_gb300 import _abi as A
+    from synthetic import hg_aerosol_moments
+    rng = np.random.default_rng(layers)
+    mom = hg_aerosol_moments(0.7, 40)
+    cases, ly = [], []
+    for i, surface in enumerate(("black_fresnel_ocean", "black", "flat") * 2):
+        cases.append(A.default_case(surface=surface, sza_deg=rng.uniform(5, 70), vza_deg=rng.uniform(0, 60),
+                                    raa_deg=rng.uniform(0, 180), wind_speed=rng.uniform(1, 10), wavelength_nm=555.0))
+        dt = rng.uniform(0.5, 1.5, layers) * 0.3 / layers if i >= 3 else None
+        ly.append(A.LayersHolder(layers, dt, None))
+    aer = A.AerosolHolder(0.2, 0.95, *mom)
+    o = A.default_opts(n_mu=24, n_layers=layers, fourier_m_max=3, max_orders=max_orders, tolerance=1e-7)
+    monkeypatch.delenv("OCRT_GB_SOURCE_KERNEL", raising=False)
+    got, _ = gpu.solve_batch_adjoint(cases, o, [aer] * 6, ly, None)
+    monkeypatch.setenv("OCRT_GB_SOURCE_KERNEL", "simt")
+    sep, _ = gpu.solve_batch_adjoint(cases, o, [aer] * 6, ly, None)
+    np.testing.assert_allclose(got["rho_I"], sep["rho_I"], rtol=1e-5, atol=0)
+    for k in ("rho_Q", "rho_U"):
+        np.testing.assert_allclose(got[k], sep[k], rtol=0, atol=1e-6)
+    for i, c in enumerate(cases):
+        ref = oracle.solve_layers(c, o, aer, ly[i].dtau, None)
+        assert_parity({k: got[k][i] for k in ("rho_I", "rho_Q", "rho_U")}, ref, f"layers={layers} pixel {i}")
