@@ -552,6 +552,7 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
     if (g.fused) {
         g.G.srf_rp = (3 * G.NR + 31) & ~31;
         g.G.srf_sun = 3 * G.N * g.G.srf_rp;
+        g.G.direct = g.any_water;
     }
     const size_t srf_elems = (size_t)g.G.srf_sun + (size_t)G.NR * 9;
     g.T = task;

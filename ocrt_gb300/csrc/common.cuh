@@ -111,6 +111,7 @@ struct Geom {
     // with the outgoing rows contiguous (surface row so * N + o, zero-weight
     // slots 3N + 3 (o - N) + so), which the fused order kernel reads coalesced.
     int srf_rp, srf_sun;
+    int direct;             // k_orders' operator and field in the direct form (else parity form)
 };
 
 __host__ __device__ inline int srf_row(const Geom &G, int o, int so)

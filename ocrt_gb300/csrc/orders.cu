@@ -29,16 +29,28 @@
 // xi_0), which give the molecular source as row factor x xi.
 //
 // Measured, 192 pixels x 17 modes at 32 streams and 200 levels (32420
-// order-modes, rough surface, aerosol): 6.7 ms for all orders against 16.7 ms
-// of source and scan passes; 24 streams, which the tensor-core source does not
-// take, 3.7 ms against 19 ms of CUDA-core source, molecular and scan passes; one
-// pixel at 400 levels 0.38 ms against 1.4 ms.  What bounds it is an order's serial
-// chain (field rows back from L2, split, three stages of MMA per tile, recurrence,
-// boundary, residual): about 39 000 cycles at 265 levels where the MMAs alone
-// take 13 000 (1440 per tile and component) and the recurrence 8 500 (32 per
-// level); with one task a CTA these overlap only within the task.
+// order-modes, rough surface, aerosol): 7.4 ms for all orders against 19.2 ms
+// of order-1, source and scan passes; 24 streams, which the tensor-core source
+// does not take, 4.0 ms against 20 ms of CUDA-core source, molecular, order-1 and
+// scan passes; one pixel at 400 levels 0.40 ms against 1.7 ms.  What bounds it is an
+// order's serial chain (field rows back from L2, split, three stages of MMA per
+// tile, recurrence, boundary, residual): about 39 000 cycles at 265 levels where
+// the MMAs alone take 13 000 (1440 per tile and component) and the recurrence
+// 8 500 (32 per level); with one task a CTA these overlap only within the task.
+// Order 1 is 0.7 ms of it.
 // Against FP64 solves (240 pixels, 24 streams) the reflectance error is 9.3e-7
 // rms, 9.4e-7 with FP32 CUDA-core products.
+//
+// Direct form (G.direct, groups with water columns).  Where the phase function is
+// so forward-peaked that A+ and A- nearly cancel in what goes up, and the order
+// sum feeds on it, the rounding of D+- at the size of the forward peak shows: the
+// water-leaving reflectance of absorbing water was up to 2.9e-5 off at 32 streams.  There the
+// two blocks are S = A+ + A- and B = A+ - A-, the field enters as F_up and
+// sigma F_dn, and both outputs take both products: twice the MMAs (64 coupled
+// pixel-bands 8.6 -> 10.2 ms of this kernel), and an error of at most 8e-6 at 32
+// streams over eight such columns, 6e-6 with the separate passes.  In the atmosphere
+// the two forms are equally far from FP64 (3.2e-6 rms at 32 streams for
+// aerosols of g = 0.85..0.93), so it keeps the parity form.
 //
 // Levels run along the MMA's N, so a thread of a scan warp owns one output row
 // and finds the levels of its recurrence in consecutive TMEM columns.  Tiles
@@ -98,6 +110,9 @@ struct Scan {
     // Ca, Cb and in what the source-only pass writes.
     float sg;
     float cm, c0;                     // molecular row factors of xi_A / xi_B and xi_0
+    // source = D+ + kq D- upward, kq D+ + km D- downward: 1, -1, or in the direct
+    // form 0, 1
+    float kq, km;
     const float *xs, *ys;             // aerosol / molecular fractions per level
     const float *wT, *wA, *wB;        // per-layer weights of the slot (non-uniform columns)
     float *F, *Js;                    // field and source-spill columns
@@ -144,7 +159,7 @@ __device__ __forceinline__ void or_tile_run(const Scan &c, Col &v, int what, uin
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const float pv = __uint_as_float(P[i]), mv = __uint_as_float(M[i]);
-                J[i] = H == 0 ? pv + mv : pv - mv;
+                J[i] = H == 0 ? fmaf(c.kq, mv, pv) : fmaf(c.kq, pv, c.km * mv);
             }
             if (mol) {
 #pragma unroll
@@ -508,6 +523,8 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
             sc.uni = !d.gas && !d.has_dtau;
             sc.mol = mol;
             sc.sg = h == 1 && s == 2 ? -1.f : 1.f;
+            sc.kq = G.direct ? 0.f : 1.f;
+            sc.km = G.direct ? 1.f : -1.f;
             sc.xs = xs; sc.ys = ys; sc.nt = nt; sc.NR = NR;
             sc.F = W.F + tk.fld_off + c;
             sc.Js = W.J + tk.fld_off + c;
@@ -614,7 +631,7 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
                 const float bc = !SRC && dst && sc.ok ? bcx[(step & 1) * 128 + row] : 0.f;
                 Col v{bc, 0.f, 0.f};
                 float *xh = xi + h * 2 * 3 * OR_TS;
-                const bool odd = tk.m & 1, rb = s != 0;
+                const bool odd = (tk.m & 1) && !G.direct, rb = s != 0;
                 if (h == 0) v = or_order<0, SRC, LDC>(sc, v, b, tmem, T, K, U, xh, f0, row, lane, quad, odd, rb);
                 else v = or_order<1, SRC, LDC>(sc, v, b, tmem, T, K, U, xh, f0, row, lane, quad, odd, rb);
                 U += T;
@@ -697,16 +714,19 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
             const int si = (j >> 1) % 3, rb = r16(0) + 8 * (j & 1);
             // F+ = up + sigma down: for U the sum is F- and the difference F+
             unsigned char *tile = sB + st * OR_BSTAGE;
-            const int cs = 4 * q + (si == 2 ? 32 : 0), cd = 4 * q + (si == 2 ? 0 : 32);
+            const bool sw = si == 2 && !G.direct;
+            const int cs = 4 * q + (sw ? 32 : 0), cd = 4 * q + (sw ? 0 : 32);
+            // direct form: F_up and sigma F_dn
+            const float ka = G.direct ? 0.f : 1.f, kb = G.direct ? (si == 2 ? 1.f : -1.f) : 1.f;
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
                 uint32_t s0[3], s1[3], d0[3], d1[3];
                 const float f = d.x[x];
                 const float4 u = d.u[x], v = d.v[x];
-                split_bf16x3(f * (u.x + v.x), f * (u.y + v.y), s0);
-                split_bf16x3(f * (u.z + v.z), f * (u.w + v.w), s1);
-                split_bf16x3(f * (u.x - v.x), f * (u.y - v.y), d0);
-                split_bf16x3(f * (u.z - v.z), f * (u.w - v.w), d1);
+                split_bf16x3(f * fmaf(ka, v.x, u.x), f * fmaf(ka, v.y, u.y), s0);
+                split_bf16x3(f * fmaf(ka, v.z, u.z), f * fmaf(ka, v.w, u.w), s1);
+                split_bf16x3(f * fmaf(ka, u.x, -kb * v.x), f * fmaf(ka, u.y, -kb * v.y), d0);
+                split_bf16x3(f * fmaf(ka, u.z, -kb * v.z), f * fmaf(ka, u.w, -kb * v.w), d1);
                 unsigned char *ps = tile + par_swz(rb + 2 * x, cs), *pd = tile + par_swz(rb + 2 * x, cd);
 #pragma unroll
                 for (int p = 0; p < 3; ++p) {
@@ -789,15 +809,20 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
                         // first: the accumulator is truncated at each step, so the
                         // fewer steps it takes at full size the better
                         constexpr int pa[6] = {2, 1, 0, 1, 0, 0}, pb[6] = {0, 1, 2, 0, 1, 0};
-#pragma unroll
-                        for (int pr = 0; pr < 2; ++pr)
+#pragma unroll 1
+                        for (int x = 0; x < (G.direct ? 4 : 2); ++x) {
+                            // output half, half of the field, block of the operator
+                            const uint32_t o = G.direct ? x >> 1 : x, i = x & 1, ab = G.direct ? o ^ i : o;
+                            const uint32_t t = ta + ab * 4, u = tb + i * 4, first = G.direct ? i == 0 : 1;
 #pragma unroll
                             for (int e = 0; e < 12; ++e) {
-                                const int q = e >> 1, k = e & 1, off = pr * 4 + k * 2;
+                                const int q = e >> 1, k = e & 1;
                                 if (k && !two) continue;
-                                umma_bf16(acc + pr * 128, dbase | (ta + off + pa[q] * at),
-                                          dbase | (tb + off + pb[q] * (OR_BPIECE >> 4)), idesc, (si > 0 || e > 0) ? 1u : 0u);
+                                umma_bf16(acc + o * 128, dbase | (t + k * 2 + pa[q] * at),
+                                          dbase | (u + k * 2 + pb[q] * (OR_BPIECE >> 4)), idesc,
+                                          (si > 0 || e > 0 || !first) ? 1u : 0u);
                             }
+                        }
                         umma_commit(&b.bempty[st]);
                         if (si == 2) umma_commit(&b.tfull[slot]);
                     }

@@ -530,16 +530,16 @@ __global__ void __launch_bounds__(256, 2) k_tables(const TaskDev *tasks, int t0,
     auto emit = [&](const float *Ea, const float *Oa, int i) {
         if (popt) {
             // parity operator of k_orders: the sums themselves, as k_tables_tc lays it out
-            float v0 = Ea[0], v1 = Oa[0];
-            if (Vm) {
-                const float *v = Vm + (size_t)(1 + i) * 2 * G.NR + os;
-                v0 = 0.5f * (v[0] + v[G.NR]);
-                v1 = 0.5f * (v[0] - v[G.NR]);
-            }
+            float ce[9], co[9];
+            par_coefs(Ea, Oa, ce);
+            par_coefs(Oa, Ea, co);
             for (int pr = 0; pr < 2; ++pr) {
                 float c[9];
-                par_coefs(pr ? Oa : Ea, pr ? Ea : Oa, c);
-                c[0] = pr ? v1 : v0;
+                for (int q = 0; q < 9; ++q) c[q] = !G.direct ? (pr ? co[q] : ce[q]) : pr ? ce[q] - co[q] : ce[q] + co[q];
+                if (Vm) {
+                    const float *v = Vm + (size_t)(1 + i) * 2 * G.NR + os;
+                    c[0] = G.direct ? (pr ? v[G.NR] : v[0]) : 0.5f * (pr ? v[0] - v[G.NR] : v[0] + v[G.NR]);
+                }
                 for (int q = 0; q < 9; ++q)
                     par_put(popt + (size_t)tl * par_bytes(G), G, q % 3, srf_row(G, os, q / 3), 32 * pr + i,
                             c[q] * (float)gw[i]);
@@ -583,7 +583,10 @@ __global__ void __launch_bounds__(256, 2) k_tables(const TaskDev *tasks, int t0,
             float c[3];
             par_functional(f, m, d.depol, basis(0, i, 2), basis(1, i, 2), basis(2, i, 2), c);
             for (int si = 0; si < 3; ++si)
-                par_put(popt + (size_t)tl * par_bytes(G), G, si, 3 * G.NR + f, 32 * (m & 1) + i, c[si] * (float)gw[i]);
+                for (int pr = 0; pr < 2; ++pr)
+                    if (G.direct || pr == (m & 1))
+                        par_put(popt + (size_t)tl * par_bytes(G), G, si, 3 * G.NR + f, 32 * pr + i,
+                                (G.direct && pr && (m & 1) ? -c[si] : c[si]) * (float)gw[i]);
         }
     }
     if (molc && mol) {

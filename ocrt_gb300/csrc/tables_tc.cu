@@ -407,9 +407,15 @@ k_tables_tc(const TaskDev *tasks, int t0, int nt_tasks, const PixDev *px, Geom G
 #pragma unroll
                         for (int q = 0; q < 13; ++q) { x[q] = X[q * TT_PS + u]; y[q] = Y[q * TT_PS + u]; }
                         par_coefs(x, y, c9);
+                        if (G.direct) {                              // S = A+ + A-, B = A+ - A-
+                            float d9[9];
+                            par_coefs(y, x, d9);
+#pragma unroll
+                            for (int q = 0; q < 9; ++q) c9[q] = pr ? d9[q] - c9[q] : c9[q] + d9[q];
+                        }
                         if (Vm && i0 + u < N) {                      // the value kernel's table instead
                             const float *v = Vm + (size_t)(1 + i0 + u) * 2 * G.NR + o;
-                            c9[0] = 0.5f * (v[0] + (pr ? -v[G.NR] : v[G.NR]));
+                            c9[0] = G.direct ? (pr ? v[G.NR] : v[0]) : 0.5f * (v[0] + (pr ? -v[G.NR] : v[G.NR]));
                         }
                     };
                     float ca[9], cb[9];
@@ -424,7 +430,7 @@ k_tables_tc(const TaskDev *tasks, int t0, int nt_tasks, const PixDev *px, Geom G
                 // and the padding rows
                 for (int row = 3 * n + ew; row < Rw; row += TT_EW) {
                     const int f = row - 3 * G.NR;
-                    const bool on = m <= 2 && f >= 0 && f < 3 && pr == (m & 1);
+                    const bool on = m <= 2 && f >= 0 && f < 3 && (G.direct || pr == (m & 1));
                     float v[3][2] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
                     if (on) {
                         const size_t gb = ((size_t)m * (L + 1) + 2) * N;
@@ -433,7 +439,8 @@ k_tables_tc(const TaskDev *tasks, int t0, int nt_tasks, const PixDev *px, Geom G
                             if (i0 + u < N) {
                                 float c[3];
                                 par_functional(f, m, d.depol, Bp[gb + i0 + u], Br[gb + i0 + u], Bt[gb + i0 + u], c);
-                                v[0][u] = c[0]; v[1][u] = c[1]; v[2][u] = c[2];
+                                const float sg = G.direct && pr && (m & 1) ? -1.f : 1.f;
+                                v[0][u] = sg * c[0]; v[1][u] = sg * c[1]; v[2][u] = sg * c[2];
                             }
                     }
 #pragma unroll
