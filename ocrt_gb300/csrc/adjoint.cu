@@ -733,13 +733,13 @@ __global__ void __launch_bounds__(512) k_adj_grad(BatchBufs B, WaveBufs W, AdjBu
         const float *Fb = W.F + tk.fld_off + (size_t)nt * G.LDC, *Tb = W.Tot + tk.fld_off + (size_t)nt * G.LDC;
         const float *Lb = W.Ttl + tk.tail_off + G.LDC;
         auto Xb = [&](int cc) -> float { return xs_in_f ? Fb[cc] : (Tb[cc] - Fb[cc]) + Lb[cc]; };
-        const float *RW = A.srfW + tk.srf_off + (size_t)g * N * 9 + s * 3;
+        const float *RW = A.srfW + tk.srf_off;
         const float *pwm = B.pw + (tk.m == 0 ? 0 : N);
         float accf = 0.f;          // FP32 like the boundary condition it differentiates
         for (int i = 0; i < N; ++i) {
-            const float *Ri = RW + (size_t)i * 9;
-            accf += pwm[i] * (Ri[0] * Xb(col_of(G, 0, 1, i)) + Ri[1] * Xb(col_of(G, 1, 1, i)) +
-                              Ri[2] * Xb(col_of(G, 2, 1, i)));
+            accf += pwm[i] * (RW[srf_entry(G, g, i, s * 3)] * Xb(col_of(G, 0, 1, i)) +
+                              RW[srf_entry(G, g, i, s * 3 + 1)] * Xb(col_of(G, 1, 1, i)) +
+                              RW[srf_entry(G, g, i, s * 3 + 2)] * Xb(col_of(G, 2, 1, i)));
         }
         const double acc = accf;
         const double tdn = exp(-d.tau_total / d.mu0);

@@ -542,19 +542,22 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
     // All orders in one kernel (k_orders) for forward groups whose shape it
     // holds: faster at every size measured, from one pixel (24 streams, 40 layers:
     // 0.71 ms a solve against 1.41) to 192 pixels at 32 streams and 200 layers
-    // (15.6 ms against 25.5).  An adjoint needs the order totals of every level
-    // in its own form, and a named scan, order-1 or source implementation keeps
-    // the separate passes.
+    // (11.9 ms against 25.5), and for gradients (96 pixels x 33 modes x 3 rows:
+    // 13.8 ms against 22.8; 7 pixels at 16 streams 1.53 ms a step against 3.04).
+    // Gradients with a value kernel keep the separate passes, whose transposed
+    // operator does not rely on the symmetry of its table; so does a named scan,
+    // order-1 or source implementation.
     int kmax = 0;
     for (const PixDev &d : g.hpx) kmax = std::max(kmax, d.nt + 1);
-    g.fused = ncot == 0 && orders_supported(G, kmax) && !force_simt() &&
+    g.fused = (ncot == 0 || !g.any_vk) && orders_supported(G, kmax, ncot > 0) && !force_simt() &&
               !getenv("OCRT_GB_SCAN") && !getenv("OCRT_GB_PRIMARY");
     if (g.fused) {
         g.G.srf_rp = (3 * G.NR + 31) & ~31;
         g.G.srf_sun = 3 * G.N * g.G.srf_rp;
         g.G.direct = g.any_water;
     }
-    const size_t srf_elems = (size_t)g.G.srf_sun + (size_t)G.NR * 9;
+    // a multiple of four floats: k_orders reads whole float4s of a task's rows
+    const size_t srf_elems = ((size_t)g.G.srf_sun + (size_t)G.NR * 9 + 3) & ~(size_t)3;
     g.T = task;
     g.nlev = lev; g.ncoef = coef; g.nmom = mb.size();
     // ---- waves of whole pixels under the workspace budget ----
@@ -689,7 +692,7 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
         g.amap_ok = adj_scan_tma_maps(G, g.AF, g.ATot, g.wave_fld * g.ncot, g.Cq, g.ncoef / G.NR, &g.amap) == 0;
     g.use_tc = tc_supported(G) && !force_simt() && !g.fused;
     if (g.fused && ((rc = alloc(g.popt, (size_t)g.wave_tasks * par_bytes(G))) ||
-                    (rc = alloc(g.molc, (size_t)g.wave_tasks * OR_MOLC)) || (rc = alloc(g.ocnt, 2))))
+                    (rc = alloc(g.molc, (size_t)g.wave_tasks * OR_MOLC)) || (rc = alloc(g.ocnt, 4))))
         return rc;
     if (g.use_tc && (rc = alloc(g.opt, 2 * g.wave_ops))) return rc;
     if (g.use_tc && (rc = alloc(g.molV, (size_t)3 * 32 * G.CIN))) return rc;
@@ -805,6 +808,22 @@ AdjBufs make_adj(Group &g)
     return A;
 }
 
+// Gradients of a wave from its forward and adjoint totals.
+int adjoint_gradient(ocrt_plan *plan, Group &g, Wave &w, const BatchBufs &B, const WaveBufs &W, const AdjBufs &A,
+                     cudaStream_t st, int nw, bool xs_in_f)
+{
+    const Geom G = g.G;
+    const int grad_threads = 2 * ((3 * G.N + 3 + 31) / 32) * 32;
+    // cotangent rows per block: up to ADJ_RB while the per-warp level sums fit
+    const size_t row_smem = sizeof(float) * 3 * ((size_t)g.ntmax + 1) * (grad_threads / 32);
+    const int grad_rb = std::max(1, std::min({ADJ_RB, g.ncot, (int)((200 * 1024) / row_smem)}));
+    LAUNCH(plan, KC_ADJ_GRAD, k_adj_grad<<<nw * ((g.ncot + grad_rb - 1) / grad_rb), grad_threads, row_smem * grad_rb, st>>>(
+               B, W, A, G, w.t0, grad_rb, xs_in_f ? 1 : 0));
+    LAUNCH(plan, KC_ADJ_GRAD, k_adj_pixel<<<(w.p1 - w.p0) * g.ncot, 256, sizeof(double) * (g.ntmax + 2), st>>>(
+               B, W, A, G, w.p0, w.t0));
+    return OCRT_OK;
+}
+
 // Adjoint of one wave, right after its forward orders (the forward fields of
 // the wave are still resident).
 int run_adjoint_wave(ocrt_plan *plan, Group &g, Wave &w, const BatchBufs &B, const WaveBufs &W, cudaStream_t st,
@@ -818,6 +837,20 @@ int run_adjoint_wave(ocrt_plan *plan, Group &g, Wave &w, const BatchBufs &B, con
     // CUDA-core passes read it from F (k_adj_prep)
     const bool xs_in_f = w.n_simt > 0 || w.n_tc == 0;
     if (xs_in_f) LAUNCH(plan, KC_ADJ_TOTALS, k_adj_prep<<<nw, scan_threads, 0, st>>>(B, W, G, w.t0));
+    const AdjBufs A = make_adj(g);
+    if (g.fused) {
+        // the same over all orders of a (task, row) in one CTA
+        LAUNCH(plan, KC_ADJ_TOTALS, orders_launch(OR_SRC, std::min(nw, g_nsm), st, B, W, G, w.t0, nw, w.Kmax, g.popt, g.molc,
+                                                  g.ocnt, 1));
+        LAUNCH(plan, KC_ADJ_OTHER, k_adj_init<<<(na + 127) / 128, 128, 0, st>>>(B, A, G, w.t0, na));
+        BatchBufs Ba = B;
+        WaveBufs Wa = W;
+        Ba.state = g.Ast;
+        Wa.F = g.AF; Wa.J = g.AJ; Wa.Tot = g.ATot;
+        LAUNCH(plan, KC_ADJ_SCAN, orders_launch(OR_ADJ, std::min(na, g_nsm), st, Ba, Wa, G, w.t0, na, w.Kmax, g.popt, g.molc,
+                                                g.ocnt, g.ncot));
+        return adjoint_gradient(plan, g, w, B, W, A, st, nw, true);
+    }
     const int it = g.max_orders + 1;
     LAUNCH(plan, KC_ADJ_TOTALS, k_fill_all<<<1, 256, 0, st>>>(B, w.t0, nw, it));
     if (w.n_simt) LAUNCH(plan, KC_ADJ_TOTALS, k_source_simt<<<sgrid, 256, 0, st>>>(B, W, G, w.t0, it));
@@ -845,7 +878,6 @@ int run_adjoint_wave(ocrt_plan *plan, Group &g, Wave &w, const BatchBufs &B, con
                    g.tasks, w.t0, nw, G, g.ops, g.opsT));
         if (w.n_mol) LAUNCH(plan, KC_ADJ_OTHER, k_mol_utrans<<<nw, 256, 0, st>>>(g.tasks, w.t0, nw, G, g.ops, g.opsT));
     }
-    const AdjBufs A = make_adj(g);
     LAUNCH(plan, KC_ADJ_OTHER, k_adj_init<<<(na + 127) / 128, 128, 0, st>>>(B, A, G, w.t0, na));
     LAUNCH(plan, KC_ADJ_OTHER, k_adj_list_all<<<(nw + 255) / 256, 256, 0, st>>>(A, nw));
     const dim3 agrid(na, (w.Kmax + ST_M_TILE - 1) / ST_M_TILE, (G.LDC + ST_N_TILE - 1) / ST_N_TILE);
@@ -880,15 +912,7 @@ int run_adjoint_wave(ocrt_plan *plan, Group &g, Wave &w, const BatchBufs &B, con
     }
     if (capture && w.adj_stop != INT_MAX)
         LAUNCH(plan, KC_ADJ_OTHER, k_stop_check<<<1, 32, 0, st>>>(g.acnt + w.adj_stop, g.err + 1));
-    const int grad_threads = 2 * ((3 * G.N + 3 + 31) / 32) * 32;
-    // cotangent rows per block: up to ADJ_RB while the per-warp level sums fit
-    const size_t row_smem = sizeof(float) * 3 * ((size_t)g.ntmax + 1) * (grad_threads / 32);
-    const int grad_rb = std::max(1, std::min({ADJ_RB, g.ncot, (int)((200 * 1024) / row_smem)}));
-    LAUNCH(plan, KC_ADJ_GRAD, k_adj_grad<<<nw * ((g.ncot + grad_rb - 1) / grad_rb), grad_threads, row_smem * grad_rb, st>>>(
-               B, W, A, G, w.t0, grad_rb, xs_in_f ? 1 : 0));
-    LAUNCH(plan, KC_ADJ_GRAD, k_adj_pixel<<<(w.p1 - w.p0) * g.ncot, 256, sizeof(double) * (g.ntmax + 2), st>>>(
-               B, W, A, G, w.p0, w.t0));
-    return OCRT_OK;
+    return adjoint_gradient(plan, g, w, B, W, A, st, nw, xs_in_f);
 }
 
 // One execute of a group.  Eager (capture == false): host polls of the active
@@ -910,7 +934,7 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
     if (g.any_layers)
         LAUNCH(plan, KC_SETUP, k_layers_apply<<<P, 256, 0, st>>>(g.px, P, g.ldt, g.lss, g.h, g.ch, g.xd, g.yd, g.err));
     LAUNCH(plan, KC_SETUP, k_coef<<<dim3(16, P), 256, 0, st>>>(g.px, P, g.N, G.NR, g.gmu, g.h, g.Tc, g.Ca, g.Cb,
-                                                             g.fused ? 1 : 0));
+                                                             g.fused && !g.ncot ? 1 : 0));
     if (g.Cq)
         LAUNCH(plan, KC_SETUP, k_coef_quads<<<dim3(16, P), 256, 0, st>>>(g.px, P, g.N, G.NR, g.Tc, g.Ca, g.Cb, g.Cq));
     LAUNCH(plan, KC_SETUP, k_gsf_coefs<<<g.Mmax + 1, 128, 0, st>>>(g.Mmax, g.Lmax, g.gcoef));
@@ -1076,7 +1100,7 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
         if (w.any_top && g.fused) {
             // skylight first-scatter source of the water column (see below)
             LAUNCH(plan, KC_PRIMARY, k_dtop_field<<<nw, 256, 0, st>>>(B, W, G, w.t0));
-            LAUNCH(plan, KC_SOURCE_TC, orders_launch(true, or_grid, st, B, W, G, w.t0, nw, w.Kmax, g.popt, g.molc, g.ocnt));
+            LAUNCH(plan, KC_SOURCE_TC, orders_launch(OR_SRC, or_grid, st, B, W, G, w.t0, nw, w.Kmax, g.popt, g.molc, g.ocnt, 1));
         } else if (w.any_top) {
             // skylight first-scatter source of the water column: the source pass
             // over the unscattered skylight field, every task active, into J
@@ -1094,7 +1118,8 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
             CK(cudaMemsetAsync(g.mol_cnt + (itd - 1), 0, sizeof(int), st));
         }
         if (g.fused) {
-            LAUNCH(plan, KC_SOURCE_TC, orders_launch(false, or_grid, st, B, W, G, w.t0, nw, w.Kmax, g.popt, g.molc, g.ocnt + 1));
+            LAUNCH(plan, KC_SOURCE_TC, orders_launch(g.ncot ? OR_TOT : OR_FWD, or_grid, st, B, W, G, w.t0, nw, w.Kmax,
+                                                       g.popt, g.molc, g.ocnt, 1));
         } else {
             if (g.Cq && !w.any_flat && !primary_column())
                 LAUNCH(plan, KC_PRIMARY, k_primary4<<<nw, scan4_threads(G), 0, st>>>(B, W, G, w.t0));

@@ -387,10 +387,14 @@ size_t couple_wa_smem_bytes(int M, int NRw);
 
 // orders.cu: every order of a task in one CTA (parity operator popt from
 // k_tables_tc, molecular row factors molc[wave task][128] from k_tables)
-bool orders_supported(const Geom &G, int Kmax);
+// OR_FWD: all orders, totals at the output levels.  OR_SRC: the source of the
+// field at hand into J.  OR_TOT: all orders, totals at every level.  OR_ADJ: the
+// adjoint's orders; items (task, cotangent row), field, source, total and states
+// the adjoint's.
+enum { OR_FWD, OR_SRC, OR_TOT, OR_ADJ };
+bool orders_supported(const Geom &G, int Kmax, bool adjoint);
 size_t orders_smem_bytes(const Geom &G, int Kmax);
 cudaError_t orders_init();
-// source: k_orders_source (the source of the field at hand into J), else k_orders
-void orders_launch(bool source, int grid, cudaStream_t st, const BatchBufs &B, const WaveBufs &W, const Geom &G, int t0,
-                   int nw, int Kmax, const unsigned char *popt, const float *molc, int *counter);
+void orders_launch(int kind, int grid, cudaStream_t st, const BatchBufs &B, const WaveBufs &W, const Geom &G, int t0,
+                   int nw, int Kmax, const unsigned char *popt, const float *molc, int *counters, int ncot);
 __global__ void k_orders_reset(int *counter);

@@ -75,3 +75,42 @@ def test_first_order(gpu, oracle, monkeypatch, max_orders, layers):
     for i, c in enumerate(cases):
         ref = oracle.solve_layers(c, o, aer, ly[i].dtau, None)
         assert_parity({k: got[k][i] for k in ("rho_I", "rho_Q", "rho_U")}, ref, f"layers={layers} pixel {i}")
+
+
+@pytest.mark.parametrize("N,layers,max_orders,van", [(8, 2, 300, 1), (8, 15, 1, 1), (16, 16, 2, 0), (24, 17, 300, 1),
+                                                     (32, 31, 2, 1), (16, 111, 300, 1), (24, 112, 300, 0),
+                                                     (32, 225, 300, 1), (8, 337, 300, 1)])
+def test_adjoint_orders_match_separate_passes(gpu, monkeypatch, N, layers, max_orders, van):
+    """The adjoint's orders in one CTA against the separate transposed passes, at
+    the edges of groups, tiles and order counts, more (task, row) items than the
+    chip has SMs (a zero output row among them), even and uneven layers, the view
+    inserted, between nodes and on a node.  Both run in FP32 on the same linear
+    system, so gradients agree to 1e-5 of the largest of their group (the order
+    sums' rounding, sqrt(337) x 6e-8, and a last order of 1e-7)."""
+    from ocrt_gb300 import _abi as A
+    from synthetic import hg_aerosol_moments
+    rng = np.random.default_rng(100 * N + layers)
+    gmu = np.polynomial.legendre.leggauss(2 * N)[0][N:]
+    n = 24
+    cases, aers, ly = [], [], []
+    for i in range(n):
+        vza = np.degrees(np.arccos(gmu[N // 2])) if i == 5 else rng.uniform(0, 60)
+        cases.append(A.default_case(surface=["black", "black_fresnel_ocean"][i % 2], sza_deg=rng.uniform(5, 70),
+                                    vza_deg=vza, raa_deg=rng.uniform(0, 180), wind_speed=rng.uniform(1, 10),
+                                    wavelength_nm=555.0))
+        aers.append(A.AerosolHolder(rng.uniform(0.05, 0.4), 0.95, *hg_aerosol_moments(0.7, 24)))
+        dt = rng.uniform(0.5, 1.5, layers) * 0.3 / layers if i % 3 == 0 else None
+        ly.append(A.LayersHolder(layers, dt, None))
+    o = A.default_opts(n_mu=N, n_layers=layers, fourier_m_max=3, max_orders=max_orders, tolerance=1e-7,
+                       view_as_node=van)
+    cot = np.broadcast_to(np.eye(3), (n, 3, 3)).copy()
+    cot[1, 0] = 0.0
+    monkeypatch.delenv("OCRT_GB_SOURCE_KERNEL", raising=False)
+    r1, g1 = gpu.solve_batch_adjoint(cases, o, aers, ly, cot)
+    monkeypatch.setenv("OCRT_GB_SOURCE_KERNEL", "simt")
+    r2, g2 = gpu.solve_batch_adjoint(cases, o, aers, ly, cot)
+    np.testing.assert_allclose(r1["rho_I"], r2["rho_I"], rtol=1e-5)
+    for k in ("d_dtau", "d_ssa", "d_wind"):
+        for i in range(n):
+            scale = np.abs(g2[k][i]).max()
+            assert np.abs(g1[k][i] - g2[k][i]).max() <= 1e-5 * scale + 1e-12, (k, i)
