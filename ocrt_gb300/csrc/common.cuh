@@ -227,6 +227,21 @@ __device__ __forceinline__ void split_bf16x3(float a, float b, uint32_t *p)
         }
     }
 }
+// The same by truncation: the three pieces hold the 24 bits of a value exactly,
+// and take no conversion instructions (a quarter of the rate of logic ones).
+// All pieces have the value's sign, so products of two such splits would drop
+// their smallest terms with one sign; the other factor is split to nearest.
+__device__ __forceinline__ void split_bf16x3_trunc(float a, float b, uint32_t *p)
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        p[i] = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+        if (i < 2) {
+            a -= __uint_as_float(__float_as_uint(a) & 0xffff0000u);
+            b -= __uint_as_float(__float_as_uint(b) & 0xffff0000u);
+        }
+    }
+}
 #endif
 
 // Parity operator of the fused order kernel (orders.cu), per task: for each

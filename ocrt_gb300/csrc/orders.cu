@@ -29,16 +29,19 @@
 // xi_0), which give the molecular source as row factor x xi.
 //
 // Measured, 192 pixels x 17 modes at 32 streams and 200 levels (32420
-// order-modes, rough surface, aerosol): 7.4 ms for all orders against 19.2 ms
+// order-modes, rough surface, aerosol): 6.9 ms for all orders against 19.2 ms
 // of order-1, source and scan passes; 24 streams, which the tensor-core source
-// does not take, 4.0 ms against 20 ms of CUDA-core source, molecular, order-1 and
-// scan passes; one pixel at 400 levels 0.40 ms against 1.7 ms.  What bounds it is an
-// order's serial chain (field rows back from L2, split, three stages of MMA per
-// tile, recurrence, boundary, residual): about 39 000 cycles at 265 levels where
-// the MMAs alone take 13 000 (1440 per tile and component) and the recurrence
-// 8 500 (32 per level); with one task a CTA these overlap only within the task.
-// Order 1 is 0.7 ms of it.
-// Against FP64 solves (240 pixels, 24 streams) the reflectance error is 9.3e-7
+// does not take, 3.7 ms against 20 ms of CUDA-core source, molecular, order-1 and
+// scan passes; one pixel at 400 levels 0.38 ms against 1.7 ms.  What bounds it is an
+// order's serial chain, 29 000 cycles at 201 levels: 9 000 to the first tile (field
+// rows back from L2, then per stage 1500 to split it, 1500 of MMA and 600 of
+// barriers, two stages in flight), 6 700 to the second, 11 000 for the upward scan
+// of both (60 cycles a level while the other roles run, 48 alone), 2 500 for
+// residual and restart.  An MMA of 128 rows takes 62 cycles at 112 as at 80 levels
+// (its operands' shared-memory reads), so tiles of 80 with three stages and three
+// in TMEM were slower (7.9 ms), as were 8-level units per producer (7.4).  Order 1
+// is 0.7 ms of it.
+// Against FP64 solves (240 pixels, 24 streams) the reflectance error is 9.6e-7
 // rms, 9.4e-7 with FP32 CUDA-core products.
 //
 // Direct form (G.direct, groups with water columns).  Where the phase function is
@@ -765,6 +768,8 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
             }
             float resid = 0.f;
             int conv = 0;
+            const int max_it = d.max_orders;
+            const float tolf = __double2float_ru(d.tol);   // resid < tol as floats
             AdjIn ai{0.f, 0.f, 0.f, 0.f, nullptr};
             float mview = 0.f;                             // the view's own part of the adjoint total
             bool begin = ADJ, only = false;                // scan without a product; nothing but order 1
@@ -890,8 +895,8 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
                 if (ADJ && only) break;
                 mt = fmaxf(mt, mview);
                 resid = mt > 0.f ? mi / mt : 0.f;
-                conv = (double)resid < d.tol;
-                if (conv || it >= d.max_orders || *b.abort) break;
+                conv = resid < tolf;
+                if (conv || it >= max_it || *b.abort) break;
                 if (tid == 0) {
                     cmd[step & 1] = 2 * item + (ADJ && begin ? 1 : 0);
                     mbar_arrive(b.order);
@@ -955,10 +960,10 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
                 uint32_t s0[3], s1[3], d0[3], d1[3];
                 const float f = d.x[x];
                 const float4 u = d.u[x], v = d.v[x];
-                split_bf16x3(f * fmaf(ka, v.x, u.x), f * fmaf(ka, v.y, u.y), s0);
-                split_bf16x3(f * fmaf(ka, v.z, u.z), f * fmaf(ka, v.w, u.w), s1);
-                split_bf16x3(f * fmaf(ka, u.x, -kb * v.x), f * fmaf(ka, u.y, -kb * v.y), d0);
-                split_bf16x3(f * fmaf(ka, u.z, -kb * v.z), f * fmaf(ka, u.w, -kb * v.w), d1);
+                split_bf16x3_trunc(f * fmaf(ka, v.x, u.x), f * fmaf(ka, v.y, u.y), s0);
+                split_bf16x3_trunc(f * fmaf(ka, v.z, u.z), f * fmaf(ka, v.w, u.w), s1);
+                split_bf16x3_trunc(f * fmaf(ka, u.x, -kb * v.x), f * fmaf(ka, u.y, -kb * v.y), d0);
+                split_bf16x3_trunc(f * fmaf(ka, u.z, -kb * v.z), f * fmaf(ka, u.w, -kb * v.w), d1);
                 unsigned char *ps = tile + par_swz(rb + 2 * x, cs), *pd = tile + par_swz(rb + 2 * x, cd);
 #pragma unroll
                 for (int p = 0; p < 3; ++p) {
