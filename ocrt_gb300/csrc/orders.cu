@@ -710,12 +710,12 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
                     float a0 = 0.f, a1 = 0.f;
                     if (row < 3 * NR)
 #pragma unroll 1
-                        for (int j = 0; j < 3 * N; j += 24) {
-                            float r[24];
+                        for (int j = 0; j < 3 * N; j += 12) {
+                            float r[12];
 #pragma unroll
-                            for (int q = 0; q < 24; ++q) r[q] = __ldg(Rm + j * RP + q * RP);
+                            for (int q = 0; q < 12; ++q) r[q] = __ldg(Rm + j * RP + q * RP);
 #pragma unroll
-                            for (int q = 0; q < 24; q += 2) {
+                            for (int q = 0; q < 12; q += 2) {
                                 a0 = fmaf(r[q], fb[j + q], a0);
                                 a1 = fmaf(r[q + 1], fb[j + q + 1], a1);
                             }
@@ -1082,8 +1082,8 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
 }
 
 // The row stride is a template argument: the scan's stores and the producers'
-// loads then take immediate offsets.  Its values for N = 8, 16, 24, 32 with one
-// or four zero-weight slots; gradients have one.
+// loads then take immediate offsets.  Its values for N = 8 .. 32 with one or four
+// zero-weight slots.
 #define OR_ARGS BatchBufs B, WaveBufs W, Geom G, int t0, int nw, int Kmax, const unsigned char *popt, const float *molc, \
                 int *counter, int ncot
 template <int LDC>
@@ -1117,10 +1117,8 @@ namespace {
 
 typedef void (*OrdersFn)(OR_ARGS);
 struct OrdersInst { int ldc; OrdersFn fn[4]; };                // by OR_FWD .. OR_ADJ
-#define OR_INST(n) {n, {k_orders<n>, k_orders_source<n>, nullptr, nullptr}}
-#define OR_INST_ADJ(n) {n, {k_orders<n>, k_orders_source<n>, k_orders_total<n>, k_orders_adjoint<n>}}
-const OrdersInst g_orders[] = {OR_INST_ADJ(64), OR_INST(96), OR_INST_ADJ(128), OR_INST_ADJ(160), OR_INST(192),
-                               OR_INST_ADJ(224)};
+#define OR_INST(n) {n, {k_orders<n>, k_orders_source<n>, k_orders_total<n>, k_orders_adjoint<n>}}
+const OrdersInst g_orders[] = {OR_INST(64), OR_INST(96), OR_INST(128), OR_INST(160), OR_INST(192), OR_INST(224)};
 
 const OrdersInst *orders_inst(int ldc)
 {
@@ -1131,14 +1129,17 @@ const OrdersInst *orders_inst(int ldc)
 
 } // namespace
 
-// N a multiple of 8 keeps the producers' rows in whole float4s and the surface
-// rows in whole steps of the boundary sum; 3 NR + 3 rows fit one MMA of 128
+// N a multiple of 4 keeps the producers' rows in whole float4s and the surface
+// rows in whole steps of the boundary sum.  N = 20, which would fill five eighths
+// of its two 16-deep MMA steps, keeps the separate passes and their scan
+// autotuner; 12 and 28 take this kernel (scene of 500 pixels, 17 modes, up to 150 layers:
+// 4.9 and 8.1 ms against 10.7 and 29.6 with the separate passes).  3 NR + 3 rows fit one MMA of 128
 // (111 at 32 streams with four zero-weight slots); larger N (48 streams) would need a
 // second M tile and twice the operator, 480 KB, more than an SM has.
 bool orders_supported(const Geom &G, int Kmax, bool adjoint)
 {
     const OrdersInst *o = orders_inst(G.LDC);
-    return G.N % 8 == 0 && G.N <= 32 && 3 * G.NR + 3 <= 128 && o && (!adjoint || (G.E == 1 && o->fn[OR_ADJ])) &&
+    return (G.N % 8 == 0 || G.N % 16 == 12) && G.N <= 32 && 3 * G.NR + 3 <= 128 && o && (!adjoint || G.E == 1) &&
            orders_smem_bytes(G, Kmax) <= 227 * 1024;
 }
 
@@ -1153,7 +1154,6 @@ cudaError_t orders_init()
 {
     for (const OrdersInst &o : g_orders)
         for (OrdersFn f : o.fn) {
-            if (!f) continue;
             const cudaError_t e = cudaFuncSetAttribute((const void *)f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                        227 * 1024);
             if (e != cudaSuccess) return e;

@@ -114,3 +114,12 @@ def test_adjoint_orders_match_separate_passes(gpu, monkeypatch, N, layers, max_o
         for i in range(n):
             scale = np.abs(g2[k][i]).max()
             assert np.abs(g1[k][i] - g2[k][i]).max() <= 1e-5 * scale + 1e-12, (k, i)
+
+
+@pytest.mark.parametrize("layers", [14, 113])
+@pytest.mark.parametrize("N", [12, 28])
+def test_orders_at_multiples_of_four(gpu, oracle, monkeypatch, N, layers):
+    """Stream counts that fill neither a 16-deep MMA step nor the boundary sum's
+    steps of 8 slots: forward and adjoint, same bounds."""
+    test_orders_match_oracle_and_separate_passes(gpu, oracle, monkeypatch, N, layers)
+    test_adjoint_orders_match_separate_passes(gpu, monkeypatch, N, layers, 300, layers % 2)
