@@ -512,8 +512,8 @@ __global__ void k_adj_surface(BatchBufs B, WaveBufs W, AdjBufs A, Geom G, int t0
         const float pw = B.pw[(tk.m == 0 ? 0 : N) + i];
         float acc = 0.f;
         for (int g = 0; g < d.n_ring; ++g) {
-            const float *Rg = R + ((size_t)g * N + i) * 9 + sp;
-            acc += Rg[0] * mb[g * 3 + 0] + Rg[3] * mb[g * 3 + 1] + Rg[6] * mb[g * 3 + 2];
+            acc += R[srf_entry(G, g, i, sp)] * mb[g * 3 + 0] + R[srf_entry(G, g, i, 3 + sp)] * mb[g * 3 + 1] +
+                   R[srf_entry(G, g, i, 6 + sp)] * mb[g * 3 + 2];
         }
         A.AF[adj_off(tk, G, A.ncot, r) + (size_t)d.nt * G.LDC + col_of(G, sp, 1, i)] += pw * acc;
     }

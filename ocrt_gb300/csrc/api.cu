@@ -551,11 +551,9 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
     for (const PixDev &d : g.hpx) kmax = std::max(kmax, d.nt + 1);
     g.fused = (ncot == 0 || !g.any_vk) && orders_supported(G, kmax, ncot > 0) && !force_simt() &&
               !getenv("OCRT_GB_SCAN") && !getenv("OCRT_GB_PRIMARY");
-    if (g.fused) {
-        g.G.srf_rp = (3 * G.NR + 31) & ~31;
-        g.G.srf_sun = 3 * G.N * g.G.srf_rp;
-        g.G.direct = g.any_water;
-    }
+    g.G.srf_rp = (3 * G.NR + 31) & ~31;
+    g.G.srf_sun = 3 * G.N * g.G.srf_rp;
+    g.G.direct = g.fused && g.any_water;
     // a multiple of four floats: k_orders reads whole float4s of a task's rows
     const size_t srf_elems = ((size_t)g.G.srf_sun + (size_t)G.NR * 9 + 3) & ~(size_t)3;
     g.T = task;
@@ -827,7 +825,7 @@ int adjoint_gradient(ocrt_plan *plan, Group &g, Wave &w, const BatchBufs &B, con
 // Adjoint of one wave, right after its forward orders (the forward fields of
 // the wave are still resident).
 int run_adjoint_wave(ocrt_plan *plan, Group &g, Wave &w, const BatchBufs &B, const WaveBufs &W, cudaStream_t st,
-                     int tc_grid, int mol_grid, int mtiles, int ltiles, dim3 sgrid, size_t tc_smem, bool capture)
+                     int tc_grid, int mol_grid, int mtiles, int ltiles, int lt, dim3 sgrid, size_t tc_smem, bool capture)
 {
     const Geom G = g.G;
     const int nw = w.t1 - w.t0, na = nw * g.ncot;
@@ -861,7 +859,7 @@ int run_adjoint_wave(ocrt_plan *plan, Group &g, Wave &w, const BatchBufs &B, con
                k_source_tc_xs<<<tc_grid, tc_fwd_threads(), tc_smem, st>>>(B, W, G, w.t0, it, mtiles));
     if (w.n_mol && !w.n_tc)
         LAUNCH(plan, KC_ADJ_TOTALS, k_mol_lowrank<<<mol_grid, 256, mol_smem_bytes(G), st>>>(
-                   B, W, G, w.t0, it, ltiles, g.Bp, g.Br, g.Bt, g.Lmax));
+                   B, W, G, w.t0, it, ltiles, lt, g.Bp, g.Br, g.Bt, g.Lmax));
     // adjoint successive orders (the adjoint field, source and total are not
     // cleared: k_adj_init writes a_1's TOA row, order 1 reads no other row of
     // a_1 nor the total, and its scan zeroes the muJ columns no order writes)
@@ -904,7 +902,7 @@ int run_adjoint_wave(ocrt_plan *plan, Group &g, Wave &w, const BatchBufs &B, con
         else
             LAUNCH(plan, KC_ADJ_SOURCE, k_adj_source<<<agrid, 256, 0, st>>>(B, W, A, G, w.t0));
         if (w.n_mol && !g.use_tc_adj)
-            LAUNCH(plan, KC_ADJ_SOURCE, k_adj_mol<<<dim3(na, ltiles), 256, adj_mol_smem_bytes(G), st>>>(
+            LAUNCH(plan, KC_ADJ_SOURCE, k_adj_mol<<<dim3(na, (w.Kmax + 31) / 32), 256, adj_mol_smem_bytes(G), st>>>(
                        B, W, A, G, w.t0, g.Bp, g.Br, g.Bt, g.Lmax));
         if (w.any_rough)
             LAUNCH(plan, KC_ADJ_OTHER, k_adj_surface<<<std::min(na, 32 * g_nsm), surf_threads, 0, st>>>(B, W, A, G,
@@ -1088,7 +1086,8 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
                                              iface_smem_bytes(g.Mmax, g.nphi_ww, 0), st>>>(
                        g.tasks, g.px, w.p0, g.pix_task0, G, g.gmu, g.nphi_ww, g.srf));
         const dim3 sgrid(w.n_simt, (w.Kmax + ST_M_TILE - 1) / ST_M_TILE, (G.COUT + ST_N_TILE - 1) / ST_N_TILE);
-        const int mtiles = (w.Kmax + 127) / 128, ltiles = (w.Kmax + 31) / 32;
+        const int mtiles = (w.Kmax + 127) / 128;
+        const int lt = mol_levels(w.n_mol, w.Kmax, g_nsm), ltiles = (w.Kmax + lt - 1) / lt;
         const size_t tc_smem = tc_smem_bytes(G);
         // Persistent grids: CTAs pull (task, level tile) items from the order's
         // active list, so tasks that have converged cost nothing.
@@ -1113,7 +1112,7 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
                            B, W, G, w.t0, itd, mtiles));
             if (w.n_mol && !w.n_tc)
                 LAUNCH(plan, KC_MOL, k_mol_lowrank<<<mol_grid, 256, mol_smem_bytes(G), st>>>(
-                           B, W, G, w.t0, itd, ltiles, g.Bp, g.Br, g.Bt, g.Lmax));
+                           B, W, G, w.t0, itd, ltiles, lt, g.Bp, g.Br, g.Bt, g.Lmax));
             CK(cudaMemsetAsync(g.active_cnt + (itd - 1), 0, sizeof(int), st));
             CK(cudaMemsetAsync(g.mol_cnt + (itd - 1), 0, sizeof(int), st));
         }
@@ -1135,7 +1134,7 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
                            B, W, G, w.t0, it, mtiles));
             if (w.n_mol && !w.n_tc)
                 LAUNCH(plan, KC_MOL, k_mol_lowrank<<<mol_grid, 256, mol_smem_bytes(G), st>>>(
-                           B, W, G, w.t0, it, ltiles, g.Bp, g.Br, g.Bt, g.Lmax));
+                           B, W, G, w.t0, it, ltiles, lt, g.Bp, g.Br, g.Bt, g.Lmax));
             {
                 int kind = scan_pick;
                 const bool tuning = kind < 0;
@@ -1153,7 +1152,7 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
                     break;
                 case SK_QUAD:
                     LAUNCH(plan, KC_SCAN, k_scan4<<<scan4_grid, scan4_threads(G),
-                                                     scan4_smem_bytes(scan4_threads(G)), st>>>(B, W, G, w.t0, it));
+                                                     scan4_smem_bytes(G), st>>>(B, W, G, w.t0, it));
                     break;
                 default: {
                     const int ch = sk_ch[kind], ns = sk_ns[kind];
@@ -1221,7 +1220,7 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
             LAUNCH(plan, KC_EXTRACT, k_edges<<<(nw * G.NR + 127) / 128, 128, 0, st>>>(B, W, G, w.t0, nw, g.edge));
         if (g.any_lut) LAUNCH(plan, KC_EXTRACT, k_lut_sample<<<nw, 128, 0, st>>>(B, W, make_lut(g), G, w.t0, nw));
         if (g.ncot) {
-            const int rc = run_adjoint_wave(plan, g, w, B, W, st, tc_grid, mol_grid, mtiles, ltiles, sgrid, tc_smem,
+            const int rc = run_adjoint_wave(plan, g, w, B, W, st, tc_grid, mol_grid, mtiles, ltiles, lt, sgrid, tc_smem,
                                             capture);
             if (rc) return rc;
         }

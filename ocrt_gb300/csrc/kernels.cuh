@@ -31,8 +31,13 @@ inline size_t scan_smem_bytes(int threads) { return (size_t)SCAN_DEPTH * threads
 // as 16-byte copies; the zero-weight columns one per thread.  It applies when
 // N is a multiple of 4.
 #define SCAN4_DEPTH 8
-__host__ __device__ inline int scan4_threads(const Geom &G) { return ((6 * G.N / 4 + 6 * G.E + 31) / 32) * 32; }
-inline size_t scan4_smem_bytes(int threads) { return (size_t)SCAN4_DEPTH * 5 * threads * 16; }
+// threads: the quads, then from the next warp on the zero-weight columns
+__host__ __device__ inline int scan4_threads(const Geom &G)
+{
+    return ((6 * G.N / 4 + 31) & ~31) + ((6 * G.E + 31) & ~31);
+}
+__host__ __device__ inline int scan4_slots(const Geom &G) { return 6 * G.N / 4 + 6 * G.E; }
+inline size_t scan4_smem_bytes(const Geom &G) { return (size_t)SCAN4_DEPTH * 5 * scan4_slots(G) * 16; }
 // Transport weights in quads (k_coef_quads): per layer, per quad of ring
 // slots g = 4q..4q+3 (the ring padded to NRq = NR rounded up to 4, padding
 // zero), four T, then four Ca, then four Cb: 3 * NRq floats per layer.
@@ -157,6 +162,46 @@ __device__ inline double tot_value(const WaveBufs &W, const TaskDev &tk, const G
     const float lo = (k == 0 || k == nt) ? W.Ttl[tot_tail_off(tk, G, k, c)] : 0.f;
     return (double)hi + (double)lo;
 }
+// Boundary value of Stokes s at outgoing slot g: sum over the incoming columns of
+// the surface's row times the level's radiance Fr of hemisphere hin.  In the row
+// form of the surface kernels neighbouring columns read neighbouring addresses
+// (one coupled pixel at 48 streams and 40 levels: 33 us an order's scan, 53 with
+// [o][i][9]); eight slots are in flight at a time.
+__device__ __forceinline__ float surface_sum(const Geom &G, const float *R, const float *pwm, const float *Fr, int hin, int g,
+                                             int s)
+{
+    const int N = G.N, si = G.srf_rp ? G.srf_rp : 9, sp = G.srf_rp ? N * G.srf_rp : 1;
+    const float *p = R + srf_entry(G, g, 0, s * 3), *F0 = Fr + hin * N;
+    float acc = 0.f;
+#pragma unroll 8
+    for (int i = 0; i < N; ++i) {
+        const float *Ri = p + (size_t)i * si;
+        acc += pwm[i] * (Ri[0] * F0[i] + Ri[sp] * F0[2 * N + i] + Ri[2 * sp] * F0[4 * N + i]);
+    }
+    return acc;
+}
+// the same at slots g .. g + 3 (N a multiple of 4, row form)
+__device__ __forceinline__ void surface_sum4(const Geom &G, const float *R, const float *pwm, const float *Fr, int hin, int g,
+                                             int s, float *bc)
+{
+    const int N = G.N, si = G.srf_rp, sp = N * G.srf_rp;
+    const float *p = R + srf_entry(G, g, 0, s * 3), *F0 = Fr + hin * N;
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+    for (int i = 0; i < N; ++i) {
+        const float *Ri = p + (size_t)i * si;
+        const float4 x = *reinterpret_cast<const float4 *>(Ri), y = *reinterpret_cast<const float4 *>(Ri + sp),
+                     z = *reinterpret_cast<const float4 *>(Ri + 2 * sp);
+        const float w = pwm[i], f0 = F0[i], f1 = F0[2 * N + i], f2 = F0[4 * N + i];
+        a[0] += w * (x.x * f0 + y.x * f1 + z.x * f2);
+        a[1] += w * (x.y * f0 + y.y * f1 + z.y * f2);
+        a[2] += w * (x.z * f0 + y.z * f1 + z.z * f2);
+        a[3] += w * (x.w * f0 + y.w * f1 + z.w * f2);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) bc[q] = a[q];
+}
+
 struct BatchBufs {
     const PixDev *px;
     const TaskDev *tasks;
@@ -318,9 +363,11 @@ int adj_scan_tma_maps(const Geom &G, float *AF, float *ATot, size_t adj_floats, 
 size_t adj_scan_tma_smem_bytes(const Geom &G, int CH, int NS);
 cudaError_t adj_scan_tma_launch(int grid, cudaStream_t st, const BatchBufs &B, const AdjBufs &A, const Geom &G,
                                 int t0, int j, const AdjScanMaps &M);
-__global__ void k_mol_lowrank(BatchBufs B, WaveBufs W, Geom G, int t0, int it, int ltiles,
+// levels of a k_mol_lowrank tile for n_mol tasks of K levels on nsm SMs (four blocks each)
+inline int mol_levels(int n_mol, int K, int nsm) { return (long long)n_mol * ((K + 7) / 8) <= 4 * nsm ? 8 : 32; }
+__global__ void k_mol_lowrank(BatchBufs B, WaveBufs W, Geom G, int t0, int it, int ltiles, int lt,
                               const float *Bp, const float *Br, const float *Bt, int L);
-inline size_t mol_smem_bytes(const Geom &G) { return sizeof(float) * (4 * G.N + G.COUT * 24 + 32 * G.CIN + 32 * 25); }
+inline size_t mol_smem_bytes(const Geom &G) { return sizeof(float) * (4 * G.N + 32 * G.CIN + 32 * 24); }
 __global__ void k_extract(BatchBufs B, WaveBufs W, Geom G, int t0, int nt_tasks);
 __global__ void k_stop_check(const int *active_after_last, int *flag);
 

@@ -265,8 +265,8 @@ extern "C" int ocrt_gb_solve_case_noalloc(const ocrt_case *cs, const ocrt_opts *
         for (int it = 2; it <= opts->max_orders; ++it) {
             NA_LAUNCH(k_source_simt<<<sgrid, 256, 0, st>>>(B, W, G, t0, it));
             if (nmol > 0)
-                NA_LAUNCH(k_mol_lowrank<<<dim3(nmol * ((K + 31) / 32)), 256, mol_smem_bytes(G), st>>>(
-                    B, W, G, t0, it, (K + 31) / 32, Bp, Br, Bt, L));
+                NA_LAUNCH(k_mol_lowrank<<<dim3(nmol * ((K + 7) / 8)), 256, mol_smem_bytes(G), st>>>(
+                    B, W, G, t0, it, (K + 7) / 8, 8, Bp, Br, Bt, L));
             NA_LAUNCH(k_scan<<<nw, scan_threads, scan_smem_bytes(scan_threads), st>>>(B, W, G, t0, it));
             if ((it - 1) % 4 == 0 || it == opts->max_orders) {
                 int left_active = 0;

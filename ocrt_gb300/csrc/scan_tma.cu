@@ -220,17 +220,8 @@ __global__ void __launch_bounds__(256, 3) k_scan_tma(BatchBufs B, WaveBufs W, Ge
                 if (water || d.rough) {
                     // water: internal reflection of the previous order's upward field at the
                     // top; atmosphere: rough reflection of the downward field at the bottom
-                    const float *Rm = W.srf + tk.srf_off + (size_t)g * N * 9 + s * 3;
-                    const float *pwm = B.pw + (tk.m == 0 ? 0 : N);
-                    const float *Fr = water ? F : F + (size_t)nt * G.LDC;
-                    const int hin = water ? 0 : 1;
-                    float acc = 0.f;
-                    for (int i = 0; i < N; ++i) {
-                        const float *Ri = Rm + (size_t)i * 9;
-                        acc += pwm[i] * (Ri[0] * Fr[col_of(G, 0, hin, i)] + Ri[1] * Fr[col_of(G, 1, hin, i)] +
-                                         Ri[2] * Fr[col_of(G, 2, hin, i)]);
-                    }
-                    bc = acc;
+                    bc = surface_sum(G, W.srf + tk.srf_off, B.pw + (tk.m == 0 ? 0 : N),
+                                     water ? F : F + (size_t)nt * G.LDC, water ? 0 : 1, g, s);
                 } else {
                     const float *Fbot = F + (size_t)nt * G.LDC;
                     const float *MF = B.frs + ((size_t)tk.pix * NR + g) * 9 + s * 3;

@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(128, 4) k_primary4(BatchBufs B, WaveBufs W, Ge
     const int tl = blockIdx.x, tg = t0 + tl;
     const TaskDev tk = B.tasks[tg];
     const PixDev &d = B.px[tk.pix];
-    const int tid = threadIdx.x, N = G.N, nq = 6 * N / 4;
+    const int tid = threadIdx.x, N = G.N, nq = 6 * N / 4, sq = (nq + 31) & ~31;   // as in k_scan4
     if (tid == 0) {
         TaskState st;
         st.orders = 1;
@@ -262,8 +262,8 @@ __global__ void __launch_bounds__(128, 4) k_primary4(BatchBufs B, WaveBufs W, Ge
         const int c = 4 * tid;
         decode_col(G, c, s, h, g);
         primary_cols<4>(B, W, G, tk, d, tl, c, s, h, g, bad);
-    } else if (tid < nq + 6 * G.E) {
-        const int c = 6 * N + (tid - nq);
+    } else if (tid >= sq && tid < sq + 6 * G.E) {
+        const int c = 6 * N + (tid - sq);
         decode_col(G, c, s, h, g);
         if (g < d.n_ring) primary_cols<1>(B, W, G, tk, d, tl, c, s, h, g, bad);
     }
@@ -271,7 +271,9 @@ __global__ void __launch_bounds__(128, 4) k_primary4(BatchBufs B, WaveBufs W, Ge
 }
 
 // Tiled SIMT GEMM: per task, J[k][c] = x_k * sum_i F[k][col(i)] A[i][c] + y_k * (... B ...).
-// Tile 64 levels x 64 output columns, 256 threads, 4x4 outputs per thread.
+// Tile 64 levels x 64 output columns, 256 threads, 4x4 outputs per thread.  The next
+// chunk is loaded while one is multiplied, and a column without aerosol, whose
+// operator is zero, writes zeros (48 streams, three tasks: 5.5 us, 63 before).
 #define ST_K 16
 #define ST_M 64
 #define ST_N 64
@@ -290,20 +292,29 @@ __global__ void __launch_bounds__(256) k_source_simt(BatchBufs B, WaveBufs W, Ge
     const float *A = W.ops + tk.op_off;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     float accA[4][4] = {{0}};
-    for (int kc = 0; kc < G.CIN; kc += ST_K) {
-        for (int idx = threadIdx.x; idx < ST_M * ST_K; idx += 256) {
-            const int lv = idx / ST_K, kk = idx - lv * ST_K;
-            const int k = k0 + lv, ci = kc + kk;
-            const size_t o = (size_t)k * G.LDC + in_to_col(G, ci);
-            Fs[kk][lv] = (k <= nt && ci < G.CIN) ? F[o] : 0.f;
+    // without an aerosol the operator is zero (k_tables) and so is the product
+    const int cin = d.mom_off >= 0 && d.tau_a > 0.0 ? G.CIN : 0;
+    // the next chunk's values are loaded while this one is multiplied
+    float fn[ST_M * ST_K / 256], an[ST_N * ST_K / 256];
+    const int kk0 = threadIdx.x & (ST_K - 1), r0 = threadIdx.x / ST_K;
+    auto load = [&](int kc) {
+        const int ci = kc + kk0;
+#pragma unroll
+        for (int u = 0; u < ST_M * ST_K / 256; ++u) {
+            const int k = k0 + r0 + u * (256 / ST_K), co = c0 + r0 + u * (256 / ST_K);
+            fn[u] = (k <= nt && ci < cin) ? F[(size_t)k * G.LDC + in_to_col(G, ci)] : 0.f;
+            an[u] = (co < G.NP && ci < cin) ? A[(size_t)co * G.CIN + ci] : 0.f;
         }
-        for (int idx = threadIdx.x; idx < ST_K * ST_N; idx += 256) {
-            const int cc = idx / ST_K, kk = idx - cc * ST_K;
-            const int ci = kc + kk, co = c0 + cc;
-            const bool ok = ci < G.CIN && co < G.NP;
-            As[kk][cc] = ok ? A[(size_t)co * G.CIN + ci] : 0.f;
+    };
+    load(0);
+    for (int kc = 0; kc < cin; kc += ST_K) {
+#pragma unroll
+        for (int u = 0; u < ST_M * ST_K / 256; ++u) {
+            Fs[kk0][r0 + u * (256 / ST_K)] = fn[u];
+            As[kk0][r0 + u * (256 / ST_K)] = an[u];
         }
         __syncthreads();
+        if (kc + ST_K < cin) load(kc + ST_K);
 #pragma unroll
         for (int kk = 0; kk < ST_K; ++kk) {
             float fr[4], ar[4];
@@ -335,8 +346,10 @@ __global__ void __launch_bounds__(256) k_source_simt(BatchBufs B, WaveBufs W, Ge
 
 // Molecular source for m <= 2 tasks: xi[k][4b+f] = sum_i w_i f(mu_i) F[k][bN+i]
 // (f in {1, P2m, R2m, T2m}), then J[k][c] += y_k sum_r U[c][r] xi[k][r].
-// Grid (task in list, tile of 32 levels), 256 threads.
-__global__ void __launch_bounds__(256) k_mol_lowrank(BatchBufs B, WaveBufs W, Geom G, int t0, int it, int ltiles,
+// Grid (task in list, tile of lt <= 32 levels), 256 threads.  A block takes 56 us
+// with 32 levels and 17 with 8, its loads one behind the other; mol_levels() picks 8
+// while the chip holds all blocks, and past it 32 (U read for four times the levels).
+__global__ void __launch_bounds__(256) k_mol_lowrank(BatchBufs B, WaveBufs W, Geom G, int t0, int it, int ltiles, int lt,
                                                      const float *Bp, const float *Br, const float *Bt, int L)
 {
     extern __shared__ float sm[];
@@ -351,21 +364,20 @@ __global__ void __launch_bounds__(256) k_mol_lowrank(BatchBufs B, WaveBufs W, Ge
     const int tl = B.mlist[it & 1][item / ltiles], tg = t0 + tl;
     const TaskDev tk = B.tasks[tg];
     const PixDev &d = B.px[tk.pix];
-    const int nt = d.nt, N = G.N, k0 = (item % ltiles) * 32;
+    const int nt = d.nt, N = G.N, k0 = (item % ltiles) * lt;
     if (k0 > nt) continue;
-    const int nk = min(32, nt - k0 + 1);
-    float *fv = sm;                          // [4][N]
-    float *U = fv + 4 * N;                   // [COUT][24]
-    float *Fs = U + G.COUT * 24;             // [32][6N]
-    float *xi = Fs + 32 * G.CIN;             // [32][25]
+    const int nk = min(lt, nt - k0 + 1);
+    float *xi = sm;                          // [32][24], 16-byte rows
+    float *fv = xi + 32 * 24;                // [4][N]
+    float *Fs = fv + 4 * N;                  // [32][6N]
     const size_t gb = (size_t)tk.m * (L + 1) * N + (size_t)2 * N;    // degree-2 row of mode m
     for (int i = threadIdx.x; i < N; i += blockDim.x) {
         const float w = (float)B.gw[i];
         fv[i] = w; fv[N + i] = w * Bp[gb + i]; fv[2 * N + i] = w * Br[gb + i]; fv[3 * N + i] = w * Bt[gb + i];
     }
     const float *Ug = W.ops + tk.mol_off;
-    for (int e = threadIdx.x; e < G.COUT * 24; e += blockDim.x) U[e] = Ug[e];
     const float *F = W.F + tk.fld_off + (size_t)k0 * G.LDC;
+#pragma unroll 8
     for (int e = threadIdx.x; e < nk * G.CIN; e += blockDim.x) {
         const int k = e / G.CIN, ci = e - k * G.CIN;
         const size_t o = (size_t)k * G.LDC + ci;
@@ -378,17 +390,30 @@ __global__ void __launch_bounds__(256) k_mol_lowrank(BatchBufs B, WaveBufs W, Ge
         const float *ff = fv + f * N;
         float acc = 0.f;
         for (int i = 0; i < N; ++i) acc = fmaf(ff[i], fr[i], acc);
-        xi[k * 25 + r] = acc;
+        xi[k * 24 + r] = acc;
     }
     __syncthreads();
-    float *J = W.J + tk.fld_off;
-    for (int e = threadIdx.x; e < nk * G.COUT; e += blockDim.x) {
-        const int k = e / G.COUT, c = e - k * G.COUT;
-        const float *u = U + c * 24, *x = xi + k * 25;
-        float acc = 0.f;
+    // a thread keeps its column's row of U and walks the levels
+    float *J = W.J + tk.fld_off + (size_t)k0 * G.LDC;
+    const float *yl = B.lvf + 3 * (d.lev_off + k0) + 1;
+    for (int c = threadIdx.x; c < G.COUT; c += blockDim.x) {
+        float u[24];
 #pragma unroll
-        for (int r = 0; r < 24; ++r) acc = fmaf(u[r], x[r], acc);
-        J[(size_t)(k0 + k) * G.LDC + c] += B.lvf[3 * (d.lev_off + k0 + k) + 1] * acc;
+        for (int r = 0; r < 24; r += 4) {
+            const float4 q = *reinterpret_cast<const float4 *>(Ug + (size_t)c * 24 + r);
+            u[r] = q.x; u[r + 1] = q.y; u[r + 2] = q.z; u[r + 3] = q.w;
+        }
+#pragma unroll 8
+        for (int k = 0; k < nk; ++k) {
+            float acc = 0.f;
+#pragma unroll
+            for (int r = 0; r < 24; r += 4) {
+                const float4 x = *reinterpret_cast<const float4 *>(xi + k * 24 + r);
+                acc = fmaf(u[r], x.x, acc); acc = fmaf(u[r + 1], x.y, acc);
+                acc = fmaf(u[r + 2], x.z, acc); acc = fmaf(u[r + 3], x.w, acc);
+            }
+            J[(size_t)k * G.LDC + c] += yl[3 * k] * acc;
+        }
     }
     }
 }
@@ -495,29 +520,12 @@ __global__ void __launch_bounds__(512, 2) k_scan(BatchBufs B, WaveBufs W, Geom G
     float bc = 0.f;
     const bool water = d.medium == 1;
     if (valid && water && h == 1) {
-        const float *R = W.srf + tk.srf_off + (size_t)g * N * 9 + s * 3;
-        const float *pwm = B.pw + (tk.m == 0 ? 0 : N);
-        float acc = 0.f;
-        for (int i = 0; i < N; ++i) {
-            const float *Ri = R + (size_t)i * 9;
-            acc += pwm[i] * (Ri[0] * F[col_of(G, 0, 0, i)] + Ri[1] * F[col_of(G, 1, 0, i)] +
-                             Ri[2] * F[col_of(G, 2, 0, i)]);
-        }
-        bc = acc;
+        bc = surface_sum(G, W.srf + tk.srf_off, B.pw + (tk.m == 0 ? 0 : N), F, 0, g, s);
     } else if (valid && h == 0 && d.surf_on) {
         const float *Fbot = F + (size_t)nt * G.LDC;
         auto Fb = [&](int col) -> float { return Fbot[col]; };
         if (d.rough) {
-            const float *R = W.srf + tk.srf_off + (size_t)g * N * 9 + s * 3;
-            const float *pwm = B.pw + (tk.m == 0 ? 0 : N);
-            float acc = 0.f;
-            for (int i = 0; i < N; ++i) {
-                const float pw = pwm[i];
-                const float *Ri = R + (size_t)i * 9;
-                acc += pw * (Ri[0] * Fb(col_of(G, 0, 1, i)) + Ri[1] * Fb(col_of(G, 1, 1, i)) +
-                             Ri[2] * Fb(col_of(G, 2, 1, i)));
-            }
-            bc = acc;
+            bc = surface_sum(G, W.srf + tk.srf_off, B.pw + (tk.m == 0 ? 0 : N), Fbot, 1, g, s);
         } else {
             const float *MF = B.frs + ((size_t)tk.pix * NR + g) * 9 + s * 3;
             bc = MF[0] * Fb(col_of(G, 0, 1, g)) + MF[1] * Fb(col_of(G, 1, 1, g)) + MF[2] * Fb(col_of(G, 2, 1, g));
@@ -582,13 +590,17 @@ __global__ void __launch_bounds__(128, 4) k_scan4(BatchBufs B, WaveBufs W, Geom 
     extern __shared__ float4 scan4_smem[];
     __shared__ int item_s;
     const int n_items = B.active_cnt[it - 1];
-    const int tid = threadIdx.x, bs = blockDim.x, N = G.N, NR = G.NR, nq = 6 * N / 4;
-    const bool quad = tid < nq, single = !quad && tid < nq + 6 * G.E;
+    const int tid = threadIdx.x, bs = scan4_slots(G), N = G.N, NR = G.NR, nq = 6 * N / 4;
+    // the zero-weight columns start on a warp of their own: in one warp the two
+    // loops would run one after the other (400 levels at 48 streams: 89 us, 137 before)
+    const int sq = (nq + 31) & ~31;
+    const bool quad = tid < nq, single = tid >= sq && tid < sq + 6 * G.E;
+    const int ti = quad ? tid : nq + (tid - sq);
     int s = 0, h = 0, g = 0, c = 0;
     if (quad) { c = 4 * tid; decode_col(G, c, s, h, g); }
-    else if (single) { c = 6 * N + (tid - nq); decode_col(G, c, s, h, g); }
+    else if (single) { c = 6 * N + (tid - sq); decode_col(G, c, s, h, g); }
     float4 *R = scan4_smem;   // [SCAN4_DEPTH][5][bs]: J, total, T, Ca, Cb
-    auto slot = [&](int sl, int f) -> float4 * { return R + ((size_t)sl * 5 + f) * bs + tid; };
+    auto slot = [&](int sl, int f) -> float4 * { return R + ((size_t)sl * 5 + f) * bs + ti; };
     for (;;) {
     __syncthreads();
     if (tid == 0) item_s = atomicAdd(&B.work[it * 4 + 2], 1);
@@ -646,22 +658,18 @@ __global__ void __launch_bounds__(128, 4) k_scan4(BatchBufs B, WaveBufs W, Geom 
     const bool water = d.medium == 1;
     if (valid && ((water && h == 1) || (!water && h == 0 && d.surf_on))) {
         const float *pwm = B.pw + (tk.m == 0 ? 0 : N);
-        for (int q = 0; q < ncol; ++q) {
+        // water: internal reflection of the previous order's upward field at
+        // the top; atmosphere: rough reflection of the downward field at the bottom
+        if (water || d.rough) {
+            const float *Fr = water ? F : F + (size_t)nt * G.LDC;
+            if (quad && G.srf_rp) surface_sum4(G, W.srf + tk.srf_off, pwm, Fr, water ? 0 : 1, g, s, bc);
+            else
+                for (int q = 0; q < ncol; ++q)
+                    bc[q] = surface_sum(G, W.srf + tk.srf_off, pwm, Fr, water ? 0 : 1, g + q, s);
+        }
+        for (int q = 0; q < ncol && !(water || d.rough); ++q) {
             const int gq = g + q;
-            if (water || d.rough) {
-                // water: internal reflection of the previous order's upward field at
-                // the top; atmosphere: rough reflection of the downward field at the bottom
-                const float *Rm = W.srf + tk.srf_off + (size_t)gq * N * 9 + s * 3;
-                const float *Fr = water ? F : F + (size_t)nt * G.LDC;
-                const int hin = water ? 0 : 1;
-                float acc = 0.f;
-                for (int i = 0; i < N; ++i) {
-                    const float *Ri = Rm + (size_t)i * 9;
-                    acc += pwm[i] * (Ri[0] * Fr[col_of(G, 0, hin, i)] + Ri[1] * Fr[col_of(G, 1, hin, i)] +
-                                     Ri[2] * Fr[col_of(G, 2, hin, i)]);
-                }
-                bc[q] = acc;
-            } else {
+            {
                 const float *Fbot = F + (size_t)nt * G.LDC;
                 const float *MF = B.frs + ((size_t)tk.pix * NR + gq) * 9 + s * 3;
                 bc[q] = MF[0] * Fbot[col_of(G, 0, 1, gq)] + MF[1] * Fbot[col_of(G, 1, 1, gq)] +
