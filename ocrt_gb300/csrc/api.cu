@@ -1066,12 +1066,10 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
                                                                       g.cs, g.Mmax, g.lam, g.srf);
             };
             if (g.cmpairs) {
-                const int per = coxmunk_tc_pairs_per_cta();
-                LAUNCH(plan, KC_COXMUNK, k_coxmunk_tc<<<dim3((g.ncmpairs + per - 1) / per, np), coxmunk_tc_threads(dw),
-                                                         coxmunk_tc_smem_bytes(g.Mmax, dw), st>>>(
-                           g.tasks, g.px, w.p0, g.pix_task0, G, g.gmu, g.cs, g.cstiles, g.Mmax, g.lam,
-                           dw ? g.lamd : nullptr, g.srf, dw ? g.srfW : nullptr, g.cmpairs, g.ncmpairs, dw ? 1 : 0,
-                           g.err));
+                LAUNCH(plan, KC_COXMUNK, coxmunk_tc_launch(dw, np, g_nsm, st, g.tasks, g.px, w.p0,
+                                                           g.pix_task0, G, g.gmu, g.cs, g.cstiles, g.Mmax, g.lam,
+                                                           dw ? g.lamd : nullptr, g.srf, dw ? g.srfW : nullptr, g.cmpairs,
+                                                           g.ncmpairs, g.err));
             } else {
                 int cb = 256;
                 rc = tuned_block(dw ? "k_coxmunk_dw" : "k_coxmunk",
@@ -1279,7 +1277,7 @@ int ocrt_gb_init(int device)
     CK(cudaDeviceGetAttribute(&g_nsm, cudaDevAttrMultiProcessorCount, device));
     CK(cudaFuncSetAttribute(k_coxmunk, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(k_coxmunk_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CK(cudaFuncSetAttribute(k_coxmunk_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    CK(coxmunk_tc_init());
     CK(cudaFuncSetAttribute(k_ipss, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(k_ipss_lut, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(k_tables, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));

@@ -12,20 +12,29 @@
 // into a second accumulator.
 //
 // K is swept in chunks of 32 azimuth nodes (one 128-byte swizzle row).  For a
-// chunk every one of the 448 threads evaluates one Mueller matrix on the CUDA
-// cores (FP32, the same coxmunk_R as the CUDA-core kernel) and stores the tf32 (hi, lo)
-// split into the SWIZZLE_128B K-major A tiles, while a TMA bulk copy brings the
-// chunk's B tiles (the cos/sin table already split and swizzled once per
-// group by k_cs_tiles).  One thread then issues the three kind::tf32 MMAs per
-// 8-node slice (hi*hi + hi*lo + lo*hi).  Two stages in the plain variant: the
-// MMAs of chunk c run while chunk c + 1 is evaluated.  The wind-derivative
-// variant's stage (four A tiles) is too large for two stages at two CTAs per
-// SM, so it keeps one: a CTA's MMAs and its next chunk's evaluation
-// alternate, and the second CTA on the SM fills the gaps (two CTAs of one
-// stage ran faster than one CTA of two: the evaluation, not the MMA, is the
-// long phase).  Gauss-Gauss pairs are evaluated once per
-// reciprocal couple and written both ways, as in k_coxmunk.  Every wait is
-// bounded by TC_WAIT_NS.
+// chunk a warp evaluates the Mueller matrices of one pair, a node per lane, on the
+// CUDA cores (FP32, the same coxmunk_R as the CUDA-core kernel) and stores the tf32
+// (hi, lo) split into the SWIZZLE_128B K-major A tiles; the chunk's B tiles (the
+// cos/sin table already split and swizzled once per group by k_cs_tiles) arrive by
+// bulk copy.  One further warp waits for both and issues the three kind::tf32 MMAs
+// per 8-node slice (hi*hi + hi*lo + lo*hi).  Two stages in the plain variant: the
+// MMAs of a chunk run while the next is evaluated.  The wind-derivative variant's
+// stage (four A tiles) is too large for two stages at two CTAs per SM, so it keeps
+// one: a chunk is evaluated into registers while the MMAs of the one before run.
+// The B tiles of all chunks are 20 KB each (33 modes) and read from L2 by every CTA,
+// 5.4 GB for 384 pixels: a CTA therefore takes up to three blocks of 14 pairs, as
+// many accumulators as fit 256 TMEM columns, and uses a chunk's B for all of them.
+// Gauss-Gauss pairs are evaluated once per reciprocal couple and written both ways,
+// as in k_coxmunk.  Every wait is bounded by TC_WAIT_NS.
+//
+// Measured, 384 rough pixels, 593 pairs, 33 modes, 512 half-grid nodes: 1.60 ms, 2.84
+// with block-wide barriers between evaluation and MMA (2.16 with the issuing warp
+// apart, 2.04 with three blocks a CTA, 1.82 with azimuths loaded ahead and pair
+// constants as vectors, the rest from shared-memory addressing); with the wind
+// derivative (96 pixels) 0.71, 1.00 before; one pixel 25 us, 43 before.  It is bound by
+// instruction issue (0.7 of the peak): ~400 instructions a node and warp, of which
+// the evaluation is about 230.
+#include <algorithm>
 #include <cuda.h>
 #include <cstdint>
 #include "kernels.cuh"
@@ -35,13 +44,12 @@
 using namespace tcg;
 
 #define CMT_P 14            // pairs per CTA (9 rows each)
-#define CMT_THREADS 224     // CMT_P x CMT_KC / 2: two Mueller evaluations per thread and chunk
-#define CMT_THREADS_DW 448  // CMT_P x CMT_KC: one Mueller evaluation per thread and chunk
 #define CMT_KC 32           // azimuth nodes per chunk
+#define CMT_THREADS (CMT_P * 32 + 32)   // a warp per pair, and one that issues
 
 // Pair constants of the Mueller evaluation (coxmunk_R in physics.cuh with
 // mu_out = mo, mu_in = -mi): everything that does not depend on the azimuth.
-struct CmPair {
+struct alignas(16) CmPair {
     float mo, mi, s1, s2, musum, A2, d12, s4, s12, inv_s1, inv_s2, inv_A2, inv_musum, inv_sig2, kfac, nw, inv_nw2;
     int pole1, pole2;
 };
@@ -88,19 +96,19 @@ __device__ inline void cm_mueller(const CmPair &c, float cphi, float sphi, float
     if (cw <= 1e-6f) return;
     const float inv_cb = 2.f * cw * c.inv_musum;             // 1 / cos(beta)
     if (inv_cb >= 1e6f) return;
-    const float sT = sqrtf(fmaxf(0.f, 1.f - cT * cT));
-    const float inv_den = 1.f / fmaxf(1e-12f, sT);
+    // rotations where the sine of the scattering angle vanishes are the identity
+    const float tiny = 1e-24f * fmaxf(1e-24f, 1.f - cT * cT);
     float c1, si1, c2, si2;
     if (c.pole2) { c1 = -copysignf(1.f, c.mi) * cphi; si1 = sphi; }
     else {
         const float u = (c.mo - c.mi * cT) * c.inv_s2, v = c.s1 * sphi, n2 = u * u + v * v;
-        if (n2 * inv_den * inv_den < 1e-24f) { c1 = 1.f; si1 = 0.f; }
+        if (n2 <= tiny) { c1 = 1.f; si1 = 0.f; }
         else { const float r = rsqrtf(n2); c1 = u * r; si1 = v * r; }
     }
     if (c.pole1) { c2 = -copysignf(1.f, c.mo) * cphi; si2 = sphi; }
     else {
         const float u = (c.mi - c.mo * cT) * c.inv_s1, v = c.s2 * sphi, n2 = u * u + v * v;
-        if (n2 * inv_den * inv_den < 1e-24f) { c2 = 1.f; si2 = 0.f; }
+        if (n2 <= tiny) { c2 = 1.f; si2 = 0.f; }
         else { const float r = rsqrtf(n2); c2 = u * r; si2 = v * r; }
     }
     // Fresnel at the facet angle cos(omega) = cw
@@ -151,31 +159,39 @@ __global__ void k_cs_tiles(int Mtab, int nphi, const float *cs_tab, float *tiles
     }
 }
 
-__global__ void __launch_bounds__(CMT_THREADS_DW)
+template <bool DW>
+__global__ void __launch_bounds__(CMT_THREADS, 2)
 k_coxmunk_tc(const TaskDev *tasks, const PixDev *px, int p0, const int *pix_task0, Geom G, const double *gmu,
              const float *cs_tab, const float *cs_tiles, int Mtab, const double *lamv, const double *lamd,
-             float *srf, float *srfW, const short2 *pairs, int npairs, int dw, int *err)
+             float *srf, float *srfW, const short2 *pairs, int npairs, int nbk, int *err)
 {
-    extern __shared__ unsigned char smem_raw[];
+    constexpr bool dw = DW;
+    constexpr int NSTG = DW ? 1 : 2, NBST = NSTG;                // stages of A and of B (see above)
+    // the declared alignment keeps the pointers below known as shared memory
+    extern __shared__ __align__(1024) unsigned char cm_smem[];
     const int p = p0 + blockIdx.y;
     const PixDev &d = px[p];
     const int N = G.N, M = d.M, nphi = d.nphi, half = nphi / 2;
-    const int pr0 = blockIdx.x * CMT_P;
+    const int pr0 = blockIdx.x * CMT_P * nbk;
     if (!d.rough || pr0 >= npairs) return;
+    const int nb = min(nbk, (npairs - pr0 + CMT_P - 1) / CMT_P);      // blocks of pairs of this CTA
     const int NM = (Mtab + 1 + 7) & ~7, NN = 2 * NM;
     const uint32_t A_BYTES = 128 * CMT_KC * 4, B_BYTES = (uint32_t)NN * CMT_KC * 4;
-    const uint32_t STAGE = (dw ? 4u : 2u) * A_BYTES + 2u * B_BYTES;
-    unsigned char *base = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    const int NSTG = dw ? 1 : 2;                                 // operand stages (see above)
-    uint64_t *mma_done = (uint64_t *)(base + NSTG * STAGE);      // [2]
-    uint64_t *fin = mma_done + 2;
+    const uint32_t A_STAGE = (dw ? 4u : 2u) * A_BYTES, B_STAGE = 2u * B_BYTES;
+    unsigned char *base = cm_smem;
+    unsigned char *bbase = base + NSTG * A_STAGE;
+    uint64_t *mma_done = (uint64_t *)(bbase + NBST * B_STAGE);   // [2]
+    uint64_t *bdone = mma_done + 2;                              // [2] a chunk's products done
+    uint64_t *fin = bdone + 2;
     uint64_t *bfull = fin + 1;                                   // [2] B tiles of the stage landed
-    uint32_t *tslot = (uint32_t *)(bfull + 2);
+    uint64_t *afull = bfull + 2;                                 // [2] A tiles of the stage written
+    uint32_t *tslot = (uint32_t *)(afull + 2);
     volatile int *abort_flag = (volatile int *)(tslot + 1);
     float *pf = (float *)(tslot + 2);                            // per pair: ca, cb (wind derivative)
-    int *pio = (int *)(pf + 2 * CMT_P);                          // per pair: outgoing slot, incoming slot, mirror
-    CmPair *pc = (CmPair *)(pio + 3 * CMT_P);                    // per pair: Mueller constants
-    long long *soff = (long long *)(((uintptr_t)(pc + CMT_P) + 7) & ~(uintptr_t)7);        // [M + 1]
+    int *pio = (int *)(pf + 2 * CMT_P * nbk);                    // per pair: outgoing slot, incoming slot, mirror
+    const uint32_t pc_off = (NSTG * A_STAGE + NBST * B_STAGE + 11 * 8 + 8 + 20 * CMT_P * nbk + 15) & ~15u;
+    CmPair *pc = (CmPair *)(base + pc_off);                      // per pair: Mueller constants
+    long long *soff = (long long *)(pc + CMT_P * nbk);           // [M + 1]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
     if (warp == 0) {
@@ -187,15 +203,19 @@ k_coxmunk_tc(const TaskDev *tasks, const PixDev *px, int p0, const int *pix_task
     if (tid == 0) {
         mbar_init(&mma_done[0], 1);
         mbar_init(&mma_done[1], 1);
+        mbar_init(&bdone[0], 1);
+        mbar_init(&bdone[1], 1);
         mbar_init(fin, 1);
         mbar_init(&bfull[0], 1);
         mbar_init(&bfull[1], 1);
+        mbar_init(&afull[0], CMT_P);
+        mbar_init(&afull[1], CMT_P);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // per-pair scalars (FP32, as in the CUDA-core kernel)
-    if (tid < CMT_P) {
-        const int q = pr0 + tid;
+    for (int t = tid; t < CMT_P * nb; t += blockDim.x) {
+        const int q = pr0 + t;
         int o = G.NR, i = 0;
         if (q < npairs) { o = pairs[q].x; i = pairs[q].y; }
         const bool ok = o < d.n_ring;
@@ -213,12 +233,12 @@ k_coxmunk_tc(const TaskDev *tasks, const PixDev *px, int p0, const int *pix_task
             ca = ds2 * (-1.f / fs2 - dlam / (1.f + flam));
             cb = ds2 / (fs2 * fs2);
         }
-        pf[2 * tid] = ca;
-        pf[2 * tid + 1] = cb;
-        pc[tid] = cm_pair(fmo, fmi, fs2, flam, (float)d.n_water);
-        pio[3 * tid] = ok ? o : -1;
-        pio[3 * tid + 1] = i;
-        pio[3 * tid + 2] = ok && o < N && i < N && o < i;
+        pf[2 * t] = ca;
+        pf[2 * t + 1] = cb;
+        pc[t] = cm_pair(fmo, fmi, fs2, flam, (float)d.n_water);
+        pio[3 * t] = ok ? o : -1;
+        pio[3 * t + 1] = i;
+        pio[3 * t + 2] = ok && o < N && i < N && o < i;
     }
     const int task_first = pix_task0[p];
     for (int m = tid; m <= M; m += blockDim.x) soff[m] = tasks[task_first + m].srf_off;
@@ -234,87 +254,130 @@ k_coxmunk_tc(const TaskDev *tasks, const PixDev *px, int p0, const int *pix_task
         *reinterpret_cast<float *>(hi + off) = h;
         *reinterpret_cast<float *>(lo + off) = round_tf32f(v - h);
     };
-    const uint32_t idesc = idesc_tf32(128, NN);
     const int nchunk = half / CMT_KC;
-    for (int c = 0; c < nchunk; ++c) {
-        const int s = dw ? 0 : (c & 1);
-        unsigned char *sp = base + (size_t)s * STAGE;
-        unsigned char *aH = sp, *aL = sp + A_BYTES;
-        unsigned char *tH = sp + 2 * A_BYTES, *tL = sp + 3 * A_BYTES;             // R tan^2(beta) (wind derivative)
-        unsigned char *bH = sp + (dw ? 4 : 2) * A_BYTES, *bL = bH + B_BYTES;
-        if (c >= NSTG) {
-            // every thread waits (bounded) for the MMAs that read this stage
-            // NSTG chunks ago; the barrier makes the abort decision block-uniform
-            if (!mbar_wait(&mma_done[s], ((c / NSTG) - 1) & 1)) *abort_flag = 1;
-            __syncthreads();
-            if (*abort_flag) break;
-        }
-        const int q0 = c * CMT_KC;
-        // B: the chunk's cos/sin tiles by one bulk copy (the stage is free: its
-        // previous MMAs completed before the wait above)
-        if (tid == 0) {
-            mbar_expect_tx(&bfull[s], 2 * B_BYTES);
-            bulk_g2s(bH, cs_tiles + (size_t)c * 2 * NN * CMT_KC, 2 * B_BYTES, &bfull[s]);
-        }
-        // A: Mueller entries of (pair, node); row = 9 pair + entry, K = node in the chunk
-        for (int x = tid; x < CMT_P * CMT_KC; x += blockDim.x) {
-            const int pp = x / CMT_KC, qq = x - pp * CMT_KC, q = q0 + qq;
-            float R[9], tb2 = 0.f;
-            if (pio[3 * pp] >= 0) {
-                cm_mueller(pc[pp], ptab[q], ptab[half + q], ptab[2 * half + q], qc, R, tb2);
-            } else {
-#pragma unroll
-                for (int e = 0; e < 9; ++e) R[e] = 0.f;
+    if (warp < CMT_P) {
+        // ================= evaluation: a warp per pair, lane = azimuth node =================
+        float cn = ptab[lane], sn = ptab[half + lane], hn = ptab[2 * half + lane];
+        for (int t = 0, c = 0; c < nchunk; ++c) {
+            bool stop = false;
+            // the next chunk's azimuths are loaded while this one's are used
+            const float cphi = cn, sphi = sn, shalf2 = hn;
+            if (c + 1 < nchunk) {
+                const int q = (c + 1) * CMT_KC + lane;
+                cn = ptab[q]; sn = ptab[half + q]; hn = ptab[2 * half + q];
             }
+            for (int j = 0; j < nb; ++j, ++t) {
+                const int s = t % NSTG, pp = j * CMT_P + warp;
+                unsigned char *aH = base + (size_t)s * A_STAGE, *aL = aH + A_BYTES;
+                unsigned char *tH = aL + A_BYTES, *tL = tH + A_BYTES;                 // R tan^2(beta) (wind derivative)
+                float R[9], tb2 = 0.f;
+                if (pio[3 * pp] >= 0) {
+                    const CmPair k = pc[pp];
+                    cm_mueller(k, cphi, sphi, shalf2, qc, R, tb2);
+                } else {
 #pragma unroll
-            for (int e = 0; e < 9; ++e) {
-                const int row = 9 * pp + e;
-                const uint32_t off = (uint32_t)row * 128u + ((uint32_t)((qq >> 2) ^ (row & 7)) << 4) + (uint32_t)(qq & 3) * 4u;
-                split_st(aH, aL, off, R[e]);
-                if (dw) split_st(tH, tL, off, R[e] * tb2);
-            }
-        }
-        // rows 126 and 127 are zero
-        for (int x = tid; x < 2 * CMT_KC; x += blockDim.x) {
-            const int row = 126 + x / CMT_KC, qq = x % CMT_KC;
-            const uint32_t off = (uint32_t)row * 128u + ((uint32_t)((qq >> 2) ^ (row & 7)) << 4) + (uint32_t)(qq & 3) * 4u;
-            split_st(aH, aL, off, 0.f);
-            if (dw) split_st(tH, tL, off, 0.f);
-        }
-        // generic-proxy stores made visible to the tensor cores
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
-            const bool bok = mbar_wait(&bfull[s], (c / NSTG) & 1);
-            if (!bok) *abort_flag = 1;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t sa_h = smem_u32(aH), sa_l = smem_u32(aL), st_h = smem_u32(tH), st_l = smem_u32(tL);
-            const uint32_t sb_h = smem_u32(bH), sb_l = smem_u32(bL);
-            for (int kk = 0; bok && kk < CMT_KC / 8; ++kk) {
-                const uint32_t off = kk * 32;
-                const uint64_t bh = sdesc_sw128(sb_h + off), bl = sdesc_sw128(sb_l + off);
-                const uint32_t acc0 = (c > 0 || kk > 0) ? 1u : 0u;
-                umma_tf32(tmem, sdesc_sw128(sa_h + off), bh, idesc, acc0);
-                umma_tf32(tmem, sdesc_sw128(sa_h + off), bl, idesc, 1u);
-                umma_tf32(tmem, sdesc_sw128(sa_l + off), bh, idesc, 1u);
-                if (dw) {
-                    umma_tf32(tmem + (uint32_t)NN, sdesc_sw128(st_h + off), bh, idesc, acc0);
-                    umma_tf32(tmem + (uint32_t)NN, sdesc_sw128(st_h + off), bl, idesc, 1u);
-                    umma_tf32(tmem + (uint32_t)NN, sdesc_sw128(st_l + off), bh, idesc, 1u);
+                    for (int e = 0; e < 9; ++e) R[e] = 0.f;
                 }
+                // the MMAs that read this stage before are done (bounded)
+                if (t >= NSTG) {
+                    stop = __any_sync(0xffffffffu, !mbar_wait(&mma_done[s], (t / NSTG - 1) & 1));
+                    if (stop) { *abort_flag = 1; break; }
+                }
+#pragma unroll
+                for (int e = 0; e < 9; ++e) {
+                    const int row = 9 * warp + e;
+                    const uint32_t off = (uint32_t)row * 128u + ((uint32_t)((lane >> 2) ^ (row & 7)) << 4) + (uint32_t)(lane & 3) * 4u;
+                    split_st(aH, aL, off, R[e]);
+                    if (dw) split_st(tH, tL, off, R[e] * tb2);
+                }
+                if (t < NSTG && warp < 2) {
+                    // rows 126 and 127 are zero
+                    const int row = 126 + warp;
+                    const uint32_t off = (uint32_t)row * 128u + ((uint32_t)((lane >> 2) ^ (row & 7)) << 4) + (uint32_t)(lane & 3) * 4u;
+                    split_st(aH, aL, off, 0.f);
+                    if (dw) split_st(tH, tL, off, 0.f);
+                }
+                // generic-proxy stores made visible to the tensor cores
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&afull[s]);
             }
-            umma_commit(&mma_done[s]);
+            if (stop) break;
         }
+    } else {
+        // ================= table copies and MMA issue =================
+        // converged, one elected lane issuing: from a divergent lane an MMA takes
+        // twice its run time to issue
+        const uint32_t idesc = idesc_tf32(128, NN);
+        const uint64_t dbase = sdesc_sw128(0);
+        // B: a chunk's cos/sin tiles by one bulk copy
+        auto copy_b = [&](int c) {
+            if (lane == 0) {
+                mbar_expect_tx(&bfull[c % NBST], 2 * B_BYTES);
+                bulk_g2s(bbase + (size_t)(c % NBST) * B_STAGE, cs_tiles + (size_t)c * 2 * NN * CMT_KC, 2 * B_BYTES,
+                         &bfull[c % NBST]);
+            }
+            __syncwarp();
+        };
+        int copied = 0;                                              // chunks whose copy has been issued
+        for (int t = 0, c = 0; c < nchunk; ++c) {
+            bool stop = false;
+            const int sb = c % NBST;
+            // copies up to NBST - 1 chunks ahead, into stages whose products are done
+            for (; copied < nchunk && copied < c + NBST && !stop; ++copied) {
+                if (copied >= NBST && !mbar_wait(&bdone[copied % NBST], (copied / NBST - 1) & 1)) *abort_flag = 1;
+                stop = __any_sync(0xffffffffu, *abort_flag != 0);
+                if (stop) break;
+                copy_b(copied);
+            }
+            if (stop) break;
+            if (!mbar_wait(&bfull[sb], (c / NBST) & 1)) *abort_flag = 1;
+            const uint32_t bH = smem_u32(bbase + (size_t)sb * B_STAGE) >> 4, bL = bH + (B_BYTES >> 4);
+            for (int j = 0; j < nb; ++j, ++t) {
+                const int s = t % NSTG;
+                const uint32_t aH = smem_u32(base + (size_t)s * A_STAGE) >> 4, aL = aH + (A_BYTES >> 4);
+                const uint32_t tH = aL + (A_BYTES >> 4), tL = tH + (A_BYTES >> 4);
+                const uint32_t D = tmem + (uint32_t)(j * NN) * (dw ? 2u : 1u);
+                if (!mbar_wait(&afull[s], (t / NSTG) & 1)) *abort_flag = 1;
+                stop = __any_sync(0xffffffffu, *abort_flag != 0);
+                if (stop) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (elect_one()) {
+#pragma unroll
+                    for (int kk = 0; kk < CMT_KC / 8; ++kk) {
+                        const uint32_t off = kk * 2;
+                        const uint64_t bh = dbase | (bH + off), bl = dbase | (bL + off);
+                        const uint32_t acc0 = (c > 0 || kk > 0) ? 1u : 0u;
+                        umma_tf32(D, dbase | (aH + off), bh, idesc, acc0);
+                        umma_tf32(D, dbase | (aH + off), bl, idesc, 1u);
+                        umma_tf32(D, dbase | (aL + off), bh, idesc, 1u);
+                        if (dw) {
+                            umma_tf32(D + (uint32_t)NN, dbase | (tH + off), bh, idesc, acc0);
+                            umma_tf32(D + (uint32_t)NN, dbase | (tH + off), bl, idesc, 1u);
+                            umma_tf32(D + (uint32_t)NN, dbase | (tL + off), bh, idesc, 1u);
+                        }
+                    }
+                    umma_commit(&mma_done[s]);
+                    if (j == nb - 1) umma_commit(&bdone[sb]);
+                }
+                __syncwarp();
+            }
+            if (stop) break;
+        }
+        // a copy still in flight lands before the CTA leaves
+        if (*abort_flag && copied > 0) (void)mbar_wait(&bfull[(copied - 1) % NBST], ((copied - 1) / NBST) & 1);
+        if (elect_one()) umma_commit(fin);
+        __syncwarp();
     }
-    if (tid == 0) umma_commit(fin);
     if (!mbar_wait(fin, 0)) *abort_flag = 1;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     __syncthreads();
     const bool done = !*abort_flag;                                  // block-uniform
-    if (warp < 4 && done) {
-        // epilogue: lane = row (pair, entry) of the warp's TMEM lane quadrant
-        const int row = warp * 32 + lane;
-        const int pp = row / 9, e = row - pp * 9;
+    // epilogue: lane = row (pair, entry) of the warp's TMEM lane quadrant; three
+    // warps a quadrant share the columns
+    for (int j = 0; warp < 12 && done && j < nb; ++j) {
+        const int quad = warp & 3, row = quad * 32 + lane;
+        const int pr = row / 9, e = row - pr * 9, pp = j * CMT_P + pr;
         const bool live = row < 9 * CMT_P && pio[3 * pp] >= 0;
         const int o = live ? pio[3 * pp] : 0, i = live ? pio[3 * pp + 1] : 0;
         const bool mirror = live && pio[3 * pp + 2];
@@ -325,8 +388,8 @@ k_coxmunk_tc(const TaskDev *tasks, const PixDev *px, int p0, const int *pix_task
         const float scale0 = 2.f / (float)nphi, scale1 = 4.f / (float)nphi;
         const size_t offp = i < N ? srf_entry(G, o, i, e) : (size_t)G.srf_sun + (size_t)o * 9 + e;
         const size_t offt = i < N && o < N ? srf_entry(G, i, o, et) : 0;
-        const uint32_t tb = tmem + ((uint32_t)(warp * 32) << 16);
-        for (int cb16 = 0; cb16 < NN / 16; ++cb16) {
+        const uint32_t tb = tmem + (uint32_t)(j * NN) * (dw ? 2u : 1u) + ((uint32_t)(quad * 32) << 16);
+        for (int cb16 = warp >> 2; cb16 < NN / 16; cb16 += 3) {
             float v[16], vt[16];
             tmem_ld16(tb + (uint32_t)(cb16 * 16), v);
             if (dw) tmem_ld16(tb + (uint32_t)(NN + cb16 * 16), vt);
@@ -357,12 +420,24 @@ k_coxmunk_tc(const TaskDev *tasks, const PixDev *px, int p0, const int *pix_task
     }
 }
 
-size_t coxmunk_tc_smem_bytes(int Mtab, bool dw)
+// Blocks of CMT_P pairs a CTA takes, with one copy of the azimuth tables for all:
+// what fits in 256 TMEM columns, while that leaves two CTAs for each of the two an
+// SM holds (384 pixels: three blocks 1.60 ms, one 1.80; one pixel at 24 streams: one
+// block 24 us, three 51).
+static int cm_blocks(int Mtab, bool dw, int npairs, int npix, int nsm)
+{
+    const int NN = 2 * ((Mtab + 1 + 7) & ~7), fit = 256 / (dw ? 2 * NN : NN), nblk = (npairs + CMT_P - 1) / CMT_P;
+    return std::max(1, std::min(fit, (int)((long long)nblk * npix / (4 * nsm))));
+}
+
+static size_t cm_smem_bytes(int Mtab, bool dw, int nbk)
 {
     const size_t NN = 2 * (size_t)((Mtab + 1 + 7) & ~7);
     const size_t stage = (dw ? 4 : 2) * (size_t)128 * CMT_KC * 4 + 2 * NN * CMT_KC * 4;
-    return 1024 + (dw ? 1 : 2) * stage + 64 + 2 * 4 * CMT_P + 3 * 4 * CMT_P + sizeof(CmPair) * CMT_P + 16 + 8 * ((size_t)Mtab + 1);
+    return 1024 + (dw ? 1 : 2) * stage + 128 + (2 * 4 + 3 * 4 + sizeof(CmPair)) * CMT_P * nbk + 16 + 8 * ((size_t)Mtab + 1);
 }
+
+size_t coxmunk_tc_smem_bytes(int Mtab, bool dw) { return cm_smem_bytes(Mtab, dw, 256 / (2 * 8)); }
 
 size_t coxmunk_tc_tiles_floats(int Mtab, int nphi)
 {
@@ -375,6 +450,20 @@ bool coxmunk_tc_supported(int Mtab, int nphi, bool dw)
     return Mtab <= 63 && nphi % (2 * CMT_KC) == 0 && coxmunk_tc_smem_bytes(Mtab, dw) <= 227 * 1024;
 }
 
-int coxmunk_tc_pairs_per_cta() { return CMT_P; }
+void coxmunk_tc_launch(bool dw, int npix, int nsm, cudaStream_t st, const TaskDev *tasks, const PixDev *px, int p0, const int *pix_task0,
+                       const Geom &G, const double *gmu, const float *cs_tab, const float *cs_tiles, int Mtab,
+                       const double *lamv, const double *lamd, float *srf, float *srfW, const short2 *pairs, int npairs,
+                       int *err)
+{
+    const int nbk = cm_blocks(Mtab, dw, npairs, npix, nsm);
+    const dim3 grid((npairs + CMT_P * nbk - 1) / (CMT_P * nbk), npix);
+    (dw ? k_coxmunk_tc<true> : k_coxmunk_tc<false>)<<<grid, CMT_THREADS, cm_smem_bytes(Mtab, dw, nbk), st>>>(
+        tasks, px, p0, pix_task0, G, gmu, cs_tab, cs_tiles, Mtab, lamv, lamd, srf, srfW, pairs, npairs, nbk, err);
+}
 
-int coxmunk_tc_threads(bool dw) { (void)dw; return CMT_THREADS_DW; }
+cudaError_t coxmunk_tc_init()
+{
+    const cudaError_t e = cudaFuncSetAttribute(k_coxmunk_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    return e != cudaSuccess ? e
+                            : cudaFuncSetAttribute(k_coxmunk_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+}
