@@ -155,14 +155,16 @@ k_tables_tc(const TaskDev *tasks, int t0, int nt_tasks, const PixDev *px, Geom G
             const double *mz, float *ops, float *opt, int plain, const float *V, int vp0, long long vstride,
             float *sprod, int *err, unsigned char *popt, const float *Bp, const float *Br, const float *Bt)
 {
-    extern __shared__ unsigned char smem_raw[];
-    unsigned char *base = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    // the declared alignment (not one made from the address) keeps the pointers
+    // below known as shared memory (scene of 384 pixels: 1.32 ms, 1.37 before)
+    extern __shared__ __align__(1024) unsigned char tt_smem[];
+    unsigned char *base = tt_smem;
     const int Kp = tt_kpad(L), nchx = Kp / TT_KC;
     const int N = G.N, E = G.E, nxr = 3 * (E + 1);
     unsigned char *aH = base, *aL = base + TT_A_BYTES, *bH = base + 2 * TT_A_BYTES, *bL = bH + TT_B_BYTES;
     float *ptab = (float *)(base + TT_STAGE);                             // [N + E][26][TT_PS]
     float *smp = ptab + (size_t)(N + E) * 26 * TT_PS;                     // [4][Kp] moments in the chunk order
-    uint64_t *bars = (uint64_t *)(((uintptr_t)(smp + 4 * Kp) + 7) & ~(uintptr_t)7);
+    uint64_t *bars = (uint64_t *)(smp + 4 * Kp);                          // an even number of floats behind ptab
     uint64_t *afull = bars, *empty = bars + 1, *acc_full = bars + 2, *acc_empty = bars + 3, *fin = bars + 4;
     uint32_t *tslot = (uint32_t *)(bars + 5);
     // abort flags, one per warp group: each is written only by its own group
