@@ -936,7 +936,7 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
     if (g.Cq)
         LAUNCH(plan, KC_SETUP, k_coef_quads<<<dim3(16, P), 256, 0, st>>>(g.px, P, g.N, G.NR, g.Tc, g.Ca, g.Cb, g.Cq));
     LAUNCH(plan, KC_SETUP, k_gsf_coefs<<<g.Mmax + 1, 128, 0, st>>>(g.Mmax, g.Lmax, g.gcoef));
-    LAUNCH(plan, KC_SETUP, k_basis_gauss<<<g.Mmax + 1, 64, 0, st>>>(g.N, g.Mmax, g.Lmax, g.gmu, g.Bp, g.Br, g.Bt,
+    LAUNCH(plan, KC_SETUP, k_basis_gauss<<<dim3(g.Mmax + 1, 2), 64, 0, st>>>(g.N, g.Mmax, g.Lmax, g.gmu, g.Bp, g.Br, g.Bt,
                                                                    g.gcoef));
     if (g.tabs_tc)
         LAUNCH(plan, KC_SETUP, k_basis_perm<<<dim3(8, g.Mmax + 1), 256, 0, st>>>(g.N, g.Mmax, g.Lmax, g.Bp, g.Br, g.Bt,
@@ -1017,7 +1017,7 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
         CK(cudaMemsetAsync(g.mol_cnt, 0, sizeof(int) * ((size_t)g.max_orders + 2), st));
         CK(cudaMemsetAsync(g.work, 0, sizeof(int) * 4 * ((size_t)g.max_orders + 2), st));
         CK(cudaMemsetAsync(g.aflag, 0, (size_t)nw, st));
-        LAUNCH(plan, KC_TABLES, k_basis_pix<<<(nw + 32 / (1 + G.E) - 1) / (32 / (1 + G.E)), 32, 0, st>>>(
+        LAUNCH(plan, KC_TABLES, k_basis_pix<<<dim3((nw + 32 / (1 + G.E) - 1) / (32 / (1 + G.E)), 2), 32, 0, st>>>(
                    g.tasks, w.t0, nw, g.px, g.Lmax, G.E, g.Bx, g.gcoef));
         if (g.any_vk)
             LAUNCH(plan, KC_TABLES, k_value_pfm<<<dim3(((G.N + 1) * 2 * G.NR + 127) / 128, w.p1 - w.p0), 128,
@@ -1238,7 +1238,7 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
     if (g.any_lut)
         LAUNCH(plan, KC_FINAL, k_lut_final<<<dim3((g.lut_ptmax + 127) / 128, P), 128, 0, st>>>(g.px, P, make_lut(g),
                                                                                               g.pix_task0));
-    LAUNCH(plan, KC_FINAL, k_finalize<<<(P + 3) / 4, 128, 0, st>>>(g.px, P, g.state, g.tout, g.gmu, g.gw, g.h,
+    LAUNCH(plan, KC_FINAL, k_finalize<<<P, 96, 0, st>>>(g.px, P, g.state, g.tout, g.gmu, g.gw, g.h,
                                                               g.kappa, g.taudir, g.res));
     return OCRT_OK;
 }

@@ -228,7 +228,7 @@ extern "C" int ocrt_gb_solve_case_noalloc(const ocrt_case *cs, const ocrt_opts *
     NA_LAUNCH(k_levels<<<dim3(lev_blocks(d.nt), 1), LEV_B, 0, st>>>(px, 1, h, ch, xd, yd, z));
     if (opts->gas) NA_LAUNCH(k_gas_apply<<<1, 256, 0, st>>>(px, 1, h, ch, xd, yd, z, tabs));
     NA_LAUNCH(k_coef<<<dim3(16, 1), 256, 0, st>>>(px, 1, N, NR, gmu, h, Tc, Ca, Cb));
-    NA_LAUNCH(k_basis_gauss<<<T, 64, 0, st>>>(N, M, L, gmu, Bp, Br, Bt, nullptr));
+    NA_LAUNCH(k_basis_gauss<<<dim3(T, 2), 64, 0, st>>>(N, M, L, gmu, Bp, Br, Bt, nullptr));
     if (rough) {
         NA_LAUNCH(k_cs_table<<<T + 1, 256, 0, st>>>(M, d.nphi, cst));
         NA_LAUNCH(k_seed_att<<<dim3(8, 1), 256, 0, st>>>(px, 1, N, gmu, h, Eatt));
@@ -256,7 +256,7 @@ extern "C" int ocrt_gb_solve_case_noalloc(const ocrt_case *cs, const ocrt_opts *
         NA_CK(cudaMemsetAsync(active, 0, sizeof(int) * ((size_t)opts->max_orders + 2), st));
         NA_CK(cudaMemsetAsync(molcnt, 0, sizeof(int) * ((size_t)opts->max_orders + 2), st));
         NA_CK(cudaMemsetAsync(work, 0, sizeof(int) * 4 * ((size_t)opts->max_orders + 2), st));
-        NA_LAUNCH(k_basis_pix<<<(nw + 15) / 16, 32, 0, st>>>(tasks, t0, nw, px, L, 1, Bx, nullptr));
+        NA_LAUNCH(k_basis_pix<<<dim3((nw + 15) / 16, 2), 32, 0, st>>>(tasks, t0, nw, px, L, 1, Bx, nullptr));
         NA_LAUNCH(k_tables<<<dim3(nw, tables_yblocks(256, G.NR, G.N)), 256, tables_smem_bytes(256, G.N, L), st>>>(
             tasks, t0, nw, px, G, L, Bp, Br, Bt, Bx, gw, mb, mg, ma, mz, ops, pvec, W.fvec, nullptr, 1, nullptr, 0, 0,
             nullptr));
@@ -281,7 +281,7 @@ extern "C" int ocrt_gb_solve_case_noalloc(const ocrt_case *cs, const ocrt_opts *
         NA_LAUNCH(k_ipss<<<dim3(IPSS_SPLIT, 1), IPSS_THREADS, ipss_smem_bytes(nt), st>>>(px, 1, h, z, xd, yd, opts->gas ? tabs : nullptr, mb, nullptr, nullptr,
                                                kappa, taudir));
     }
-    NA_LAUNCH(k_finalize<<<1, 32, 0, st>>>(px, 1, state, tout, gmu, gw, h, kappa, taudir, res));
+    NA_LAUNCH(k_finalize<<<1, 96, 0, st>>>(px, 1, state, tout, gmu, gw, h, kappa, taudir, res));
     int dev_err = 0;
     NA_CK(cudaMemcpyAsync(out, res, sizeof(ocrt_result), cudaMemcpyDeviceToHost, st));
     NA_CK(cudaMemcpyAsync(&dev_err, err, sizeof(int), cudaMemcpyDeviceToHost, st));

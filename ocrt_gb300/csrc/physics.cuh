@@ -157,12 +157,13 @@ __host__ __device__ inline void gsf_step_coefs(int l, int m, double *c)
 }
 
 // Runs the scalar and spin-2 recurrences for one direction cosine x and
-// hands every degree l = 0..L to sink(l, P, R, T).  ctab, when given, holds
+// hands every degree l = 0..L to sink(l, P, R, T): P where part is 0, R and T
+// where it is 1.  ctab, when given, holds
 // gsf_step_coefs(l, m) at ctab[5 l] and gsf_start_norms(m) at ctab[0]
 // (k_gsf_coefs), so the steps need no square root or division; the
 // coefficients of four steps are loaded ahead.
 template <class Sink>
-__device__ inline void gsf_recur(int L, int m, double x, Sink sink, const double *ctab = nullptr)
+__device__ inline void gsf_recur(int L, int m, double x, Sink sink, int part, const double *ctab = nullptr)
 {
     double p0 = 0, p1 = 0, r0 = 0, r1 = 0, t0 = 0, t1 = 0;   // degree l-1 and l
     // degrees below the start are zero
@@ -197,12 +198,17 @@ __device__ inline void gsf_recur(int L, int m, double x, Sink sink, const double
     // the terms in degree l - 1 first: a dependent FP64 operation takes ~100
     // cycles, and two of them are a step's chain
     auto step = [&](int l, const double *k) {
-        const double fx = k[0] * x, sx = k[2] * x;
-        const double p2 = fma(fx, p1, -(k[1] * p0));
+        if (part == 0) {
+            const double p2 = fma(k[0] * x, p1, -(k[1] * p0));
+            p0 = p1; p1 = p2;
+            sink(l + 1, p2, 0.0, 0.0);
+            return;
+        }
+        const double sx = k[2] * x;
         const double r2 = fma(sx, r1, fma(-k[4], t1, -(k[3] * r0)));
         const double t2 = fma(sx, t1, fma(-k[4], r1, -(k[3] * t0)));
-        p0 = p1; p1 = p2; r0 = r1; r1 = r2; t0 = t1; t1 = t2;
-        sink(l + 1, p2, r2, t2);
+        r0 = r1; r1 = r2; t0 = t1; t1 = t2;
+        sink(l + 1, 0.0, r2, t2);
     };
     if (!ctab) {
         for (int l = l0; l < L; ++l) {

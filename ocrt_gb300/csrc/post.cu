@@ -350,48 +350,68 @@ __global__ void k_ipss_lut(const PixDev *px, int P, const double *h, const doubl
     }
 }
 
-// One warp per pixel: lane l takes the modes l, l + 32, ...; the IPSS parts
-// (kpart, nullptr without IPSS) are added in order.
-__global__ void k_finalize(const PixDev *px, int P, const TaskState *state, const TaskOut *tout,
+// A block of three warps per pixel, whose FP64 chains run side by side: the Fourier
+// sums (lane l takes the modes l, l + 32, ...; the IPSS parts, kpart, nullptr
+// without IPSS, are added in order), the direct sunglint, the transmittances.  One
+// pixel: 32 us, 40 with one warp.
+__global__ void __launch_bounds__(96) k_finalize(const PixDev *px, int P, const TaskState *state, const TaskOut *tout,
                            const double *gmu, const double *gw, const double *h,
                            const double *kpart, const double *tau_dir, ocrt_result *res)
 {
-    const int p = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    __shared__ double sg[3], sT[2];
+    const int p = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (p >= P) return;
     const PixDev &d = px[p];
     const int M = d.M;
-    const double phi = d.raa_deg * OCRT_PI / 180.0 + OCRT_PI;
+    const double mu0 = d.mu0, tau = d.tau_total;
+    const double td = d.pssa ? tau_dir[p] : -1.0;
     double I = 0, Q = 0, U = 0, Dn = 0;
     int max_orders = 0, conv = 1, om = 0;
-    for (int m = lane; m <= M; m += 32) {
-        const TaskOut &o = tout[d.task0 + m];
-        const TaskState &st = state[d.task0 + m];
-        const double cm = m == 0 ? 1.0 : 2.0 * cos((double)m * phi);
-        const double sm = m == 0 ? 0.0 : 2.0 * sin((double)m * phi);
-        I += cm * o.vI; Q += cm * o.vQ; U += sm * o.vU;
-        Dn += cm * o.dn_view;
-        if (st.orders > max_orders) max_orders = st.orders;
-        if (!st.converged) conv = 0;
-        om += st.orders;
+    if (warp == 1) {
+        if (lane == 0 && d.surface == 2) {
+            const double phi_v = (d.raa_deg - 180.0) * OCRT_PI / 180.0;
+            const double mv = d.vza_deg > 0.0 ? d.mu_view : 1.0;
+            double g[3];
+            sunglint(d, mv, phi_v, tau, g);
+            const double cg = td >= 0.0 ? exp(-(td - tau / mu0)) : 1.0;
+            for (int i = 0; i < 3; ++i) sg[i] = g[i] * cg;
+        }
+    } else if (warp == 2) {
+        if (lane < 2) sT[lane] = lane == 0 ? (td >= 0.0 ? exp(-td) : exp(-tau / mu0))
+                                           : exp(-tau / (d.mu_view > 0.0 ? d.mu_view : 1.0));
+    } else {
+        const double phi = d.raa_deg * OCRT_PI / 180.0 + OCRT_PI;
+        for (int m = lane; m <= M; m += 32) {
+            const TaskOut &o = tout[d.task0 + m];
+            const TaskState &st = state[d.task0 + m];
+            double cm, sm;
+            sincos((double)m * phi, &sm, &cm);
+            cm = m == 0 ? 1.0 : 2.0 * cm;
+            sm = m == 0 ? 0.0 : 2.0 * sm;
+            I += cm * o.vI; Q += cm * o.vQ; U += sm * o.vU;
+            Dn += cm * o.dn_view;
+            if (st.orders > max_orders) max_orders = st.orders;
+            if (!st.converged) conv = 0;
+            om += st.orders;
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            I += __shfl_xor_sync(0xffffffffu, I, o);
+            Q += __shfl_xor_sync(0xffffffffu, Q, o);
+            U += __shfl_xor_sync(0xffffffffu, U, o);
+            Dn += __shfl_xor_sync(0xffffffffu, Dn, o);
+        }
+        max_orders = __reduce_max_sync(0xffffffffu, max_orders);
+        conv = __reduce_min_sync(0xffffffffu, conv);
+        om = __reduce_add_sync(0xffffffffu, om);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        I += __shfl_xor_sync(0xffffffffu, I, o);
-        Q += __shfl_xor_sync(0xffffffffu, Q, o);
-        U += __shfl_xor_sync(0xffffffffu, U, o);
-        Dn += __shfl_xor_sync(0xffffffffu, Dn, o);
-    }
-    max_orders = __reduce_max_sync(0xffffffffu, max_orders);
-    conv = __reduce_min_sync(0xffffffffu, conv);
-    om = __reduce_add_sync(0xffffffffu, om);
-    if (lane) return;
+    __syncthreads();
+    if (threadIdx.x) return;
     ocrt_result r;
     memset(&r, 0, sizeof(r));
-    const double mu0 = d.mu0, tau = d.tau_total;
     r.I_TOA = I; r.Q_TOA = Q; r.U_TOA = U;
     r.rho_I = I / mu0; r.rho_Q = Q / mu0; r.rho_U = U / mu0;
     r.tau_R_total = d.tau_r;
     r.kappa_ipss = 1.0;
-    const double td = d.pssa ? tau_dir[p] : -1.0;
     if (d.pssa) {
         const double *kp = kpart + (size_t)p * (IPSS_SPLIT + 1);
         double Iss = 0.0;
@@ -402,14 +422,7 @@ __global__ void k_finalize(const PixDev *px, int P, const TaskState *state, cons
         r.I_TOA *= k; r.Q_TOA *= k; r.U_TOA *= k;
     }
     if (d.surface == 2) {
-        const double phi_v = (d.raa_deg - 180.0) * OCRT_PI / 180.0;
-        const double mv = d.vza_deg > 0.0 ? d.mu_view : 1.0;
-        double g[3];
-        sunglint(d, mv, phi_v, tau, g);
-        if (td >= 0.0) {
-            const double cg = exp(-(td - tau / mu0));
-            g[0] *= cg; g[1] *= cg; g[2] *= cg;
-        }
+        const double g[3] = {sg[0], sg[1], sg[2]};
         if (!d.decouple) { r.rho_I += g[0]; r.rho_Q += g[1]; r.rho_U += -g[2]; }
         if (d.wind > 0.0) {
             r.T_sg_up_dir = g[0] * mu0;
@@ -419,11 +432,11 @@ __global__ void k_finalize(const PixDev *px, int P, const TaskState *state, cons
     r.n_orders_used = max_orders;
     r.converged = conv;
     r.order_modes = om;
-    r.T_dir_dn = td >= 0.0 ? exp(-td) : exp(-tau / mu0);
+    r.T_dir_dn = sT[0];
     r.T_diff_dn_hemi = 2.0 * OCRT_PI * tout[d.task0].fdn / (OCRT_PI * mu0);
     r.T_total_dn_hemi = r.T_dir_dn + r.T_diff_dn_hemi;
     r.T_diff_dn_dir = 2.0 * OCRT_PI * d.mu_view * Dn / (OCRT_PI * mu0);
     r.T_total_up_dir = r.rho_I * mu0;
-    r.T_dir_up_view = exp(-tau / (d.mu_view > 0.0 ? d.mu_view : 1.0));
+    r.T_dir_up_view = sT[1];
     res[p] = r;
 }

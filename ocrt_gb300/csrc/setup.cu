@@ -17,9 +17,10 @@
 // One thread per node; one block.  A chain of dependent FP64 operations: with
 // the step P_{q+1} = t P_q + q/(q+1) (t P_q - P_{q-1}) and its ratios tabulated
 // first it is two operations long instead of a division's dozens, and from the
-// second-order start below Newton ends after two or three passes.  The error of
-// the nodes (1.5e-16) and weights is that of the three-term form with divisions.
-// 32 streams: 33 us, 155 us before.
+// fourth-order start below (Tricomi) Newton ends after two or three passes, the last of
+// which also gives the weight: the derivative at the final node is that of the last pass
+// plus its second-order term.  The error of the nodes (1.5e-16) and weights is that of
+// the three-term form with divisions.  32 streams: 28 us, 155 us before.
 __global__ void k_gauss(int N, double *mu, double *w, float *pw)
 {
     __shared__ double ratio[2 * 64];
@@ -29,8 +30,11 @@ __global__ void k_gauss(int N, double *mu, double *w, float *pw)
     const int k = threadIdx.x + 1;               // 1..N (largest root first)
     if (k > N) return;
     const double no = (double)order;
-    double t = cos(OCRT_PI * ((double)k - 0.25) / (no + 0.5)) * (1.0 - (1.0 - 1.0 / no) / (8.0 * no * no));
-    double a, b;
+    double sth, cth;
+    sincos(OCRT_PI * ((double)k - 0.25) / (no + 0.5), &sth, &cth);
+    double t = cth * (1.0 - (no - 1.0) / (8.0 * no * no * no) -
+                      (39.0 - 28.0 / (sth * sth)) / (384.0 * no * no * no * no));
+    double a, b, dp = 1.0;
     auto legendre = [&]() {
         a = 1.0; b = t;
         for (int q = 1; q < order; ++q) {
@@ -40,13 +44,13 @@ __global__ void k_gauss(int N, double *mu, double *w, float *pw)
     };
     for (int it = 0; it < 100; ++it) {
         legendre();
-        const double step = -b * (t * t - 1.0) / (no * (t * b - a));
+        const double om = 1.0 - t * t, dpt = no * (a - t * b) / om, step = -b / dpt;
+        // P'' = (2 t P' - n (n + 1) P) / (1 - t^2); what is left of the node after the
+        // step is about step^2 t / (1 - t^2)
+        dp = dpt + step * (2.0 * t * dpt - no * (no + 1.0) * b) / om;
         t += step;
-        // what is left is about step^2 t / (1 - t^2), below 1e-17 from here
-        if (fabs(step) < 1.0e-10) break;
+        if (step * step * fabs(t) < 1.0e-17 * om) break;
     }
-    legendre();
-    const double dp = no * (t * b - a) / (t * t - 1.0);
     mu[N - k] = t;
     w[N - k] = 2.0 / ((1.0 - t * t) * dp * dp);
     // surface-operator weights (2 pi or pi) mu w, rounded once (rt_surface_boundary.c:137-208)
@@ -325,14 +329,15 @@ __global__ void k_coef_deriv(const PixDev *px, int P, int N, const double *gmu, 
 __global__ void k_basis_gauss(int N, int M, int L, const double *gmu, float *Bp, float *Br, float *Bt,
                               const double *gcoef)
 {
-    const int m = blockIdx.x, g = threadIdx.x;
+    // grid y: the scalar function by one block, the two coupled ones by another
+    const int m = blockIdx.x, g = threadIdx.x, part = blockIdx.y;
     if (m > M || g >= N) return;
     const size_t base = (size_t)m * (L + 1) * N;
     gsf_recur(L, m, gmu[g], [&](int l, double P, double R, double T) {
-        Bp[base + (size_t)l * N + g] = (float)P;
+        if (part == 0) { Bp[base + (size_t)l * N + g] = (float)P; return; }
         Br[base + (size_t)l * N + g] = (float)R;
         Bt[base + (size_t)l * N + g] = (float)T;
-    }, gcoef ? gcoef + (size_t)m * (L + 1) * 5 : nullptr);
+    }, part, gcoef ? gcoef + (size_t)m * (L + 1) * 5 : nullptr);
 }
 
 // Step coefficients of the GSF recurrences for every (m, l) of a group:
@@ -360,13 +365,15 @@ __global__ void __launch_bounds__(128) k_gsf_coefs(int M, int L, double *gcoef)
 
 // GSF basis at the solar direction (-mu0) and at the E zero-weight slots for
 // every task of a wave: Bx[((t*(1+E) + which)*3 + comp)*(L+1) + l], which 0 =
-// sun, 1 + e = slot N + e.  A serial FP64 recurrence per thread, bound by the
-// FP64 issue rate of an SM: blocks of one warp spread a few tasks over many SMs.
-// One pixel, 17 modes, L = 120: 67 us, 155 us before; 3264 tasks 101 us, 252 before.
+// sun, 1 + e = slot N + e.  A serial FP64 recurrence per thread, bound by the FP64
+// operations of an SM: blocks of one warp spread a few tasks over many SMs, grid y the
+// scalar and the spin-2 functions.  One pixel, 33 modes, L = 120: 57 us, 155 us before;
+// 384 pixels 102 us, 252 before.  (Three warps of a block, one per function of the
+// decoupled R + T and R - T recurrences: 60 and 202 us.)
 __global__ void k_basis_pix(const TaskDev *tasks, int t0, int nt_tasks, const PixDev *px, int L, int E, float *Bx,
                             const double *gcoef)
 {
-    const int W = 1 + E, per = blockDim.x / W;
+    const int W = 1 + E, per = blockDim.x / W, part = blockIdx.y;      // as in k_basis_gauss
     if ((int)threadIdx.x >= per * W) return;
     const int tl = blockIdx.x * per + threadIdx.x / W;
     const int which = threadIdx.x % W;
@@ -375,10 +382,15 @@ __global__ void k_basis_pix(const TaskDev *tasks, int t0, int nt_tasks, const Pi
     const PixDev &d = px[tk.pix];
     const double x = which == 0 ? -d.mu0 : d.xmu[which - 1];
     float *dst = Bx + ((size_t)tl * W + which) * 3 * (L + 1);
-    for (int l = d.L + 1; l <= L; ++l) { dst[l] = 0.f; dst[L + 1 + l] = 0.f; dst[2 * (L + 1) + l] = 0.f; }
+    for (int l = d.L + 1; l <= L; ++l) {
+        if (part == 0) { dst[l] = 0.f; continue; }
+        dst[L + 1 + l] = 0.f;
+        dst[2 * (L + 1) + l] = 0.f;
+    }
     gsf_recur(d.L, tk.m, x, [&](int l, double P, double R, double T) {
-        dst[l] = (float)P; dst[L + 1 + l] = (float)R; dst[2 * (L + 1) + l] = (float)T;
-    }, gcoef ? gcoef + (size_t)tk.m * (L + 1) * 5 : nullptr);
+        if (part == 0) { dst[l] = (float)P; return; }
+        dst[L + 1 + l] = (float)R; dst[2 * (L + 1) + l] = (float)T;
+    }, part, gcoef ? gcoef + (size_t)tk.m * (L + 1) * 5 : nullptr);
 }
 
 // One block per task.  Phase tables by contraction over l in FP32 with the
