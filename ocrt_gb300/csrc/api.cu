@@ -418,6 +418,34 @@ template <class T> int up(T *&dst, const std::vector<T> &src)
     return OCRT_OK;
 }
 
+// The small arrays of a group in one allocation and one copy (a pageable copy takes
+// ~4 us of the host's time whatever its size; one pixel has nine of them).  Large ones
+// keep a copy of their own, straight from the caller's vector.  Freeing the first
+// array frees the block: the others are not allocations.
+struct Upload {
+    std::vector<char> host;
+    std::vector<std::pair<void **, size_t>> at;
+    template <class T> int add(T *&dst, const std::vector<T> &src)
+    {
+        const size_t bytes = sizeof(T) * src.size();
+        if (bytes > 32 * 1024) return up(dst, src);
+        const size_t off = (host.size() + 255) & ~size_t(255);
+        host.resize(off + std::max<size_t>(bytes, 1));
+        if (bytes) memcpy(host.data() + off, src.data(), bytes);
+        at.push_back({(void **)&dst, off});
+        return OCRT_OK;
+    }
+    int flush()
+    {
+        if (at.empty()) return OCRT_OK;
+        char *d = (char *)dalloc(host.size());
+        if (!d) return fail(OCRT_ERR_ALLOC, "device allocation failed");
+        for (auto &a : at) *a.first = d + a.second;
+        CK(cudaMemcpyAsync(d, host.data(), host.size(), cudaMemcpyHostToDevice, g_stream));
+        return OCRT_OK;
+    }
+};
+
 template <class T> int alloc(T *&dst, size_t n)
 {
     dst = (T *)dalloc(sizeof(T) * std::max<size_t>(n, 1));
@@ -617,8 +645,9 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
     close(g.P);
     // ---- device buffers ----
     int rc;
-    if ((rc = up(g.px, g.hpx)) || (rc = up(g.tasks, g.htask)) || (rc = up(g.pix_task0, g.hpix_task0)) ||
-        (rc = up(g.mb, mb)) || (rc = up(g.mg, mgv)) || (rc = up(g.ma, ma)) || (rc = up(g.mz, mz)) ||
+    Upload ul;
+    if ((rc = ul.add(g.px, g.hpx)) || (rc = ul.add(g.tasks, g.htask)) || (rc = ul.add(g.pix_task0, g.hpix_task0)) ||
+        (rc = ul.add(g.mb, mb)) || (rc = ul.add(g.mg, mgv)) || (rc = ul.add(g.ma, ma)) || (rc = ul.add(g.mz, mz)) ||
         (rc = alloc(g.state, g.T)) || (rc = alloc(g.tout, g.T)) || (rc = alloc(g.res, g.P)) ||
         (rc = alloc(g.gmu, g.N)) || (rc = alloc(g.gw, g.N)) || (rc = alloc(g.pw, 2 * (size_t)g.N)) ||
         (rc = alloc(g.h, g.nlev)) || (rc = alloc(g.ch, g.nlev)) || (rc = alloc(g.xd, g.nlev)) ||
@@ -646,14 +675,14 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
         (rc = alloc(g.Bx, (size_t)g.wave_tasks * 3 * (1 + G.E) * (g.Lmax + 1))) ||
         (rc = alloc(g.gcoef, (size_t)(g.Mmax + 1) * (g.Lmax + 1) * 5)))
         return rc;
-    if (g.any_layers && ((rc = up(g.ldt, ldt)) || (rc = up(g.lss, lss)))) return rc;
+    if (g.any_layers && ((rc = ul.add(g.ldt, ldt)) || (rc = ul.add(g.lss, lss)))) return rc;
     if (g.any_vk) {
         g.vk_stride = (long long)(g.Mmax + 1) * (G.N + 1) * 2 * G.NR;
-        if ((rc = up(g.vk_th, vth)) || (rc = up(g.vk_p11, vp11)) ||
+        if ((rc = ul.add(g.vk_th, vth)) || (rc = ul.add(g.vk_p11, vp11)) ||
             (rc = alloc(g.vkV, (size_t)g.wave_pix * g.vk_stride)))
             return rc;
     }
-    if (g.any_lut && ((rc = up(g.lut_vza, hlv)) || (rc = up(g.lut_raa, hlr)) ||
+    if (g.any_lut && ((rc = ul.add(g.lut_vza, hlv)) || (rc = ul.add(g.lut_raa, hlr)) ||
                       (rc = alloc(g.lut_samp, (size_t)g.T * g.lut_nvmax * 4)) ||
                       (rc = alloc(g.lut_kappa, (size_t)g.lut_ntot)) || (rc = alloc(g.lut_out, 6 * (size_t)g.lut_ntot))))
         return rc;
@@ -662,7 +691,7 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
         g.gstride = 3 * g.kstride + 2;
         g.grad_stride = 2 * g.ntmax + 1;
         const size_t na = (size_t)g.wave_tasks * ncot;
-        if ((rc = up(g.cot, hcot)) || (rc = alloc(g.lamd, (size_t)g.P * (G.N + 2))) ||
+        if ((rc = ul.add(g.cot, hcot)) || (rc = alloc(g.lamd, (size_t)g.P * (G.N + 2))) ||
             (rc = alloc(g.dTc, g.ncoef)) || (rc = alloc(g.dCa, g.ncoef)) || (rc = alloc(g.dCb, g.ncoef)) ||
             (rc = alloc(g.srfW, g.wave_srf)) || (rc = alloc(g.AF, g.wave_fld * ncot)) ||
             (rc = alloc(g.AJ, g.wave_fld * ncot)) ||
@@ -708,7 +737,7 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
             for (int i = 0; i <= G.N; ++i)
                 if (!(o < G.N && i < G.N && o > i)) pl.push_back(make_short2((short)o, (short)i));
         g.ncmpairs = (int)pl.size();
-        if ((rc = up(g.cmpairs, pl)) || (rc = alloc(g.cstiles, coxmunk_tc_tiles_floats(g.Mmax, g.nphi)))) return rc;
+        if ((rc = ul.add(g.cmpairs, pl)) || (rc = alloc(g.cstiles, coxmunk_tc_tiles_floats(g.Mmax, g.nphi)))) return rc;
     }
     if (g.use_tc && ncot > 0 && tc_adj_supported(G)) {
         const int KP = (G.COUT + 31) & ~31;
@@ -721,7 +750,7 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
         w.n_mol = 0;
         for (int t = w.t0; t < w.t1; ++t) w.n_mol += g.htask[t].has_mol ? 1 : 0;
     }
-    return OCRT_OK;
+    return ul.flush();
 }
 
 #define LAUNCH(plan, cls, ...)                                                        \
@@ -1011,12 +1040,15 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
         // molecular factors it reads are written in full by k_tables, and
         // k_tables_tc writes every row of the plain operator it keeps
         if (!g.fused && (!g.use_tc || (g.ncot > 0 && !g.tabs_tc))) CK(cudaMemsetAsync(g.ops, 0, sizeof(float) * w.ops, st));
-        CK(cudaMemsetAsync(g.pvec, 0, sizeof(float) * (size_t)nw * 2 * G.LDC, st));
         if (g.any_flat) CK(cudaMemsetAsync(g.fvec, 0, sizeof(float) * (size_t)nw * 24 * G.NR, st));
-        CK(cudaMemsetAsync(g.active_cnt, 0, sizeof(int) * ((size_t)g.max_orders + 2), st));
-        CK(cudaMemsetAsync(g.mol_cnt, 0, sizeof(int) * ((size_t)g.max_orders + 2), st));
-        CK(cudaMemsetAsync(g.work, 0, sizeof(int) * 4 * ((size_t)g.max_orders + 2), st));
-        CK(cudaMemsetAsync(g.aflag, 0, (size_t)nw, st));
+        // the order kernel reads no column of an unused slot, lists or counters
+        if (!g.fused) {
+            CK(cudaMemsetAsync(g.pvec, 0, sizeof(float) * (size_t)nw * 2 * G.LDC, st));
+            CK(cudaMemsetAsync(g.active_cnt, 0, sizeof(int) * ((size_t)g.max_orders + 2), st));
+            CK(cudaMemsetAsync(g.mol_cnt, 0, sizeof(int) * ((size_t)g.max_orders + 2), st));
+            CK(cudaMemsetAsync(g.work, 0, sizeof(int) * 4 * ((size_t)g.max_orders + 2), st));
+            CK(cudaMemsetAsync(g.aflag, 0, (size_t)nw, st));
+        }
         LAUNCH(plan, KC_TABLES, k_basis_pix<<<dim3((nw + 32 / (1 + G.E) - 1) / (32 / (1 + G.E)), 2), 32, 0, st>>>(
                    g.tasks, w.t0, nw, g.px, g.Lmax, G.E, g.Bx, g.gcoef));
         if (g.any_vk)
