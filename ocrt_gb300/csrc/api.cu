@@ -1580,19 +1580,26 @@ int ocrt_gb_plan_kernel_stats(ocrt_plan *plan, int cls, const char **name, doubl
                 const TaskDev &tk = g.htask[t];
                 const PixDev &d = g.hpx[tk.pix];
                 const double K = tk.K, nt = d.nt, ords = std::max(0, st[t].orders - 1);
-                const int sc = g.use_tc || g.fused ? KC_SOURCE_TC : KC_SOURCE;
-                plan->flops[sc] += ords * 72.0 * N * N * K;
-                plan->bytes[sc] += ords * (K * 6 * N + K * 6 * NR + 36.0 * N * NR) * 4.0;
-                if (tk.has_mol && (g.use_tc || g.fused)) {          // dense U V inside the tensor-core pass
-                    plan->flops[KC_SOURCE_TC] += ords * 72.0 * N * N * K;
-                    plan->bytes[KC_SOURCE_TC] += ords * (36.0 * N * NR) * 4.0;
-                } else if (tk.has_mol) {               // rank-24 form on CUDA cores
-                    plan->flops[KC_MOL] += ords * 2.0 * K * 24.0 * (N + 6 * NR);
-                    plan->bytes[KC_MOL] += ords * (K * 6 * N + 2.0 * K * 6 * NR) * 4.0;
+                if (g.fused) {
+                    // one kernel: the contraction and the recurrences of every order;
+                    // the operator once, the field written and read back per order
+                    plan->flops[KC_SOURCE_TC] += ords * 72.0 * N * N * K + (ords + 1.0) * 6.0 * N * nt * 5.0;
+                    plan->bytes[KC_SOURCE_TC] += (ords + 1.0) * 2.0 * K * 6 * N * 4.0 + par_bytes(g.G);
+                } else {
+                    const int sc = g.use_tc ? KC_SOURCE_TC : KC_SOURCE;
+                    plan->flops[sc] += ords * 72.0 * N * N * K;
+                    plan->bytes[sc] += ords * (K * 6 * N + K * 6 * NR + 36.0 * N * NR) * 4.0;
+                    if (tk.has_mol && g.use_tc) {          // dense U V inside the tensor-core pass
+                        plan->flops[KC_SOURCE_TC] += ords * 72.0 * N * N * K;
+                        plan->bytes[KC_SOURCE_TC] += ords * (36.0 * N * NR) * 4.0;
+                    } else if (tk.has_mol) {               // rank-24 form on CUDA cores
+                        plan->flops[KC_MOL] += ords * 2.0 * K * 24.0 * (N + 6 * NR);
+                        plan->bytes[KC_MOL] += ords * (K * 6 * N + 2.0 * K * 6 * NR) * 4.0;
+                    }
+                    plan->bytes[KC_SCAN] += ords * (2.0 * 6 * N * K + N * nt) * 4.0;
+                    plan->flops[KC_SCAN] += ords * 6.0 * N * nt * 5.0;
+                    plan->bytes[KC_PRIMARY] += K * 6 * NR * 12.0;
                 }
-                plan->bytes[KC_SCAN] += ords * (2.0 * 6 * N * K + N * nt) * 4.0;
-                plan->flops[KC_SCAN] += ords * 6.0 * N * nt * 5.0;
-                plan->bytes[KC_PRIMARY] += K * 6 * NR * 12.0;
                 const double Lm = d.L - tk.m + 1;
                 plan->flops[KC_TABLES] += 2.0 * 26.0 * NR * N * Lm;
                 plan->bytes[KC_TABLES] += 36.0 * N * NR * 4.0 * (tk.has_mol ? 2 : 1);
