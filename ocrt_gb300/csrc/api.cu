@@ -29,6 +29,11 @@ thread_local std::string g_err;
 int g_device = -1;
 int g_nsm = 152;           // SM count of the device, read at init
 cudaStream_t g_stream = nullptr;
+// A second stream for the surface kernels of an execute, which need only the pixels'
+// geometry and run beside the altitudes, bases and tables (they are joined before the
+// orders); its fork and join events.  Used under g_mu, in the order of the executes.
+cudaStream_t g_side = nullptr;
+cudaEvent_t g_fork = nullptr, g_join = nullptr;
 std::multimap<size_t, void *> g_free;      // caching allocator: size -> block
 std::map<void *, size_t> g_live;
 int *g_pinned = nullptr;
@@ -953,6 +958,24 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
     CK(cudaMemsetAsync(g.err, 0, 2 * sizeof(int), st));
     LAUNCH(plan, KC_SETUP, k_gauss<<<1, 64, 0, st>>>(g.N, g.gmu, g.gw, g.pw));
     LAUNCH(plan, KC_SETUP, k_pixel_setup<<<(P + 127) / 128, 128, 0, st>>>(g.px, P, g.N, g.gmu));
+    // the surface kernels beside the rest of the setup (one pixel 388 -> 346 us, 61 pixels
+    // 1084 -> 1013, 384 pixels 10.36 -> 10.26 ms); timed executes keep one stream, so
+    // that their classes add up
+    const bool fork = !g_timing && (g.any_rough || g.any_water);
+    const cudaStream_t side = fork ? g_side : st;
+    auto forked = [&]() -> int {
+        if (!fork) return OCRT_OK;
+        CK(cudaEventRecord(g_fork, st));
+        CK(cudaStreamWaitEvent(side, g_fork, 0));
+        return OCRT_OK;
+    };
+    auto joined = [&]() -> int {
+        if (!fork) return OCRT_OK;
+        CK(cudaEventRecord(g_join, side));
+        CK(cudaStreamWaitEvent(st, g_join, 0));
+        return OCRT_OK;
+    };
+    if (int rc = forked()) return rc;
     LAUNCH(plan, KC_SETUP, k_levels<<<dim3(lev_blocks(g.ntmax), P), LEV_B, 0, st>>>(g.px, P, g.h, g.ch, g.xd, g.yd, g.z));
     if (g.any_water)
         LAUNCH(plan, KC_SETUP, k_levels_water<<<dim3(2, P), 256, 0, st>>>(g.px, P, g.h, g.ch, g.xd, g.yd, g.z));
@@ -974,10 +997,13 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
         LAUNCH(plan, KC_SETUP, k_mol_vtab<<<std::min(g.Mmax, 2) + 1, 256, 0, st>>>(G, g.Lmax, g.Bp, g.Br, g.Bt, g.gw,
                                                                                   g.molV));
     if (g.any_rough) {
-        LAUNCH(plan, KC_SETUP, k_cs_table<<<g.Mmax + 2, 256, 0, st>>>(g.Mmax, g.nphi, g.cs));
-        if (g.cstiles) LAUNCH(plan, KC_SETUP, k_cs_tiles<<<g.nphi / 64, 256, 0, st>>>(g.Mmax, g.nphi, g.cs, g.cstiles));
         LAUNCH(plan, KC_SETUP, k_seed_att<<<dim3(8, P), 256, 0, st>>>(g.px, P, g.N, g.gmu, g.h, g.Eatt));
-        LAUNCH(plan, KC_SETUP, k_sancer<<<P, 128, 0, st>>>(g.px, P, g.N, g.gmu, g.lam, g.ncot ? g.lamd : nullptr));
+        {
+            const cudaStream_t st = side;
+            LAUNCH(plan, KC_SETUP, k_cs_table<<<g.Mmax + 2, 256, 0, st>>>(g.Mmax, g.nphi, g.cs));
+            if (g.cstiles) LAUNCH(plan, KC_SETUP, k_cs_tiles<<<g.nphi / 64, 256, 0, st>>>(g.Mmax, g.nphi, g.cs, g.cstiles));
+            LAUNCH(plan, KC_SETUP, k_sancer<<<P, 128, 0, st>>>(g.px, P, g.N, g.gmu, g.lam, g.ncot ? g.lamd : nullptr));
+        }
     }
     LAUNCH(plan, KC_SETUP, k_level_float<<<dim3(2, P), 256, 0, st>>>(g.px, P, g.xd, g.yd, g.ch, g.lvf));
     if (g.any_flat) LAUNCH(plan, KC_SETUP, k_flat_fresnel<<<P, 128, 0, st>>>(g.px, P, g.N, g.gmu, g.frs));
@@ -1036,6 +1062,9 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
     for (Wave &w : g.waves) {
         const int nw = w.t1 - w.t0;
         if (!capture) w.fwd_stop = INT_MAX;
+        // the wave before has read the surface kernels' buffer
+        if (&w != &g.waves[0])
+            if (int rc = forked()) return rc;
         // the plain operators are read only off the forward tensor-core path; the
         // molecular factors it reads are written in full by k_tables, and
         // k_tables_tc writes every row of the plain operator it keeps
@@ -1085,7 +1114,9 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
         if (g.use_tc)
             LAUNCH(plan, KC_TABLES, k_mol_dense<<<nw, 256, 0, st>>>(g.tasks, w.t0, nw, G, g.Lmax, g.Bp, g.Br, g.Bt,
                                                                      g.gw, g.ops, g.opt));
+        const cudaStream_t main = st;
         if (w.any_rough) {
+            const cudaStream_t st = side;
             const bool dw = g.ncot > 0;
             const int np = w.p1 - w.p0;
             const size_t smem = coxmunk_smem_bytes(g.nphi, dw);
@@ -1104,6 +1135,10 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
                                                            g.ncmpairs, g.err));
             } else {
                 int cb = 256;
+                // launch shapes are timed with nothing beside them
+                if (fork && !capture &&
+                    !g_tune_idx.count({dw ? "k_coxmunk_dw" : "k_coxmunk", std::vector<int>{G.N, g.nphi, g.Mmax}}))
+                    CK(cudaStreamSynchronize(main));
                 rc = tuned_block(dw ? "k_coxmunk_dw" : "k_coxmunk",
                                  dw ? (const void *)k_coxmunk_dw : (const void *)k_coxmunk, {G.N, g.nphi, g.Mmax},
                                  !capture, st, coxmunk, &cb);
@@ -1111,10 +1146,13 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
                 LAUNCH(plan, KC_COXMUNK, coxmunk(cb));
             }
         }
-        if (w.any_water)
+        if (w.any_water) {
+            const cudaStream_t st = side;
             LAUNCH(plan, KC_COXMUNK, k_rww<<<dim3(G.NR, w.p1 - w.p0), 256,
                                              iface_smem_bytes(g.Mmax, g.nphi_ww, 0), st>>>(
                        g.tasks, g.px, w.p0, g.pix_task0, G, g.gmu, g.nphi_ww, g.srf));
+        }
+        if ((rc = joined())) return rc;
         const dim3 sgrid(w.n_simt, (w.Kmax + ST_M_TILE - 1) / ST_M_TILE, (G.COUT + ST_N_TILE - 1) / ST_N_TILE);
         const int mtiles = (w.Kmax + 127) / 128;
         const int lt = mol_levels(w.n_mol, w.Kmax, g_nsm), ltiles = (w.Kmax + lt - 1) / lt;
@@ -1305,6 +1343,9 @@ int ocrt_gb_init(int device)
     if (device < 0 || device >= n) return fail(OCRT_ERR_ARGS, "device index out of range");
     CK(cudaSetDevice(device));
     CK(cudaStreamCreateWithFlags(&g_stream, cudaStreamNonBlocking));
+    CK(cudaStreamCreateWithFlags(&g_side, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&g_fork, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&g_join, cudaEventDisableTiming));
     CK(cudaMallocHost(&g_pinned, sizeof(int) * 16));
     CK(cudaDeviceGetAttribute(&g_nsm, cudaDevAttrMultiProcessorCount, device));
     CK(cudaFuncSetAttribute(k_coxmunk, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -1335,11 +1376,14 @@ void ocrt_gb_shutdown(void)
     std::lock_guard<std::mutex> lk(g_mu);
     if (g_device < 0) return;
     cudaStreamSynchronize(g_stream);
+    cudaStreamSynchronize(g_side);
     for (auto &kv : g_free) cudaFree(kv.second);
     for (auto &kv : g_live) cudaFree(kv.first);
     g_free.clear(); g_live.clear();
     cudaFreeHost(g_pinned); g_pinned = nullptr;
     cudaStreamDestroy(g_stream); g_stream = nullptr;
+    cudaStreamDestroy(g_side); g_side = nullptr;
+    cudaEventDestroy(g_fork); cudaEventDestroy(g_join); g_fork = g_join = nullptr;
     g_device = -1;
 }
 
@@ -1523,6 +1567,11 @@ int ocrt_gb_plan_execute(ocrt_plan *plan, void *stream)
         plan->launches = 0;
         for (int c = 0; c < KC_N; ++c) plan->cnt[c] = 0;
     }
+    // an eager execute may synchronise (host polls, tuning): not under a caller's capture
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone)
+        for (const Group &g : plan->groups)
+            if (g.max_orders > 1) return fail(OCRT_ERR_DEVICE, "the stream is being captured");
     for (Group &g : plan->groups) {
         const int rc = run_group(plan, g, st, false);
         if (rc) return rc;
@@ -1662,7 +1711,7 @@ void ocrt_gb_plan_destroy(ocrt_plan *plan)
 {
     if (!plan) return;
     std::lock_guard<std::mutex> lk(g_mu);
-    if (g_stream) cudaStreamSynchronize(g_stream);
+    if (g_stream) { cudaStreamSynchronize(g_stream); cudaStreamSynchronize(g_side); }
     for (Group &g : plan->groups) free_group(g);
     for (auto &e : plan->ev) { cudaEventDestroy(e.second.first); cudaEventDestroy(e.second.second); }
     if (plan->gexec) cudaGraphExecDestroy(plan->gexec);
