@@ -28,11 +28,11 @@
 // zero-weight outputs and, for m <= 2, three molecular functionals (xi_A, xi_B,
 // xi_0), which give the molecular source as row factor x xi.
 //
-// Measured, 192 pixels x 17 modes at 32 streams and 200 levels (32420
+// Measured, 384 pixels x 33 modes at 32 streams and 50 to 400 levels (65181
 // order-modes, rough surface, aerosol): 6.9 ms for all orders against 19.2 ms
-// of order-1, source and scan passes; 24 streams, which the tensor-core source
-// does not take, 3.7 ms against 20 ms of CUDA-core source, molecular, order-1 and
-// scan passes; one pixel at 400 levels 0.38 ms against 1.7 ms.  What bounds it is an
+// of order-1, source and scan passes; 500 pixels x 17 modes at 24 streams, which the
+// tensor-core source does not take, 3.6 ms against 20 ms of CUDA-core source,
+// molecular, order-1 and scan passes; one pixel at 400 levels 0.38 ms against 1.7 ms.  What bounds it is an
 // order's serial chain, 29 000 cycles at 201 levels: 9 000 to the first tile (field
 // rows back from L2, then per stage 1500 to split it, 1500 of MMA and 600 of
 // barriers, two stages in flight), 6 700 to the second, 11 000 for the upward scan
