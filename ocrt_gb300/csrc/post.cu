@@ -313,10 +313,15 @@ __global__ void k_ipss(const PixDev *px, int P, const double *h, const double *z
     }
 }
 
+// The correction is even about the principal plane, so an azimuth r and its mirror
+// image 360 - r share one evaluation; this key (exact: r is at least 180 where it is
+// subtracted) is equal for exactly those.
+__device__ __forceinline__ double ipss_azimuth_key(double r) { return r > 180.0 ? 360.0 - r : r; }
+
 // IPSS kappa at every (vza, raa) of each pixel's LUT grid: blocks stride over
-// the directions of a pixel.  The correction is even in the azimuth, so a
-// direction whose mirror image 360 - raa stands earlier in the grid is
-// written by the block of that one.
+// the directions of a pixel.  The first azimuth of a key, in whatever order the grid
+// lists them, is evaluated and written to every entry with that key, so each entry
+// has one writer.
 __global__ void k_ipss_lut(const PixDev *px, int P, const double *h, const double *z, const double *xd,
                            const double *yd, const double *tabs, const double *mb, const double *vk_th,
                            const double *vk_p11, const double *lut_vza, const double *lut_raa, double *lut_kappa)
@@ -336,9 +341,9 @@ __global__ void k_ipss_lut(const PixDev *px, int P, const double *h, const doubl
     int have = -1;
     for (int pt = blockIdx.x; pt < npts; pt += gridDim.x) {
         const int iv = pt / d.lut_nr, ir = pt - iv * d.lut_nr;
-        const double r = raa[ir], mr = 360.0 - r;
+        const double r = raa[ir], key = ipss_azimuth_key(r);
         int before = 0;
-        for (int k = threadIdx.x; k < ir; k += blockDim.x) before |= raa[k] == mr;
+        for (int k = threadIdx.x; k < ir; k += blockDim.x) before |= ipss_azimuth_key(raa[k]) == key;
         if (__syncthreads_or(before)) continue;
         if (have < 0) have = ipss_pixel(d, h, z, xd, m);
         double Iss = 0.0, Ipp = 0.0;
@@ -346,7 +351,7 @@ __global__ void k_ipss_lut(const PixDev *px, int P, const double *h, const doubl
                   true, &Iss, &Ipp);
         const double kap = ipss_ratio(Iss, Ipp);
         for (int k = ir + threadIdx.x; k < d.lut_nr; k += blockDim.x)
-            if (k == ir || raa[k] == mr) out[iv * d.lut_nr + k] = kap;
+            if (ipss_azimuth_key(raa[k]) == key) out[iv * d.lut_nr + k] = kap;
     }
 }
 
