@@ -364,8 +364,11 @@ k_coxmunk_tc(const TaskDev *tasks, const PixDev *px, int p0, const int *pix_task
             }
             if (stop) break;
         }
-        // a copy still in flight lands before the CTA leaves
-        if (*abort_flag && copied > 0) (void)mbar_wait(&bfull[(copied - 1) % NBST], ((copied - 1) / NBST) & 1);
+        // copies still in flight, one per stage at most, land before the CTA leaves
+        // (without an abort each has been waited for above)
+        if (*abort_flag)
+            for (int k = max(0, copied - NBST); k < copied; ++k) (void)mbar_wait(&bfull[k % NBST], (k / NBST) & 1);
+        __syncwarp();
         if (elect_one()) umma_commit(fin);
         __syncwarp();
     }
