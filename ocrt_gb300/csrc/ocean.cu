@@ -24,6 +24,7 @@
 // quadrature sums over many terms accumulate in FP64.
 #include "kernels.cuh"
 #include "physics.cuh"
+#include "sum2.cuh"
 
 namespace {
 
@@ -468,17 +469,47 @@ __global__ void k_water_modes(OceanPix *op, int P, const PixDev *pxw, const int 
 // projections per block instead of 1120.  Bound: FP32 issue of the Mueller
 // evaluations.  The quadrature nodes of one ring segment are consecutive, so
 // a thread (azimuth q, node class) keeps the segment's two sums of 9 entries
-// in registers; the node constants (FP64 differences, then FP32) are formed
-// once per block, as FP64 issues at 2 per clock and SM here.
+// in registers.
+//
+// Precision.  With a projection per quadrature node the rounding of 1120 FP32
+// projections averaged out in an FP64 sum; with one per ring node it does not, so
+// the sums over nodes and over azimuths are kept in two words (sum2.cuh; FP64 issues
+// at 2 lanes per clock and SM here): FP32 over at most CWA_SLICE / CWA_GRP nodes of a
+// thread, two words across threads, slices and azimuths.  The node weights and
+// sines are rounded once from FP64.  Error of the sums alone, on the FP32 matrices
+// and relative to the largest output (8 to 48 streams, rms): 2.3e-9..3.2e-9 as here,
+// 6.1e-9..7.7e-9 with a projection per quadrature node, 0.7e-8..1.2e-8 with one per
+// ring node and plain FP32 sums.
 #define CWA_WIN 1024
 #define CWA_GLO 96
 #define CWA_NODES (CWA_WIN + CWA_GLO)
 #define CWA_GRP 4                                   // node classes (256 threads over 64 azimuths)
+#define CWA_SLICE 128                               // nodes summed between two hand-overs
+#define CWA_HALF 64                                 // azimuths of the half grid
 size_t couple_wa_smem_bytes(int M, int NRw)
 {
-    return sizeof(double) * (3 * (size_t)(M + 1) + NRw) +
-           sizeof(float) * (iface_floats(M, 128) + 5 * (size_t)CWA_NODES + (size_t)CWA_GRP * 18 * 64 + 9 * 64) +
-           sizeof(int) * 3 * ((size_t)NRw + 1) + 16;
+    const size_t m1 = (size_t)M + 1, pitch = CWA_HALF + 1;
+    return sizeof(double) * (12 * m1 + 2 * (size_t)NRw) +
+           sizeof(float) * (m1 * 2 * pitch + 5 * (size_t)CWA_NODES + (size_t)CWA_GRP * 18 * CWA_HALF + 4 * 9 * pitch) +
+           sizeof(int) * 3 * ((size_t)NRw + 1);
+}
+
+// Fourier coefficients of a two-word kernel sampled on the half grid, heads H and
+// tails L of rows of half + 1: as project_block with the U fold, in two words, to FP64.
+// 2 dphi / (2 pi) and 2 dphi / pi of the half grid are 1 / half and 2 / half.
+__device__ void project_block2(const float *H, const float *L, const float *cs, int half, int M, double *out)
+{
+    for (int o = threadIdx.x; o < (M + 1) * 9; o += blockDim.x) {
+        const int m = o / 9, e = o - 9 * m;
+        const int sin_e = (e == 2 || e == 5 || e == 6 || e == 7);
+        const float *t = cs + (size_t)(2 * m + sin_e) * (half + 1), *h = H + e * (half + 1), *l = L + e * (half + 1);
+        float s = 0.f, c = 0.f;
+#pragma unroll 4
+        for (int q = 0; q < half; ++q) sum2_mul_add(s, c, h[q], l[q], t[q]);
+        const double v = ((double)s + (double)c) * ((m == 0 ? 1.0 : 2.0) / half);
+        out[o] = m > 0 && (e == 2 || e == 5) ? -v : v;
+    }
+    __syncthreads();
 }
 
 __global__ void __launch_bounds__(256)
@@ -501,24 +532,24 @@ k_couple_wa(const OceanPix *op, int P, const PixDev *pxa, const PixDev *pxw, con
         mua = o.mu_va;
         M = o.m_nodes;
     }
-    constexpr int half = 64;
+    constexpr int half = CWA_HALF, pitch = half + 1;
     extern __shared__ double smd[];
     double *acc = smd;                               // [3 (M + 1)]
-    double *wmu = acc + 3 * (M + 1);                 // sorted unique water cosines [NRw]
-    float *cs = reinterpret_cast<float *>(wmu + NRw);
-    float *Rq = cs + (size_t)(M + 1) * 2 * (half + 1);
-    float *out = Rq + 9 * (half + 1);
-    float *nd = cs + iface_floats(M, 2 * half);      // [5][CWA_NODES]: mu, sine, shadowing, xi w (1 - t), xi w t
+    double *out = acc + 3 * (M + 1);                 // [9 (M + 1)]
+    double *wmu = out + 9 * (M + 1);                 // sorted unique water cosines [NRw]
+    double *winv = wmu + NRw;                        // 1 / gap to the next one [NRw]
+    float *cs = reinterpret_cast<float *>(winv + NRw);
+    float *nd = cs + (size_t)(M + 1) * 2 * pitch;    // [5][CWA_NODES]: mu, sine, shadowing, xi w (1 - t), xi w t
     float *part = nd + 5 * CWA_NODES;                // [CWA_GRP][18][half]
-    float *carry = part + CWA_GRP * 18 * half;       // [9][half]: the next ring node's sum so far
-    int *wsrc = reinterpret_cast<int *>(carry + 9 * half);   // ring slots of wmu [NRw]
+    float *sums = part + CWA_GRP * 18 * half;        // [ring node mod 2][head, tail][9][pitch]
+    int *wsrc = reinterpret_cast<int *>(sums + 4 * 9 * pitch);   // ring slots of wmu [NRw]
     int *wbeg = wsrc + NRw, *gbeg = wbeg + NRw + 1;  // first window / Gauss node of each segment
     __shared__ double srt[OCRT_MAX_N + OCRT_MAX_EXTRA];
     __shared__ int sid[OCRT_MAX_N + OCRT_MAX_EXTRA];
     __shared__ int nu_s;
     fill_cs(cs, M, half);
     for (int x = tid; x < 3 * (M + 1); x += blockDim.x) acc[x] = 0.0;
-    for (int x = tid; x < 9 * half; x += blockDim.x) carry[x] = 0.f;
+    for (int x = tid; x < 4 * 9 * pitch; x += blockDim.x) sums[x] = 0.f;
     const int n = dw.n_ring;
     if (tid < n) {
         const double mk = ring_mu(dw, gmu, N, tid);
@@ -563,6 +594,7 @@ k_couple_wa(const OceanPix *op, int P, const PixDev *pxa, const PixDev *pxw, con
         }
         wbeg[s] = w;
         gbeg[s] = g;
+        if (s + 1 < nu) winv[s] = 1.0 / (wmu[s + 1] - wmu[s]);
     }
     __syncthreads();
     const float lama = sancer_f((float)mua, slen);
@@ -574,24 +606,28 @@ k_couple_wa(const OceanPix *op, int P, const PixDev *pxa, const PixDev *pxw, con
         const int id = i < CWA_WIN ? i : i - CWA_WIN;
         int a = 0, b = nu - 1;                       // beg[a] <= id < beg[b]
         while (b - a > 1) { const int c = (a + b) >> 1; if (beg[c] <= id) a = c; else b = c; }
-        const float x = (float)xi, d0 = (float)(xi - wmu[a]), d1 = (float)(wmu[a + 1] - xi);
-        const float wx = x * (float)wi / (float)(wmu[a + 1] - wmu[a]);
+        const float x = (float)xi;
+        const double wx = xi * wi * winv[a], s2 = 1.0 - xi * xi;
+        const float sh = (float)s2;
         nd[i] = x;
-        nd[CWA_NODES + i] = sqrtf(fmaxf(0.f, (float)(1.0 - xi) * (1.f + x)));
+        nd[CWA_NODES + i] = s2 > 0.0 ? sum2_sqrt(sh, (float)(s2 - (double)sh)) : 0.f;
         nd[2 * CWA_NODES + i] = 1.f / (1.f + sancer_f(x, slen) + lama);
-        nd[3 * CWA_NODES + i] = wx * d1;
-        nd[4 * CWA_NODES + i] = wx * d0;
+        nd[3 * CWA_NODES + i] = (float)(wx * (wmu[a + 1] - xi));
+        nd[4 * CWA_NODES + i] = (float)(wx * (xi - wmu[a]));
     }
     __syncthreads();
     const double *ew = edge_w + (size_t)task0_w[o.pw] * NRw * OCRT_EDGE;
-    // projection of ring node s from Rq and its contraction with the field
+    // projection of ring node s and its contraction with the field; its sums then
+    // become those of node s + 2
     auto contract = [&](int s) {
-        project_block(Rq, cs, half, M, true, out);
+        float *S = sums + (s & 1) * 2 * 9 * pitch;
+        project_block2(S, S + 9 * pitch, cs, half, M, out);
+        for (int x = tid; x < 2 * 9 * pitch; x += blockDim.x) S[x] = 0.f;
         for (int x = tid; x < 3 * (M + 1); x += blockDim.x) {
             const int m = x / 3, r = x - 3 * m;
-            const float *T = out + m * 9 + r * 3;
+            const double *T = out + m * 9 + r * 3;
             const double *e = ew + ((size_t)m * NRw + wsrc[s]) * OCRT_EDGE;
-            const double v = (double)T[0] * e[0] + (double)T[1] * e[1] + (double)T[2] * e[2];
+            const double v = T[0] * e[0] + T[1] * e[1] + T[2] * e[2];
             acc[x] += (m == 0 ? 2.0 * OCRT_PI : OCRT_PI) * v;
         }
     };
@@ -599,40 +635,42 @@ k_couple_wa(const OceanPix *op, int P, const PixDev *pxa, const PixDev *pxw, con
     float sp, cp;
     sincosf((q + 0.5f) * (3.14159265359f / (float)half), &sp, &cp);
     for (int s = 0; s + 1 < nu; ++s) {
-        float a[9], b[9];
-#pragma unroll
-        for (int e = 0; e < 9; ++e) a[e] = b[e] = 0.f;
         const int w0 = wbeg[s], nwin = wbeg[s + 1] - w0, g0 = gbeg[s], nn = nwin + gbeg[s + 1] - g0;
-        for (int k = grp; k < nn; k += CWA_GRP) {
-            const int i = k < nwin ? w0 + k : CWA_WIN + g0 + (k - nwin);
-            const float wa = nd[3 * CWA_NODES + i], wb = nd[4 * CWA_NODES + i];
-            if (wa == 0.f && wb == 0.f) continue;
-            float T[9];
-            twa_mueller((float)mua, sva, nd[i], nd[CWA_NODES + i], cp, sp, s2v, nd[2 * CWA_NODES + i], nw, o.qc, T);
+        int k0 = 0;
+        do {                                         // once at least: its barriers also part two contractions
+            float a[9], b[9];
 #pragma unroll
-            for (int e = 0; e < 9; ++e) { a[e] = fmaf(wa, T[e], a[e]); b[e] = fmaf(wb, T[e], b[e]); }
-        }
+            for (int e = 0; e < 9; ++e) a[e] = b[e] = 0.f;
+            const int k1 = min(nn, k0 + CWA_SLICE);
+            for (int k = k0 + grp; k < k1; k += CWA_GRP) {
+                const int i = k < nwin ? w0 + k : CWA_WIN + g0 + (k - nwin);
+                const float wa = nd[3 * CWA_NODES + i], wb = nd[4 * CWA_NODES + i];
+                if (wa == 0.f && wb == 0.f) continue;
+                float T[9];
+                twa_mueller((float)mua, sva, nd[i], nd[CWA_NODES + i], cp, sp, s2v, nd[2 * CWA_NODES + i], nw, o.qc, T);
 #pragma unroll
-        for (int e = 0; e < 9; ++e) {
-            part[(grp * 18 + e) * half + q] = a[e];
-            part[(grp * 18 + 9 + e) * half + q] = b[e];
-        }
-        __syncthreads();
-        for (int x = tid; x < 9 * half; x += blockDim.x) {
-            const int e = x / half, qq = x - e * half;
-            float va = carry[x], vb = 0.f;
-#pragma unroll
-            for (int g = 0; g < CWA_GRP; ++g) {
-                va += part[(g * 18 + e) * half + qq];
-                vb += part[(g * 18 + 9 + e) * half + qq];
+                for (int e = 0; e < 9; ++e) { a[e] = fmaf(wa, T[e], a[e]); b[e] = fmaf(wb, T[e], b[e]); }
             }
-            Rq[e * (half + 1) + qq] = va;
-            carry[x] = vb;
-        }
-        __syncthreads();
+#pragma unroll
+            for (int e = 0; e < 9; ++e) {
+                part[(grp * 18 + e) * half + q] = a[e];
+                part[(grp * 18 + 9 + e) * half + q] = b[e];
+            }
+            __syncthreads();
+            for (int x = tid; x < 18 * half; x += blockDim.x) {
+                const int j = x / half, qq = x - j * half, e = j < 9 ? j : j - 9;
+                float *S = sums + ((j < 9 ? s : s + 1) & 1) * 2 * 9 * pitch + e * pitch + qq;
+                float h = S[0], l = S[9 * pitch];
+#pragma unroll
+                for (int g = 0; g < CWA_GRP; ++g) sum2_add(h, l, part[(g * 18 + j) * half + qq]);
+                S[0] = h;
+                S[9 * pitch] = l;
+            }
+            __syncthreads();
+            k0 += CWA_SLICE;
+        } while (k0 < nn);
         contract(s);
     }
-    for (int x = tid; x < 9 * half; x += blockDim.x) Rq[(x / half) * (half + 1) + (x % half)] = carry[x];
     __syncthreads();
     contract(nu - 1);
     const double f = o.F_w / OCRT_PI;
