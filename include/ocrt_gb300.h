@@ -169,14 +169,20 @@ int ocrt_gb_solve_batch(int n, const ocrt_case *cases,
  * A plan holds the device copy of a batch.  ocrt_gb_plan_execute runs the
  * full solve on device-resident inputs (no host traffic); results stay on the
  * device until ocrt_gb_plan_results copies them out.
- * The first execute runs eagerly: host polls of the device active-task counts
- * end each order loop, and the order count each wave needed is recorded.  The
- * second execute captures the same launch sequence with those counts and no
- * host polls into a CUDA graph; later executes replay the graph (one launch
- * call, no host synchronisation).  A replay that ends with a task still
- * iterating is reported by ocrt_gb_plan_results as an error and the plan goes
- * back to eager executes.  OCRT_GB_GRAPH=0, or timing enabled, keeps every
- * execute eager. */
+ * An execute returns with its work queued on the stream.  What touches the
+ * plan's buffers next waits for it, on whichever stream it was: a later
+ * execute, ocrt_gb_plan_results and ocrt_gb_plan_gradients on the device,
+ * ocrt_gb_plan_kernel_stats and ocrt_gb_plan_destroy on the host.  (Replays of a
+ * graph that the caller captured an execute into are the caller's to order.)
+ * The first execute runs eagerly, the second captures the same launch sequence
+ * into a CUDA graph, later ones replay it (one launch call, no host
+ * synchronisation).  Where all orders of a task run in one kernel, the kernel
+ * itself ends them.  On the separate per-order passes the eager execute ends
+ * each order loop by host polls of the device's active-task counts and records
+ * the order count, with which the graph is captured; a replay that ends with a
+ * task still iterating is reported by ocrt_gb_plan_results as an error and the
+ * plan goes back to eager executes.  OCRT_GB_GRAPH=0, or timing enabled, keeps
+ * every execute eager. */
 typedef struct ocrt_plan ocrt_plan;
 int  ocrt_gb_plan_create(int n, const ocrt_case *cases,
                          const ocrt_opts *opts, int opts_per_case,

@@ -411,6 +411,11 @@ struct ocrt_plan {
     int executes = 0;
     bool graph_off = false;
     long long graph_launches = 0;
+    // Where the last execute was queued: nowhere, on the library's stream, or on a
+    // caller's, which may be gone by the time the plan is looked at again, so that an
+    // event is recorded behind it.
+    enum { NOWHERE, LIBRARY, CALLER } last = NOWHERE;
+    cudaEvent_t done = nullptr;
 };
 
 namespace {
@@ -1537,13 +1542,42 @@ int group_flags(ocrt_plan *plan, Group &g, cudaStream_t st)
     return OCRT_OK;
 }
 
-} // namespace
-
-int ocrt_gb_plan_execute(ocrt_plan *plan, void *stream)
+bool being_captured(cudaStream_t st)
 {
-    if (!plan) return fail(OCRT_ERR_ARGS, "null plan");
-    std::lock_guard<std::mutex> lk(g_mu);
-    cudaStream_t st = stream ? (cudaStream_t)stream : g_stream;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone;
+}
+
+// An execute returns with its work queued, and its buffers are its own until that has
+// ended.  Called before anything else touches them: work on st waits for it.
+int after_last(ocrt_plan *plan, cudaStream_t st)
+{
+    if (plan->last == ocrt_plan::NOWHERE || (plan->last == ocrt_plan::LIBRARY && st == g_stream)) return OCRT_OK;
+    if (!plan->done) CK(cudaEventCreateWithFlags(&plan->done, cudaEventDisableTiming));
+    if (plan->last == ocrt_plan::LIBRARY) CK(cudaEventRecord(plan->done, g_stream));
+    CK(cudaStreamWaitEvent(st, plan->done, 0));
+    return OCRT_OK;
+}
+
+// and after an execute (or the part of one that was queued before it failed) on st
+int mark_last(ocrt_plan *plan, cudaStream_t st)
+{
+    plan->last = st == g_stream ? ocrt_plan::LIBRARY : ocrt_plan::CALLER;
+    if (st == g_stream) return OCRT_OK;
+    if (!plan->done) CK(cudaEventCreateWithFlags(&plan->done, cudaEventDisableTiming));
+    CK(cudaEventRecord(plan->done, st));
+    return OCRT_OK;
+}
+
+// The host waits for the plan's queued work.
+void wait_last(ocrt_plan *plan)
+{
+    if (g_stream) { cudaStreamSynchronize(g_stream); cudaStreamSynchronize(g_side); }
+    if (plan->last == ocrt_plan::CALLER && plan->done) cudaEventSynchronize(plan->done);
+}
+
+int execute_on(ocrt_plan *plan, cudaStream_t st, bool captured)
+{
     plan->launches = 0;
     for (auto &e : plan->ev) { cudaEventDestroy(e.second.first); cudaEventDestroy(e.second.second); }
     plan->ev.clear();
@@ -1568,8 +1602,7 @@ int ocrt_gb_plan_execute(ocrt_plan *plan, void *stream)
         for (int c = 0; c < KC_N; ++c) plan->cnt[c] = 0;
     }
     // an eager execute may synchronise (host polls, tuning): not under a caller's capture
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone)
+    if (captured)
         for (const Group &g : plan->groups)
             if (g.max_orders > 1) return fail(OCRT_ERR_DEVICE, "the stream is being captured");
     for (Group &g : plan->groups) {
@@ -1580,11 +1613,32 @@ int ocrt_gb_plan_execute(ocrt_plan *plan, void *stream)
     return OCRT_OK;
 }
 
+} // namespace
+
+int ocrt_gb_plan_execute(ocrt_plan *plan, void *stream)
+{
+    if (!plan) return fail(OCRT_ERR_ARGS, "null plan");
+    std::lock_guard<std::mutex> lk(g_mu);
+    cudaStream_t st = stream ? (cudaStream_t)stream : g_stream;
+    // under a caller's capture nothing is queued yet: its graph's replays are the
+    // caller's to order
+    const bool captured = being_captured(st);
+    int rc = captured ? OCRT_OK : after_last(plan, st);
+    if (rc) return rc;
+    rc = execute_on(plan, st, captured);
+    if (!captured) {
+        const int rm = mark_last(plan, st);
+        if (!rc) rc = rm;
+    }
+    return rc;
+}
+
 int ocrt_gb_plan_results(ocrt_plan *plan, ocrt_result *out, void *stream)
 {
     if (!plan || (!out && plan->n > 0)) return fail(OCRT_ERR_ARGS, "null plan or output");
     std::lock_guard<std::mutex> lk(g_mu);
     cudaStream_t st = stream ? (cudaStream_t)stream : g_stream;
+    if (const int rc = after_last(plan, st)) return rc;
     double om = 0;
     for (Group &g : plan->groups) {
         std::vector<ocrt_result> r(g.P);
@@ -1606,8 +1660,8 @@ int ocrt_gb_plan_kernel_stats(ocrt_plan *plan, int cls, const char **name, doubl
     if (cls == -1) return KC_N;
     if (cls < 0 || cls >= KC_N) return fail(OCRT_ERR_ARGS, "kernel class out of range");
     std::lock_guard<std::mutex> lk(g_mu);
+    if (!plan->ev.empty() || !plan->work_done) wait_last(plan);
     if (!plan->ev.empty()) {
-        CK(cudaStreamSynchronize(g_stream));
         for (auto &e : plan->ev) {
             float t = 0.f;
             if (cudaEventSynchronize(e.second.second) == cudaSuccess &&
@@ -1711,8 +1765,9 @@ void ocrt_gb_plan_destroy(ocrt_plan *plan)
 {
     if (!plan) return;
     std::lock_guard<std::mutex> lk(g_mu);
-    if (g_stream) { cudaStreamSynchronize(g_stream); cudaStreamSynchronize(g_side); }
+    wait_last(plan);
     for (Group &g : plan->groups) free_group(g);
+    if (plan->done) cudaEventDestroy(plan->done);
     for (auto &e : plan->ev) { cudaEventDestroy(e.second.first); cudaEventDestroy(e.second.second); }
     if (plan->gexec) cudaGraphExecDestroy(plan->gexec);
     delete plan;
@@ -1755,6 +1810,7 @@ int ocrt_gb_plan_gradients(ocrt_plan *plan, ocrt_grad *grad, void *stream)
         if (!grad[i].d_dtau || !grad[i].d_ssa) return fail(OCRT_ERR_ARGS, "null gradient array");
     std::lock_guard<std::mutex> lk(g_mu);
     cudaStream_t st = stream ? (cudaStream_t)stream : g_stream;
+    if (const int rc = after_last(plan, st)) return rc;
     for (Group &g : plan->groups) {
         std::vector<double> h((size_t)g.P * n_cot * g.grad_stride);
         CK(cudaMemcpyAsync(h.data(), g.grad, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, st));
@@ -2138,7 +2194,10 @@ int ocean_solve(int n, const ocrt_case *cases, const ocrt_opts *opts, int opp, c
     OceanPix *d_op = nullptr;
     ocrt_result *d_out = nullptr;
     ocrt_ocean_result *d_wout = nullptr;
+    // what has been queued reads these buffers: it ends before they go back
     auto cleanup = [&]() {
+        cudaStreamSynchronize(st);
+        cudaStreamSynchronize(g_side);
         for (Group &g : plan.groups) { dfree(g.edge); free_group(g); }
         dfree(d_top); dfree(d_ext3); dfree(d_td); dfree(d_view); dfree(d_glo); dfree(d_op); dfree(d_out); dfree(d_wout);
     };
