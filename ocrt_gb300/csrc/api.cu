@@ -456,6 +456,14 @@ struct Upload {
     }
 };
 
+// Uploads run on the library's stream; work that a caller's stream is about to be given
+// must find them done (a pageable copy returns once it is staged, not once it has landed).
+int uploaded(cudaStream_t st)
+{
+    if (st != g_stream) CK(cudaStreamSynchronize(g_stream));
+    return OCRT_OK;
+}
+
 template <class T> int alloc(T *&dst, size_t n)
 {
     dst = (T *)dalloc(sizeof(T) * std::max<size_t>(n, 1));
@@ -2215,11 +2223,12 @@ int ocean_solve(int n, const ocrt_case *cases, const ocrt_opts *opts, int opp, c
         return rc;
     }
     rc = alloc(GA.edge, (size_t)GA.T * GeA.NR * OCRT_EDGE);
+    if (!rc) rc = uploaded(st);
     if (!rc) rc = run_group(&plan, GA, st, false);
     if (rc) { cleanup(); return rc; }
     // ---- skylight into the water ----
     if ((rc = up(d_op, hop)) || (rc = alloc(d_td, (size_t)n * (GeA.NR + 1))) ||
-        (rc = alloc(d_top, (size_t)n * (Ma + 1) * Nw * 3))) { cleanup(); return rc; }
+        (rc = alloc(d_top, (size_t)n * (Ma + 1) * Nw * 3)) || (rc = uploaded(st))) { cleanup(); return rc; }
     LAUNCH(&plan, KC_COXMUNK, k_taw_direct<<<dim3(Nw + 1, n), 128, 0, st>>>(d_op, n, GA.px, GA.gmu, Nw, GeA.NR, d_td));
     LAUNCH(&plan, KC_COXMUNK, k_ocean_prep<<<(n + 127) / 128, 128, 0, st>>>(d_op, n, GA.pix_task0, GA.gmu, GA.gw, Nw,
                                                                              GeA.NR, GA.edge, d_td));
@@ -2275,6 +2284,7 @@ int ocean_solve(int n, const ocrt_case *cases, const ocrt_opts *opts, int opp, c
     }
     GW.ext = d_top;
     rc = alloc(GW.edge, (size_t)GW.T * GeW.NR * OCRT_EDGE);
+    if (!rc) rc = uploaded(st);
     if (!rc) {
         CK(cudaFuncSetAttribute(k_rww, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)std::min<size_t>(iface_smem_bytes(GW.Mmax, GW.nphi_ww, 0) + 1024, 227 * 1024)));
@@ -2305,7 +2315,7 @@ int ocean_solve(int n, const ocrt_case *cases, const ocrt_opts *opts, int opp, c
         }
         for (int k = 0; k < 96; ++k) { hg[k] = xg[k]; hg[96 + k] = wg[k]; }
         if ((rc = up(d_glo, hg)) || (rc = alloc(d_ext3, (size_t)n * (Ma + 1) * GeA.NR * 3)) ||
-            (rc = alloc(d_view, (size_t)n * 3 * (OCRT_MAX_M + 1)))) { cleanup(); return rc; }
+            (rc = alloc(d_view, (size_t)n * 3 * (OCRT_MAX_M + 1))) || (rc = uploaded(st))) { cleanup(); return rc; }
         CK(cudaMemsetAsync(d_ext3, 0, sizeof(double) * (size_t)n * (Ma + 1) * GeA.NR * 3, st));
         CK(cudaMemsetAsync(d_view, 0, sizeof(double) * (size_t)n * 3 * (OCRT_MAX_M + 1), st));
         LAUNCH(&plan, KC_COXMUNK, k_water_modes<<<(n + 127) / 128, 128, 0, st>>>(d_op, n, GW.px, GW.pix_task0, GeW.NR,
@@ -2322,7 +2332,7 @@ int ocean_solve(int n, const ocrt_case *cases, const ocrt_opts *opts, int opp, c
         return rc;
     }
     GC.ext = d_ext3;
-    if ((rc = run_group(&plan, GC, st, false))) { cleanup(); return rc; }
+    if ((rc = uploaded(st)) || (rc = run_group(&plan, GC, st, false))) { cleanup(); return rc; }
     // ---- outputs ----
     if ((rc = alloc(d_out, n)) || (rc = alloc(d_wout, n))) { cleanup(); return rc; }
     LAUNCH(&plan, KC_FINAL, k_ocean_final<<<(n + 127) / 128, 128, 0, st>>>(
