@@ -988,6 +988,11 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
         CK(cudaStreamWaitEvent(st, g_join, 0));
         return OCRT_OK;
     };
+    // launch shapes are timed with nothing beside them on the other stream
+    auto timed_alone = [&](const char *kernel, const std::vector<int> &key, cudaStream_t other) -> int {
+        if (fork && !capture && autotune_enabled() && !g_tune_idx.count({kernel, key})) CK(cudaStreamSynchronize(other));
+        return OCRT_OK;
+    };
     if (int rc = forked()) return rc;
     LAUNCH(plan, KC_SETUP, k_levels<<<dim3(lev_blocks(g.ntmax), P), LEV_B, 0, st>>>(g.px, P, g.h, g.ch, g.xd, g.yd, g.z));
     if (g.any_water)
@@ -1120,7 +1125,11 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
             // the rows and columns of the parity operator that no pair writes
             if (g.fused) CK(cudaMemsetAsync(g.popt, 0, (size_t)nw * par_bytes(G), st));
             int tb = 256;
-            rc = tuned_block("k_tables", (const void *)k_tables, {G.N, g.Lmax, g.Mmax}, !capture, st, tables, &tb);
+            // the pairs' share of the work depends on the zero-weight slots and on the form
+            // the operator is written in (parity pieces or plain entries)
+            const std::vector<int> tkey = {G.N, g.Lmax, g.Mmax, G.E, g.fused ? 1 : 0};
+            if ((rc = timed_alone("k_tables", tkey, side))) return rc;
+            rc = tuned_block("k_tables", (const void *)k_tables, tkey, !capture, st, tables, &tb);
             if (rc) return rc;
             LAUNCH(plan, KC_TABLES, tables(tb));
         }
@@ -1148,13 +1157,11 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
                                                            g.ncmpairs, g.err));
             } else {
                 int cb = 256;
-                // launch shapes are timed with nothing beside them
-                if (fork && !capture &&
-                    !g_tune_idx.count({dw ? "k_coxmunk_dw" : "k_coxmunk", std::vector<int>{G.N, g.nphi, g.Mmax}}))
-                    CK(cudaStreamSynchronize(main));
-                rc = tuned_block(dw ? "k_coxmunk_dw" : "k_coxmunk",
-                                 dw ? (const void *)k_coxmunk_dw : (const void *)k_coxmunk, {G.N, g.nphi, g.Mmax},
-                                 !capture, st, coxmunk, &cb);
+                const char *name = dw ? "k_coxmunk_dw" : "k_coxmunk";
+                const std::vector<int> ckey = {G.N, g.nphi, g.Mmax};
+                if ((rc = timed_alone(name, ckey, main))) return rc;
+                rc = tuned_block(name, dw ? (const void *)k_coxmunk_dw : (const void *)k_coxmunk, ckey, !capture, st,
+                                 coxmunk, &cb);
                 if (rc) return rc;
                 LAUNCH(plan, KC_COXMUNK, coxmunk(cb));
             }
