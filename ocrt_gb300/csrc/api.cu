@@ -964,7 +964,7 @@ int run_adjoint_wave(ocrt_plan *plan, Group &g, Wave &w, const BatchBufs &B, con
 // counts end each wave's order loop and record where it ended.  Capture: the
 // same launch sequence with the recorded order counts and no host polls, for
 // a CUDA graph; a device check flags a replay that ends with tasks active.
-int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
+int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture, bool captured = false)
 {
     const Geom G = g.G;
     const int P = g.P;
@@ -973,8 +973,9 @@ int run_group(ocrt_plan *plan, Group &g, cudaStream_t st, bool capture)
     LAUNCH(plan, KC_SETUP, k_pixel_setup<<<(P + 127) / 128, 128, 0, st>>>(g.px, P, g.N, g.gmu));
     // the surface kernels beside the rest of the setup (one pixel 388 -> 346 us, 61 pixels
     // 1084 -> 1013, 384 pixels 10.36 -> 10.26 ms); timed executes keep one stream, so
-    // that their classes add up
-    const bool fork = !g_timing && (g.any_rough || g.any_water);
+    // that their classes add up, and so does an execute under a caller's capture, which
+    // would hold the second stream in it until the caller ends it
+    const bool fork = !g_timing && !captured && (g.any_rough || g.any_water);
     const cudaStream_t side = fork ? g_side : st;
     auto forked = [&]() -> int {
         if (!fork) return OCRT_OK;
@@ -1557,12 +1558,6 @@ int group_flags(ocrt_plan *plan, Group &g, cudaStream_t st)
     return OCRT_OK;
 }
 
-bool being_captured(cudaStream_t st)
-{
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone;
-}
-
 // An execute returns with its work queued, and its buffers are its own until that has
 // ended.  Called before anything else touches them: work on st waits for it.
 int after_last(ocrt_plan *plan, cudaStream_t st)
@@ -1621,7 +1616,7 @@ int execute_on(ocrt_plan *plan, cudaStream_t st, bool captured)
         for (const Group &g : plan->groups)
             if (g.max_orders > 1) return fail(OCRT_ERR_DEVICE, "the stream is being captured");
     for (Group &g : plan->groups) {
-        const int rc = run_group(plan, g, st, false);
+        const int rc = run_group(plan, g, st, false, captured);
         if (rc) return rc;
     }
     plan->executes++;
@@ -1637,7 +1632,8 @@ int ocrt_gb_plan_execute(ocrt_plan *plan, void *stream)
     cudaStream_t st = stream ? (cudaStream_t)stream : g_stream;
     // under a caller's capture nothing is queued yet: its graph's replays are the
     // caller's to order
-    const bool captured = being_captured(st);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool captured = cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone;
     int rc = captured ? OCRT_OK : after_last(plan, st);
     if (rc) return rc;
     rc = execute_on(plan, st, captured);
