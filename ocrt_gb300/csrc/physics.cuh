@@ -45,7 +45,7 @@ __device__ inline double clamp01d(double x) { return x <= 0.0 ? 0.0 : (x >= 1.0 
 // copies for the search.
 struct AboveEval {
     int prof;
-    double rh, ah, et_r, et_a;
+    double rh, ah, et_r, et_a, dr, da;       // dr, da: -1 / (h (1 - exp(-ztop / h))), the slopes' factors
     double z[8], lp[8], a45, q0, ft;
     float rh_f, ah_f, et_r_f, et_a_f, z_f[8], lp_f[8], a45_f, q0_f, ft_f;
 };
@@ -68,8 +68,9 @@ __device__ inline void above_init(AboveEval &E, int prof, double ray_h, double a
         E.lp_f[tid] = (float)E.lp[tid];
     } else if (tid == 8 || tid == 9) {
         const double hh = tid == 8 ? ray_h : aer_h, et = exp(-OCRT_ZTOP_KM / hh);
-        if (tid == 8) { E.rh = hh; E.et_r = et; E.rh_f = (float)hh; E.et_r_f = (float)et; }
-        else { E.ah = hh; E.et_a = et; E.ah_f = (float)hh; E.et_a_f = (float)et; }
+        const double ds = -1.0 / (hh * (1.0 - et));
+        if (tid == 8) { E.rh = hh; E.et_r = et; E.dr = ds; E.rh_f = (float)hh; E.et_r_f = (float)et; }
+        else { E.ah = hh; E.et_a = et; E.da = ds; E.ah_f = (float)hh; E.et_a_f = (float)et; }
     } else if (tid == 10) {
         E.prof = prof;
         const double lat = 45.0 * OCRT_PI / 180.0;
@@ -81,20 +82,21 @@ __device__ inline void above_init(AboveEval &E, int prof, double ray_h, double a
     }
 }
 
-// slope, where given: d/dz in FP32
-__device__ inline double above_exp(double z, double h, double et, float *slope = nullptr)
+// slope, where given: d/dz, rounded to FP32 (ds: its factor from the struct; 1 - et has
+// no digits left in FP32 from scale heights of 1e9 km on)
+__device__ inline double above_exp(double z, double h, double et, double ds, float *slope = nullptr)
 {
     if (slope) *slope = 0.f;
     if (z <= 0.0) return 1.0;
     if (z >= OCRT_ZTOP_KM) return 0.0;
     const double e = exp(-z / h);
-    if (slope) *slope = -(float)e / ((float)h * (1.f - (float)et));
+    if (slope) *slope = (float)(e * ds);
     return (e - et) / (1.0 - et);
 }
 
 __device__ inline double above_ray(const AboveEval &E, double z, float *slope = nullptr)
 {
-    if (E.prof == 1) return above_exp(z, E.rh, E.et_r, slope);
+    if (E.prof == 1) return above_exp(z, E.rh, E.et_r, E.dr, slope);
     if (slope) *slope = 0.f;
     if (z <= 0.0) return 1.0;
     if (z >= 84.852) return 0.0;

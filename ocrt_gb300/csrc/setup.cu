@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(LEV_B) k_levels(const PixDev *px, int P, doubl
                 for (int it = 0; it < 64; ++it) {
                     float sr, sa;
                     const double v = (wr != 0.0 ? wr * above_ray(E, zk, &sr) : (sr = 0.f, 0.0)) +
-                                     (wa != 0.0 ? wa * above_exp(zk, ah, E.et_a, &sa) : (sa = 0.f, 0.0));
+                                     (wa != 0.0 ? wa * above_exp(zk, ah, E.et_a, E.da, &sa) : (sa = 0.f, 0.0));
                     const double df = v - target;
                     if (df > 0.0) lo = zk; else hi = zk;
                     double zn = zk - df / (double)(fr * sr + fa * sa);
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(LEV_B) k_levels(const PixDev *px, int P, doubl
         }
         if (aer) {
             sray[tid] = tr * above_ray(E, zk);
-            saer[tid] = ta * above_exp(zk, ah, E.et_a);
+            saer[tid] = ta * above_exp(zk, ah, E.et_a, E.da);
         }
         if (tid > 0) {
             z[o] = zk;
