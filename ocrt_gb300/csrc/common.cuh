@@ -142,6 +142,7 @@ __host__ __device__ inline Geom make_geom(int N, int E = 1)
     g.tot_all = 1;
     g.srf_rp = 0;
     g.srf_sun = g.NR * N * 9;
+    g.direct = 0;
     return g;
 }
 
