@@ -41,8 +41,12 @@
 // (its operands' shared-memory reads), so tiles of 80 with three stages and three
 // in TMEM were slower (7.9 ms), as were 8-level units per producer (7.4).  Order 1
 // is 0.7 ms of it.
-// Against FP64 solves (240 pixels, 24 streams) the reflectance error is 9.6e-7
-// rms, 9.4e-7 with FP32 CUDA-core products.
+// The accumulator truncates at every step, so the incoming components are taken in
+// the order U, Q, I: the sums stay small until the largest products, which come last.
+// Against FP64 solves (96 pixels each, black, rough and flat surfaces) the error of the
+// reflectance is 8.0, 7.6, 7.2 and 6.3e-7 rms at 8, 12, 24 and 28 streams, with FP32
+// CUDA-core products 8.4, 8.2, 7.6 and 8.0e-7 (in the order I, Q, U 8.2, 7.8, 7.9 and
+// 7.6e-7); at 16 and 32 streams 6.6 and 6.3e-7 (7.0 and 6.9e-7).
 //
 // Direct form (G.direct, groups with water columns).  Where the phase function is
 // so forward-peaked that A+ and A- nearly cancel in what goes up, and the order
@@ -577,6 +581,8 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
     volatile int *nop_s = (volatile int *)(tslot + 5);    // operator copies issued
     volatile int *quit = (volatile int *)(tslot + 6);     // [2 orders]: the abort flag as the scan warps act on it
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // incoming component of the x-th stage of a tile
+    auto comp = [&](int x) -> int { return G.direct ? x : 2 - x; };
 
     if (warp == 15) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(512)
@@ -944,11 +950,11 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
         uint32_t gi = 0;                                  // stages filled
         int K = 0, T = 0;
         const float *Fb = nullptr, *lv = nullptr;
-        // half stage j = 2 (3 a + si) + hh of an order: rows of iterations
+        // half stage j = 2 (3 a + x) + hh of an order, component si = comp(x): rows of iterations
         // 2 hh, 2 hh + 1 into registers
         struct Rows { float4 u[2], v[2]; float x[2]; };
         auto load = [&](Rows &d, int j) {
-            const int e = j >> 1, a = e / 3, si = e - 3 * a;
+            const int e = j >> 1, a = e / 3, si = comp(e - 3 * a);
             const int k0 = or_tile(a, T) * OR_TS, nl = min(OR_TS, K - k0);
             const int rb = r16(0) + 8 * (j & 1);
             const float *src = Fb + (size_t)(k0 + rb) * LDC + 2 * N * si + 4 * q;
@@ -962,7 +968,7 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
         };
         // F+- of half a stage into its B tile
         auto fill = [&](const Rows &d, int j, uint32_t st) {
-            const int si = (j >> 1) % 3, rb = r16(0) + 8 * (j & 1);
+            const int si = comp((j >> 1) % 3), rb = r16(0) + 8 * (j & 1);
             // F+ = up + sigma down: for U the sum is F- and the difference F+
             unsigned char *tile = sB + st * OR_BSTAGE;
             const bool sw = si == 2 && !G.direct;
@@ -1053,7 +1059,7 @@ __device__ __forceinline__ void orders_body(const BatchBufs &B, const WaveBufs &
                     or_wait(b, &b.bfull[st], (gi >> 1) & 1);
                     if (__any_sync(0xffffffffu, *b.abort != 0)) { stop = true; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t ta = sa + si * 3 * at, tb = sb + st * (OR_BSTAGE >> 4);
+                    const uint32_t ta = sa + comp(si) * 3 * at, tb = sb + st * (OR_BSTAGE >> 4);
                     if (elect_one()) {
                         // pieces (operator, field) of the six products, the small ones
                         // first: the accumulator is truncated at each step, so the
