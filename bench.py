@@ -391,8 +391,9 @@ def run_ours(args, rank, world):
     value = args.pixels * world / (ms_step / 1e3)
 
     # ---- roofline of the dominant kernel ----
-    # The binding roof is the one the kernel's algorithmic intensity hits first:
-    # tensor (or the FP32 pipes) above the ridge point peak_flops / peak_bw, HBM below.
+    # The roof the kernel's algorithmic intensity hits first: tensor (or the FP32 pipes)
+    # above the ridge point peak_flops / peak_bw, HBM below.  A kernel that is below half
+    # of both is bound by neither but by its own dependences (latency).
     pk = peaks()
     dom = max(kstats, key=lambda k: kstats[k]["ms"])
     d = kstats[dom]
@@ -400,23 +401,22 @@ def run_ours(args, rank, world):
     secs = d["ms"] / 1e3
     ridge = pk["bf16_tflops_sustained"] * 1e12 / (pk["hbm_gbs"] * 1e9)
     intensity = d["flops"] / d["bytes"] if d["bytes"] > 0 else float("inf")
-    tensor_frac = (d["flops"] / secs / 1e12) / pk["bf16_tflops_sustained"] if d["flops"] > 0 else None
+    tensor_frac = (d["flops"] / secs / 1e12) / pk["bf16_tflops_sustained"]
+    hbm_frac = (d["bytes"] / secs / 1e9) / pk["hbm_gbs"]
     if d["flops"] > 0 and intensity >= ridge:
-        achieved = d["flops"] / secs / 1e12
-        roof = {"kernel": dom, "bound": "tensor", "achieved": achieved, "peak": pk["bf16_tflops_sustained"],
-                "unit": "TFLOP/s", "frac": achieved / pk["bf16_tflops_sustained"],
-                "peak_source": f"{pk['src']} bf16 sustained",
-                "traffic": traffic_from_profiles(dom, d["bytes"] / max(d["launches"], 1)),
-                "avg_launch_ms": per_launch_ms, "alg_flops_per_launch": d["flops"] / max(d["launches"], 1),
-                "intensity_flop_per_byte": intensity, "ridge_flop_per_byte": ridge}
+        roof = {"kernel": dom, "bound": "tensor", "achieved": d["flops"] / secs / 1e12,
+                "peak": pk["bf16_tflops_sustained"], "unit": "TFLOP/s", "frac": tensor_frac,
+                "peak_source": f"{pk['src']} bf16 sustained"}
     else:
-        achieved = d["bytes"] / secs / 1e9
-        roof = {"kernel": dom, "bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
-                "frac": achieved / pk["hbm_gbs"], "peak_source": f"{pk['src']} HBM copy",
-                "traffic": traffic_from_profiles(dom, d["bytes"] / max(d["launches"], 1)),
-                "avg_launch_ms": per_launch_ms, "alg_bytes_per_launch": d["bytes"] / max(d["launches"], 1),
-                "intensity_flop_per_byte": intensity if d["flops"] > 0 else None, "ridge_flop_per_byte": ridge,
-                "tensor_frac_of_bf16": tensor_frac}
+        roof = {"kernel": dom, "bound": "hbm", "achieved": d["bytes"] / secs / 1e9, "peak": pk["hbm_gbs"],
+                "unit": "GB/s", "frac": hbm_frac, "peak_source": f"{pk['src']} HBM copy"}
+    if max(tensor_frac, hbm_frac) < 0.5:
+        roof["bound"] = "latency"
+    roof.update({"tensor_frac_of_bf16": tensor_frac, "hbm_frac": hbm_frac, "avg_launch_ms": per_launch_ms,
+                 "alg_flops_per_launch": d["flops"] / max(d["launches"], 1),
+                 "alg_bytes_per_launch": d["bytes"] / max(d["launches"], 1),
+                 "intensity_flop_per_byte": intensity if d["flops"] > 0 else None, "ridge_flop_per_byte": ridge,
+                 "traffic": traffic_from_profiles(dom, d["bytes"] / max(d["launches"], 1))})
     if roof.get("traffic"):
         # DRAM bytes actually moved per launch (measured ratio x algorithmic) over the launch time
         roof["traffic_gbs"] = roof["traffic"] / (per_launch_ms / 1e3) / 1e9

@@ -200,7 +200,8 @@ int  ocrt_gb_plan_graph_ready(const ocrt_plan *plan);
 
 /* Launch-shape autotuner (no reference counterpart).  The Cox-Munk Fourier
  * projection and the phase-table kernels are timed at 128, 256 and 512
- * threads per block the first time a shape (N, n_phi, M / N, L, M) is met,
+ * threads per block the first time a shape (N, n_phi, M / N, L, M, zero-weight
+ * slots, form of the operator) is met,
  * and the fastest is used from then on (OCRT_GB_AUTOTUNE=0: 256 always).
  * Writes one line per tuned shape into buf (NUL-terminated, truncated to
  * len) and returns the length of the full text. */
@@ -211,7 +212,10 @@ int  ocrt_gb_autotune_summary(char *buf, int len);
  * stream.  ocrt_gb_plan_kernel_stats(plan, -1, ...) returns the number of
  * classes; for a class index it returns the class name, summed device time of
  * the last execute, launch count, and the algorithmic FLOPs and bytes that
- * execute performed (derived from the orders each task ran). */
+ * execute performed (derived from the orders each task ran).  Class
+ * source_gemm_tcgen05 is the whole order loop where one kernel runs it, its
+ * bytes then what must cross the memory bus (operators, surface rows, totals;
+ * not the field, which stays in L2), and the source pass otherwise. */
 void ocrt_gb_set_timing(int enable);
 int  ocrt_gb_plan_kernel_stats(ocrt_plan *plan, int cls, const char **name, double *ms,
                                long long *launches, double *alg_flops, double *alg_bytes);

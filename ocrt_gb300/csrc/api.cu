@@ -1695,10 +1695,13 @@ int ocrt_gb_plan_kernel_stats(ocrt_plan *plan, int cls, const char **name, doubl
                 const PixDev &d = g.hpx[tk.pix];
                 const double K = tk.K, nt = d.nt, ords = std::max(0, st[t].orders - 1);
                 if (g.fused) {
-                    // one kernel: the contraction and the recurrences of every order;
-                    // the operator once, the field written and read back per order
-                    plan->flops[KC_SOURCE_TC] += ords * 72.0 * N * N * K + (ords + 1.0) * 6.0 * N * nt * 5.0;
-                    plan->bytes[KC_SOURCE_TC] += (ords + 1.0) * 2.0 * K * 6 * N * 4.0 + par_bytes(g.G);
+                    // one kernel: the contraction (half the products in the parity form)
+                    // and the recurrences of every order.  Bytes are what must come from or
+                    // go to memory: the operator and the surface rows once, the totals;
+                    // the field's round trip per order is L2's
+                    plan->flops[KC_SOURCE_TC] += ords * (g.G.direct ? 72.0 : 36.0) * N * N * K + (ords + 1.0) * 6.0 * N * nt * 5.0;
+                    plan->bytes[KC_SOURCE_TC] += (double)par_bytes(g.G) + (tk.srf_off >= 0 ? 3.0 * N * g.G.srf_rp * 4.0 : 0.0) +
+                                                 (g.ncot ? K : 2.0) * 6.0 * NR * 4.0;
                 } else {
                     const int sc = g.use_tc ? KC_SOURCE_TC : KC_SOURCE;
                     plan->flops[sc] += ords * 72.0 * N * N * K;
