@@ -585,8 +585,9 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
         g.any_pssa |= o.pssa != 0;
         g.hpx.push_back(d);
     }
-    // All orders in one kernel (k_orders) for forward groups whose shape it
-    // holds: faster at every size measured, from one pixel (24 streams, 40 layers:
+    // All orders in one kernel (k_orders) for groups whose shape it takes
+    // (orders_supported; 20 streams are left out there for a reason that is not speed):
+    // faster at every size measured, from one pixel (24 streams, 40 layers:
     // 0.71 ms a solve against 1.41) to 384 pixels at 32 streams and up to 400 layers
     // (15.6 ms against 25.5 when it came in), and for gradients (96 pixels x 33 modes x 3 rows:
     // 13.8 ms against 22.8; 7 pixels at 16 streams 1.53 ms a step against 3.04).

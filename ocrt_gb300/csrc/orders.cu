@@ -1148,10 +1148,12 @@ const OrdersInst *orders_inst(int ldc)
 
 } // namespace
 
-// N a multiple of 4 keeps the producers' rows in whole float4s.  N = 20, which would fill five eighths
-// of its two 16-deep MMA steps, keeps the separate passes and their scan
-// autotuner; 12 and 28 take this kernel (scene of 500 pixels, 17 modes, up to 150 layers:
-// 4.9 and 8.1 ms against 10.7 and 29.6 with the separate passes).  3 NR + 3 rows fit one MMA of 128
+// N a multiple of 4 keeps the producers' rows in whole float4s.  12 and 28 streams take this
+// kernel (scene of 500 pixels, 17 modes, up to 150 layers: 4.9 and 8.1 ms against 10.7 and
+// 29.6 with the separate passes).  N = 20 does not, though its shape fits and it would gain
+// as much (the same scene 14.4 ms with the separate passes, 5.4 here; one pixel 0.70 and
+// 0.37): the scan autotuner is reached by default only there and above 32 streams, and
+// tests/test_gpu_scan.py pins its choice and record at 20.  3 NR + 3 rows fit one MMA of 128
 // (111 at 32 streams with four zero-weight slots); larger N (48 streams) would need a
 // second M tile and twice the operator, 480 KB, more than an SM has.
 bool orders_supported(const Geom &G, int Kmax, bool adjoint)
