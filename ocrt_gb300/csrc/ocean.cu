@@ -479,7 +479,8 @@ __global__ void k_water_modes(OceanPix *op, int P, const PixDev *pxw, const int 
 // sines are rounded once from FP64.  Error of the sums alone, on the FP32 matrices
 // and relative to the largest output (8 to 48 streams, rms): 2.3e-9..3.2e-9 as here,
 // 6.1e-9..7.7e-9 with a projection per quadrature node, 0.7e-8..1.2e-8 with one per
-// ring node and plain FP32 sums.
+// ring node and plain FP32 sums.  64 pixel-bands at 32 streams and 17 modes: 3.5 ms, of
+// which the two-word sums are 0.5; 38 ms with a projection per quadrature node.
 #define CWA_WIN 1024
 #define CWA_GLO 96
 #define CWA_NODES (CWA_WIN + CWA_GLO)
