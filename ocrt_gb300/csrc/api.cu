@@ -734,7 +734,7 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
         for (int i = 0; i < 3 && g.smap_ok; ++i)
             g.smap_ok = scan_tma_maps(G, chs[i], g.J, g.Tot, g.wave_fld, g.Cq, g.ncoef / G.NR, &g.smap[i]) == 0;
     }
-    if (g.smap_ok && g.ncot > 0 && g.AF && !adj_scan_column())
+    if (g.smap_ok && g.ncot > 0 && g.AF && !adj_scan_column() && adj_scan_tma_supported(G))
         g.amap_ok = adj_scan_tma_maps(G, g.AF, g.ATot, g.wave_fld * g.ncot, g.Cq, g.ncoef / G.NR, &g.amap) == 0;
     g.use_tc = tc_supported(G) && !force_simt() && !g.fused;
     if (g.fused && ((rc = alloc(g.popt, (size_t)g.wave_tasks * par_bytes(G))) ||

@@ -341,7 +341,7 @@ __global__ void k_scan(BatchBufs B, WaveBufs W, Geom G, int t0, int it);
 __global__ void k_scan4(BatchBufs B, WaveBufs W, Geom G, int t0, int it);
 // k_scan_tma<CH, NS> (levels per chunk, ring stages) instances: (8, 3), (8, 4), (4, 6), (16, 2)
 const void *scan_tma_fn(int ch, int ns);
-cudaError_t scan_tma_launch(int ch, int ns, int grid, cudaStream_t st, const BatchBufs &B, const WaveBufs &W,
+void scan_tma_launch(int ch, int ns, int grid, cudaStream_t st, const BatchBufs &B, const WaveBufs &W,
                             const Geom &G, int t0, int it, const ScanMaps &M);
 cudaError_t scan_tma_init();   // dynamic shared-memory limits of the instances
 size_t scan_tma_smem_bytes(const Geom &G, int CH, int NS);
@@ -361,7 +361,8 @@ struct AdjBufs;
 int adj_scan_tma_maps(const Geom &G, float *AF, float *ATot, size_t adj_floats, const float *Cq, size_t layers,
                       AdjScanMaps *M);
 size_t adj_scan_tma_smem_bytes(const Geom &G, int CH, int NS);
-cudaError_t adj_scan_tma_launch(int grid, cudaStream_t st, const BatchBufs &B, const AdjBufs &A, const Geom &G,
+bool adj_scan_tma_supported(const Geom &G);
+void adj_scan_tma_launch(int grid, cudaStream_t st, const BatchBufs &B, const AdjBufs &A, const Geom &G,
                                 int t0, int j, const AdjScanMaps &M);
 // levels of a k_mol_lowrank tile for n_mol tasks of K levels on nsm SMs (four blocks each)
 inline int mol_levels(int n_mol, int K, int nsm) { return (long long)n_mol * ((K + 7) / 8) <= 4 * nsm ? 8 : 32; }

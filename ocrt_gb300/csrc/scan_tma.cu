@@ -581,12 +581,17 @@ __global__ void __launch_bounds__(256, 2) k_adj_scan_tma(BatchBufs B, AdjBufs A,
     }
 }
 
-cudaError_t adj_scan_tma_launch(int grid, cudaStream_t st, const BatchBufs &B, const AdjBufs &A, const Geom &G,
-                                int t0, int j, const AdjScanMaps &M)
+// The kernel's launch bound and shared memory end at 36 streams.
+bool adj_scan_tma_supported(const Geom &G)
 {
-    const int th = scan_tma_threads(G);
-    k_adj_scan_tma<4, 4><<<grid, th, adj_scan_tma_smem_bytes(G, 4, 4), st>>>(B, A, G, t0, j, M);
-    return cudaGetLastError();
+    return scan_tma_threads(G) <= 256 && adj_scan_tma_smem_bytes(G, 4, 4) <= 200 * 1024;
+}
+
+// Launch errors stay for the caller's check.
+void adj_scan_tma_launch(int grid, cudaStream_t st, const BatchBufs &B, const AdjBufs &A, const Geom &G, int t0, int j,
+                         const AdjScanMaps &M)
+{
+    k_adj_scan_tma<4, 4><<<grid, scan_tma_threads(G), adj_scan_tma_smem_bytes(G, 4, 4), st>>>(B, A, G, t0, j, M);
 }
 
 int adj_scan_tma_maps(const Geom &G, float *AF, float *ATot, size_t adj_floats, const float *Cq, size_t layers,
@@ -614,8 +619,8 @@ const void *scan_tma_fn(int ch, int ns)
     return nullptr;
 }
 
-cudaError_t scan_tma_launch(int ch, int ns, int grid, cudaStream_t st, const BatchBufs &B, const WaveBufs &W,
-                            const Geom &G, int t0, int it, const ScanMaps &M)
+void scan_tma_launch(int ch, int ns, int grid, cudaStream_t st, const BatchBufs &B, const WaveBufs &W, const Geom &G, int t0,
+                     int it, const ScanMaps &M)
 {
     const int th = scan_tma_threads(G);
     const size_t sb = scan_tma_smem_bytes(G, ch, ns);
@@ -624,9 +629,7 @@ cudaError_t scan_tma_launch(int ch, int ns, int grid, cudaStream_t st, const Bat
     else if (ch == 4 && ns == 6) k_scan_tma<4, 6><<<grid, th, sb, st>>>(B, W, G, t0, it, M);
     else if (ch == 16 && ns == 2) k_scan_tma<16, 2><<<grid, th, sb, st>>>(B, W, G, t0, it, M);
     else if (ch == 8 && ns == 5) k_scan_tma<8, 5><<<grid, th, sb, st>>>(B, W, G, t0, it, M);
-    else if (ch == 4 && ns == 10) k_scan_tma<4, 10><<<grid, th, sb, st>>>(B, W, G, t0, it, M);
-    else return cudaErrorInvalidValue;
-    return cudaGetLastError();
+    else k_scan_tma<4, 10><<<grid, th, sb, st>>>(B, W, G, t0, it, M);
 }
 
 cudaError_t scan_tma_init()
