@@ -301,7 +301,8 @@ struct Group {
     std::vector<TaskDev> htask;
     std::vector<int> hpix_task0;
     std::vector<Wave> waves;
-    int Lmax = 2, Mmax = 0, max_orders = 1, nphi = 1024;
+    int Lmax = 2, Mmax = 0, max_orders = 1;
+    int nphi = 0;                         // Cox-Munk azimuths, common to the group's pixels
     bool any_pssa = false, any_rough = false, any_flat = false, any_gas = false, any_water = false;
     // coupled atmosphere-ocean: boundary sources read by the solve (owned by the
     // ocean plan), the edge export written after each wave's orders (k_edges)
@@ -575,7 +576,7 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
         g.Lmax = std::max(g.Lmax, d.L);
         g.Mmax = std::max(g.Mmax, d.M);
         g.max_orders = std::max(g.max_orders, d.max_orders);
-        g.nphi = std::max(g.nphi, d.nphi);
+        g.nphi = d.nphi;
         const bool surf = c.surface == OCRT_SURFACE_BLACK_FRESNEL_OCEAN || c.surface == OCRT_SURFACE_FLAT;
         const bool flat = c.surface == OCRT_SURFACE_FLAT || (c.surface == OCRT_SURFACE_BLACK_FRESNEL_OCEAN && c.wind_speed <= 0.0);
         if (patch) patch(q, d);
