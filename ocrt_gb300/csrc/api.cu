@@ -608,7 +608,7 @@ int build_group(Group &g, const ocrt_case *cases, const ocrt_opts *opts, int opp
     g.nlev = lev; g.ncoef = coef; g.nmom = mb.size();
     // ---- waves of whole pixels under the workspace budget ----
     const size_t budget = wave_budget_bytes();
-    const size_t op_elems = (size_t)G.NP * G.CIN;
+    const size_t op_elems = op_floats(G);
     const bool tiles = tc_supported(G) && !force_simt() && !g.fused;
     Wave w{0, 0, 0, 0, 0, 0, 0, 0, false, false};
     size_t bytes = 0;

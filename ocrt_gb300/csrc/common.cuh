@@ -288,6 +288,14 @@ __device__ __forceinline__ void par_put(unsigned char *P, const Geom &g, int si,
 }
 #endif
 
+// Floats of one operator slot: the plain operator, NP rows of CIN, or the molecular
+// factor U, COUT rows of 24, which is the larger at two streams.
+__host__ __device__ inline size_t op_floats(const Geom &g)
+{
+    const size_t a = (size_t)g.NP * g.CIN, u = (size_t)g.COUT * 24;
+    return a > u ? a : u;
+}
+
 // Operator entry (row, cin) into the pre-split tensor-core tiles of one
 // operator: per 32-column K tile kt, a tf32 hi tile then a lo tile of NP rows
 // x 128 bytes in the SWIZZLE_128B K-major layout the MMA reads (16-byte chunk

@@ -145,7 +145,7 @@ extern "C" int ocrt_gb_solve_case_noalloc(const ocrt_case *cs, const ocrt_opts *
     const bool flat = cs->surface == OCRT_SURFACE_FLAT ||
                       (cs->surface == OCRT_SURFACE_BLACK_FRESNEL_OCEAN && cs->wind_speed <= 0.0);
     const bool rough = surf && !flat;
-    const size_t op_elems = (size_t)G.NP * G.CIN;
+    const size_t op_elems = op_floats(G);
     const size_t srf_elems = (size_t)NR * N * 9 + (size_t)NR * 9;
 
     // ---- carve the static array: fixed part, then as many mode tasks per wave as fit ----
